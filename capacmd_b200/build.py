@@ -85,9 +85,9 @@ def build_driver(verbose: bool = False) -> str:
 
 def reference_dir(reference: str | None = None) -> str | None:
     """The reference source folder: the argument, else $CAPAC_REFERENCE_SRC;
-    None when neither names an existing folder."""
+    None when neither names a folder that holds the sources."""
     ref = reference or os.environ.get("CAPAC_REFERENCE_SRC")
-    return ref if ref and os.path.isdir(ref) else None
+    return ref if ref and os.path.isfile(os.path.join(ref, "force.c")) else None
 
 
 def build_oracle(verbose: bool = False, reference: str | None = None) -> None:
