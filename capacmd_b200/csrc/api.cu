@@ -557,6 +557,12 @@ int capac_create(const capac_desc *d, const capac_options *opt, capac_ctx **out)
                                     if (c->tmem_tiles) c->group_grid = g;
                                 }
                             }
+                            // small systems; CAPAC_SOLVER_TILED at creation keeps the tiled solver
+                            if ((!mixed || c->grouped) && !getenv("CAPAC_SOLVER_TILED") &&
+                                dense_fits(c->device, n, mixed)) {
+                                c->dense_ex = dalloc<unsigned char>(dense_exchange_bytes(n));
+                                CAPAC_CUDA(cudaMemsetAsync(c->dense_ex, 0, dense_exchange_bytes(n), s));
+                            }
                         }
                     } else if (mixed) {
                         c->matf = dalloc<float>((size_t)M * 16 * c->Mp);
@@ -637,7 +643,7 @@ int capac_destroy(capac_ctx *c)
                    c->cl_nbr, c->cl_nnb, c->cl_metal, c->cl_of, c->cl_next, c->cl_sel, c->n_cl_sel, c->partials2,
                    c->cp_list,
                    c->cp_n, c->cp_cent, c->cp_off, c->cp_ti, c->cz_az, c->cz_w, c->cz_einv, c->cz_aug, c->cz_zbuf, c->scan_tmp, c->isd, c->vec_ext, c->vec_pq,
-                   c->diag, c->mat, c->matf, c->msym, c->sympart, c->coop_bp, c->coop_bar, c->g_atoms, c->dinv, c->slot_np, c->np_off, c->np_rows, c->gvec, c->gw, c->em_buf, c->phase_buf, c->rres, c->dcorr, c->xprev, c->bw, c->bwf, c->ss, c->partials, c->pot, c->vir, c->th};
+                   c->diag, c->mat, c->matf, c->msym, c->sympart, c->dense_ex, c->coop_bp, c->coop_bar, c->g_atoms, c->dinv, c->slot_np, c->np_off, c->np_rows, c->gvec, c->gw, c->em_buf, c->phase_buf, c->rres, c->dcorr, c->xprev, c->bw, c->bwf, c->ss, c->partials, c->pot, c->vir, c->th};
     for (void *p : dev)
         if (p) cudaFree(p);
     for (void *p : c->bonded_buffers)

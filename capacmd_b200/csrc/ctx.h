@@ -18,6 +18,8 @@ struct SolverScalars {
     double res0;     // refinement: FP64 residual norm^2 at the sweep start
     double rr0;      // (r, r) of the warm start
     int iter, done, status, max_iter;
+    int error;       // dense solver: a bounded poll gave up
+    int outer;       // dense solver, mixed path: refinement sweeps
 };
 
 // Thermostat and integrator scalars (System, typedef.h:353-401).
@@ -267,6 +269,9 @@ struct capac_ctx {
     double phase_ns[8] = {};
     long phase_iters = 0;
     double *gw = nullptr;                 // gradient workspace (k_grad.cu), allocated on first use
+    // small systems: the dense solver's exchange buffers (null: not used) and next exchange number
+    void *dense_ex = nullptr;
+    unsigned long long dense_seq = 1;
     double *coop_bp = nullptr;   // its per-block dot partials
     void *coop_bar = nullptr;    // its grid barrier
     double *bw = nullptr;        // BiCGSTAB work vectors, 11 * n_mat
@@ -348,6 +353,11 @@ int coop_grid_size(int device, bool mixed);
 size_t coop_barrier_bytes();
 size_t coop_partial_doubles(int grid);
 int bicgstab_coop(capac_ctx *c, const double *b, double *x, double tol, double skip);
+// small systems: the FP64 matrix on chip (k_solve_dense.cu)
+bool dense_fits(int device, int n, bool mixed);
+size_t dense_exchange_bytes(int n);
+int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double skip, double *hist = nullptr,
+                   int order = 0);
 // group-ordered solver (k_solve_coop.cu): internal vector length, blocks
 int group_tmem_tiles();
 int coarse_columns(int M, int n_nps, int modes);

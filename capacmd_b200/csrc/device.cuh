@@ -63,6 +63,32 @@ __device__ __forceinline__ float warp_sumf(float v)
     return v;
 }
 
+// Sums of V values over the 32 lanes of a warp by recursive halving: at
+// each step a lane keeps half of its values and adds the partner's copy of
+// that half (V/2 + V/4 + ... + 1 exchanges), then plain exchanges for the
+// remaining lane bits; V - 1 + 5 - log2 V shuffles instead of 5 V.  Lane l
+// returns the sum of value l >> (5 - log2 V).  The order of additions is
+// fixed.
+template <int V, typename R>
+__device__ __forceinline__ R warp_sum_halving(R (&v)[V], int lane)
+{
+    int m = 16;
+#pragma unroll
+    for (int half = V / 2; half >= 1; half >>= 1, m >>= 1) {
+        const bool upper = (lane & m) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const R send = upper ? v[i] : v[i + half];
+            const R keep = upper ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+        }
+    }
+    R s = v[0];
+#pragma unroll
+    for (; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    return s;
+}
+
 // Sum K values over the block (blockDim.x a multiple of 32, at most 1024) in
 // a fixed order; thread 0 receives the totals in v[].  `sh` needs 32*K doubles.
 template <int K>

@@ -259,7 +259,11 @@ void launch_cpim_block_rows(capac_ctx *c, int i0, int rows, double *out)
 void launch_cpim_matrix(capac_ctx *c)
 {
     if (c->msym) {
-        launch_sym_assemble(c);
+        // (the dense solver forms the mixed path's matrix from the positions
+        // itself: the tiles then serve the coarse refreshes only)
+        const bool due = c->dinv && c->precond_age % kPrecondEvery == 0;
+        const bool coarse = due && c->twolevel && (c->precond_age == 0 || c->coarse_age % kCoarseEvery == 0);
+        if (!c->dense_ex || c->opt.precision != CAPAC_PREC_MIXED || coarse) launch_sym_assemble(c);
         // the preconditioner only steers the inner solves (the FP64 residual
         // defines the answer), so its inverse blocks are refreshed every
         // kPrecondEvery matrix builds, not every step
@@ -801,6 +805,17 @@ constexpr double kInnerReduction = 1.0e-5;
 // an inner solve whose (r, r) has not halved for this many iterations stops
 // and returns its iterate to the refinement
 constexpr int kInnerStall = 60;
+// The status of a refinement that ended at (r, r) = rr, short of its target or not.
+static int refined_status(bool missed, double rr, double bTb)
+{
+    if (!missed) return CAPAC_OK;
+    if (rr < 1.0e-8 * bTb) {  // the reference's own criterion still holds
+        fprintf(stderr, "Note: refinement stopped at relative residual %.3e\n", sqrt(rr / bTb));
+        return CAPAC_OK;
+    }
+    return CAPAC_ERR_NOT_CONVERGED;
+}
+
 int run_refined_solve(capac_ctx *c)
 {
     const int n = c->n_mat;
@@ -809,6 +824,21 @@ int run_refined_solve(capac_ctx *c)
     const double rtol = c->opt.refine_tol > 0.0 ? c->opt.refine_tol : 1.0e-10;
     const int max_sweeps = 12;
 
+    if (c->dense_ex) {  // small systems: predictor, solve and residual in one launch
+        const bool hist = c->opt.predictor > 0 && c->xprev;
+        const int st = bicgstab_dense(c, c->vec_ext, c->vec_pq, rtol * rtol, 1.0e-10, hist ? c->xprev : nullptr,
+                                      std::min(c->opt.predictor, c->n_solves - 1));
+        c->last_iters = c->last_outer = 0;
+        c->last_rel_res = 0.0;
+        const double bTb = c->h_ss->bTb, rr = c->h_ss->rTr;
+        if (bTb < 1.0e-10) return CAPAC_OK;  // zero right-hand side: keep x
+        ++c->n_solves;
+        c->last_iters = c->h_ss->iter;
+        c->last_outer = c->h_ss->outer;
+        c->last_init_res = sqrt(c->h_ss->rr0 / bTb);
+        c->last_rel_res = sqrt(rr / bTb);
+        return refined_status(st < 0 || !(rr <= rtol * rtol * bTb), rr, bTb);
+    }
     k_vec_dot<<<nbv, 256, 0, s>>>(n, c->vec_ext, c->vec_ext, c->partials);
     k_bcg_start<<<1, 256, 0, s>>>(c->partials, nbv, 1.0, 1.0e-10, solver_max_iter(c), c->ss);
     c->launches += 2;
@@ -859,12 +889,7 @@ int run_refined_solve(capac_ctx *c)
     c->last_iters = total;
     c->last_outer = sweep;
     c->last_rel_res = sqrt(rr / bTb);
-    if (rr <= rtol * rtol * bTb) return CAPAC_OK;
-    if (rr < 1.0e-8 * bTb) {  // the reference's own criterion still holds
-        fprintf(stderr, "Note: refinement stopped at relative residual %.3e\n", c->last_rel_res);
-        return CAPAC_OK;
-    }
-    return CAPAC_ERR_NOT_CONVERGED;
+    return refined_status(!(rr <= rtol * rtol * bTb), rr, bTb);
 }
 
 // ------------------------------------------------- CPIM metal-side forces

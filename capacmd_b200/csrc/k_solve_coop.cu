@@ -107,32 +107,6 @@ __device__ __forceinline__ void ldsc(const R *p, R (&out)[kCols])
     }
 }
 
-// Sums of V values over the 32 lanes of a warp by recursive halving: at
-// each step a lane keeps half of its values and adds the partner's copy of
-// that half (V/2 + V/4 + ... + 1 exchanges), then plain exchanges for the
-// remaining lane bits; V - 1 + 5 - log2 V shuffles instead of 5 V.  Lane l
-// returns the sum of value l >> (5 - log2 V).  The order of additions is
-// fixed.
-template <int V, typename R>
-__device__ __forceinline__ R warp_sum_halving(R (&v)[V], int lane)
-{
-    int m = 16;
-#pragma unroll
-    for (int half = V / 2; half >= 1; half >>= 1, m >>= 1) {
-        const bool upper = (lane & m) != 0;
-#pragma unroll
-        for (int i = 0; i < half; ++i) {
-            const R send = upper ? v[i] : v[i + half];
-            const R keep = upper ? v[i + half] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
-        }
-    }
-    R s = v[0];
-#pragma unroll
-    for (; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
-    return s;
-}
-
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count)
@@ -1853,6 +1827,7 @@ int bicgstab_group(capac_ctx *c, const double *b, double *x, double tol, double 
 // Launch the persistent solver; returns the status as bicgstab_core does.
 int bicgstab_coop(capac_ctx *c, const double *b, double *x, double tol, double skip)
 {
+    if (c->dense_ex) return bicgstab_dense(c, b, x, tol, skip);
     if (c->grouped) return bicgstab_group(c, b, x, tol, skip);
     const int n = c->n_mat;
     double *bw = c->bw;
