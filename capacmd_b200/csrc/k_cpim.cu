@@ -1104,7 +1104,7 @@ size_t partials_needed(const capac_ctx *c)
     need = std::max(need, (size_t)c->num_sms * 2 * 11);  // resident pair grids (two blocks per SM)
     need = std::max(need, (size_t)grid_for((long)c->N, 256) * 16);
     need = std::max(need, (size_t)(c->M + c->n_nps + 8) * 16);
-    need = std::max(need, (size_t)grid_for((long)c->n_mols, 256) * 16);
+    need = std::max(need, (size_t)grid_for((long)c->n_mols, 128) * 16);  // RATTLE blocks
     need = std::max(need, (size_t)grid_for((long)c->n_mat, 256) * 4);
     need = std::max(need, (size_t)c->M * 20);  // gradient sums (k_grad.cu)
     return need + 64;

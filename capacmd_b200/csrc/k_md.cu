@@ -38,45 +38,86 @@ __global__ void k_heating(ThermoState *th, long step, int n_heating)
     th->kT = kBoltz * th->ref_temp;
 }
 
-// nose_hoover_chain, thermostat.c:117-191: 10 links, Nc = 5, 5th-order
-// Suzuki-Yoshida weights; the velocity scale is left in th->scale.
-__global__ void k_nhc(ThermoState *th, MdParams m)
+// exp(x) for |x| < 1/64: the Taylor sum to x^7, whose remainder there is 9e-20
+// of the result, in pairs so that four dependent operations form it.
+__device__ __forceinline__ double exp_small(double x)
+{
+    const double x2 = x * x;
+    const double a = fma(x, 1.0 / 6.0, 0.5), b = fma(x, 1.0 / 120.0, 1.0 / 24.0), c = fma(x, 1.0 / 5040.0, 1.0 / 720.0);
+    return 1.0 + fma(x2, fma(x2, fma(x2, c, b), a), x);
+}
+
+// The Nose-Hoover chain of k_nhc from the given velocities; returns the
+// velocity scale.  SMALL: with exp_small; `most` is then the largest argument
+// met, and the result holds only below 1/64.
+template <bool SMALL>
+__device__ __forceinline__ double nhc_chain(double (&vQ)[kNhc], double (&aQ)[kNhc], double ek, double NkT, double c0,
+                                            double inv_q, double dt, double &most)
 {
     const int Nc = 5, L = kNhc;
     const double w1 = 0.41449077179437571194, w3 = -0.65796308717750284778;
     const double w[5] = {w1, w1, w3, w1, w1};
-    const double Q = m.q_mass, kT = th->kT, NkT = kT * m.ndf, dt = m.dt, ek = th->eksum;
-    // the chain in registers (every index is fixed once the loops unroll),
-    // written back at the end
-    double vQ[kNhc], aQ[kNhc], scale = 1.0;
+    double scale = 1.0;
+    most = 0.0;
+    auto ex = [&](double x) {
+        if (!SMALL) return exp(x);
+        most = fmax(most, fabs(x));
+        return exp_small(x);
+    };
+    aQ[0] = (ek - NkT) * inv_q;
 #pragma unroll
-    for (int k = 0; k < L; ++k) vQ[k] = th->vQ[k];
-    aQ[0] = (ek - NkT) / Q;
-#pragma unroll
-    for (int k = 0; k < L - 1; ++k) aQ[k + 1] = (Q * vQ[k] * vQ[k] - kT) / Q;
+    for (int k = 0; k < L - 1; ++k) aQ[k + 1] = fma(vQ[k], vQ[k], -c0);
     for (int c = 0; c < Nc; ++c) {
 #pragma unroll
         for (int y = 0; y < 5; ++y) {
             const double h4 = w[y] * dt / (4 * Nc), h8 = w[y] * dt / (8 * Nc), h2 = w[y] * dt / (2 * Nc);
             vQ[L - 1] += aQ[L - 1] * h4;
 #pragma unroll
-            for (int k = 0; k < L - 1; ++k) {
-                const double e = exp(-h8 * vQ[L - (k + 1)]);
-                vQ[L - 1 - (k + 1)] = vQ[L - 1 - (k + 1)] * e * e + h4 * aQ[L - 1 - (k + 1)] * e;
+            for (int k = L - 2; k >= 0; --k) {
+                const double e = ex(-h8 * vQ[k + 1]);
+                vQ[k] = e * fma(vQ[k], e, h4 * aQ[k]);
             }
-            scale *= exp(-h2 * vQ[0]);
-            aQ[0] = (ek * scale * scale - NkT) / Q;
+            scale *= ex(-h2 * vQ[0]);
+            aQ[0] = fma(ek * scale, scale, -NkT) * inv_q;
+            double e[kNhc];
+#pragma unroll
+            for (int k = 0; k < L - 1; ++k) e[k] = ex(-h8 * vQ[k + 1]);
 #pragma unroll
             for (int k = 0; k < L - 1; ++k) {
-                const double e = exp(-h8 * vQ[k + 1]);
-                vQ[k] = vQ[k] * e * e + h4 * aQ[k] * e;
-                aQ[k + 1] = (Q * vQ[k] * vQ[k] - kT) / Q;
+                vQ[k] = fma(h4 * e[k], aQ[k], vQ[k] * e[k] * e[k]);
+                aQ[k + 1] = fma(vQ[k], vQ[k], -c0);
             }
             vQ[L - 1] += aQ[L - 1] * h4;
         }
     }
+    return scale;
+}
+
+// nose_hoover_chain, thermostat.c:117-191: 10 links, Nc = 5, 5th-order
+// Suzuki-Yoshida weights; the velocity scale is left in th->scale.  One
+// thread: 25 sweeps down and up the chain, each link waiting for the last, so
+// the length of one link's chain of operations is the time.  The exponentials'
+// arguments are a time step over 40 times a thermostat velocity, far below the
+// 1/64 up to which exp_small serves (else the chain runs again with the
+// library's); on the way up they are those of velocities the way down left
+// final, so only a multiply-add pair waits; the divisions by Q are folded into
+// kT / Q.  41 us a launch with the library's exp and the divisions, 14.6 so.
+__global__ void k_nhc(ThermoState *th, MdParams m)
+{
+    const double Q = m.q_mass, kT = th->kT, NkT = kT * m.ndf, ek = th->eksum, inv_q = 1.0 / Q;
+    // the chain in registers (every index is fixed once the loops unroll),
+    // written back at the end
+    double vQ[kNhc], aQ[kNhc], most;
 #pragma unroll
-    for (int k = 0; k < L; ++k) {
+    for (int k = 0; k < kNhc; ++k) vQ[k] = th->vQ[k];
+    double scale = nhc_chain<true>(vQ, aQ, ek, NkT, kT * inv_q, inv_q, m.dt, most);
+    if (!(most < 0.015625)) {
+#pragma unroll
+        for (int k = 0; k < kNhc; ++k) vQ[k] = th->vQ[k];
+        scale = nhc_chain<false>(vQ, aQ, ek, NkT, kT * inv_q, inv_q, m.dt, most);
+    }
+#pragma unroll
+    for (int k = 0; k < kNhc; ++k) {
         th->vQ[k] = vQ[k];
         th->aQ[k] = aQ[k];
     }
@@ -151,36 +192,54 @@ struct CstrView {
     const int *mol_atoms;  // atoms per molecule type
 };
 
-// Three-atom molecules with at most three constraints (the 3-site waters)
-// iterate on a copy of their atoms held in registers, written back once: the
-// same operations in the same order as on the global arrays, without a round
-// trip to L2 per constraint and iteration.  Mol3 reads and updates atom a of
-// a molecule with selects, so the values never leave registers.
-struct Mol3 {
-    double v0, v1, v2;
-    __device__ __forceinline__ double get(int a) const { return a == 0 ? v0 : (a == 1 ? v1 : v2); }
-    __device__ __forceinline__ void add(int a, double x)
+// Three-atom molecules with at most three constraints (the 3-site waters) are
+// iterated in the constraints' own variables, in registers.  A correction g of
+// constraint k moves atom t by sgn(t, k) m_t g times a vector d_k that does not
+// change during the iteration (the old bond in the first stage, the bond in the
+// second), so a bond's difference vector or projected velocity changes by
+// weight(l, k) g d_k: the loop updates those and sums the g of each constraint,
+// and the atoms are moved once at the end by the sums.  The same corrections
+// and tests in the same order as on the atoms, to rounding; an iteration of a
+// constraint waits for a few operations where the selects of its atoms'
+// coordinates, the image shifts and the updates of positions and velocities
+// made ~1,500 cycles of it (first and second stage, us a launch: 31 and 48 -> 14
+// and 9 for 3,000 waters, 74 and 117 -> 45 and 25 for 150,000).
+struct Bonds3 {
+    int ca[3], cb[3];
+    double im[3], d[3][3];  // inverse masses; d_k
+    __device__ __forceinline__ void load(const CstrView &cv, int first, int c0, int nc)
     {
-        if (a == 0) v0 += x;
-        else if (a == 1) v1 += x;
-        else v2 += x;
+#pragma unroll
+        for (int t = 0; t < 3; ++t) im[t] = cv.inv_mass[first + t];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            ca[k] = k < nc ? cv.ci[c0 + k] : 0;
+            cb[k] = k < nc ? cv.cj[c0 + k] : 0;
+        }
     }
-    __device__ __forceinline__ void load(const double *p, int first)
+    __device__ __forceinline__ double mass(int t) const { return t == 0 ? im[0] : (t == 1 ? im[1] : im[2]); }
+    // the move of atom t per g of constraint k, along d_k
+    __device__ __forceinline__ double move(int t, int k) const
     {
-        v0 = p[first];
-        v1 = p[first + 1];
-        v2 = p[first + 2];
+        return (t == ca[k] ? mass(t) : 0.0) - (t == cb[k] ? mass(t) : 0.0);
     }
-    __device__ __forceinline__ void store(double *p, int first) const
+    // the change of bond l's difference per g of constraint k, along d_k
+    __device__ __forceinline__ double weight(int l, int k) const { return move(ca[l], k) - move(cb[l], k); }
+    // bond k's difference of the atoms' values r
+    __device__ __forceinline__ double diff(const double (&r)[3], int k) const
     {
-        p[first] = v0;
-        p[first + 1] = v1;
-        p[first + 2] = v2;
+        const double a = ca[k] == 0 ? r[0] : (ca[k] == 1 ? r[1] : r[2]);
+        const double b = cb[k] == 0 ? r[0] : (cb[k] == 1 ? r[1] : r[2]);
+        return a - b;
     }
 };
 
+// Threads of a block of the RATTLE kernels: one warp per scheduler, so that a
+// few thousand molecules spread over as many SMs as they can.
+constexpr int kRattleBlock = 128;
+
 // rattle_1st, force.c:1907-1997: one thread per molecule.
-__global__ void __launch_bounds__(256, 2) k_rattle1(MdParams m, CstrView cv, double *rx, double *ry, double *rz, const double *ox,
+__global__ void __launch_bounds__(kRattleBlock) k_rattle1(MdParams m, CstrView cv, double *rx, double *ry, double *rz, const double *ox,
                           const double *oy, const double *oz, double *vx, double *vy, double *vz, int *flags)
 {
     const int im = blockIdx.x * blockDim.x + threadIdx.x;
@@ -191,50 +250,63 @@ __global__ void __launch_bounds__(256, 2) k_rattle1(MdParams m, CstrView cv, dou
     const double tol2 = 2.0e-05, inv_dt = 1.0 / m.dt;  // the velocity update multiplies by 1/dt
     int iter = 0, done = 0;
     if (cv.mol_atoms[mt] == 3 && nc <= 3) {
-        Mol3 X, Y, Z, VX, VY, VZ, OX, OY, OZ, IM;
-        X.load(rx, first); Y.load(ry, first); Z.load(rz, first);
-        VX.load(vx, first); VY.load(vy, first); VZ.load(vz, first);
-        OX.load(ox, first); OY.load(oy, first); OZ.load(oz, first);
-        IM.load(cv.inv_mass, first);
-        int ca[3] = {0, 0, 0}, cb[3] = {0, 0, 0};
-        double l2[3] = {0.0, 0.0, 0.0};
+        Bonds3 B;
+        B.load(cv, first, c0, nc);
+        double *const r[3] = {rx, ry, rz}, *const v[3] = {vx, vy, vz};
+        const double *const o[3] = {ox, oy, oz};
+        double x[3][3], p[3][3], len2[3], scale[3], w[3][3], G[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (k < nc) {
-                ca[k] = cv.ci[c0 + k];
-                cb[k] = cv.cj[c0 + k];
-                l2[k] = cv.len[c0 + k] * cv.len[c0 + k];
+        for (int a = 0; a < 3; ++a) {
+            double old[3];
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                x[a][t] = r[a][first + t];
+                old[t] = o[a][first + t];
             }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                p[k][a] = wrap1(B.diff(x[a], k), m.box.L[a]);
+                B.d[k][a] = wrap1(B.diff(old, k), m.box.L[a]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double len = k < nc ? cv.len[c0 + k] : 0.0;
+            len2[k] = len * len;
+            scale[k] = 2.0 * (B.mass(B.ca[k]) + B.mass(B.cb[k]));
+#pragma unroll
+            for (int l = 0; l < 3; ++l) w[l][k] = B.weight(l, k);
+        }
         while (!done) {
             done = 1;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 if (k >= nc) continue;
-                const int a = ca[k], b = cb[k];
-                const double len2 = l2[k];
-                const double px = wrap1(X.get(a) - X.get(b), m.box.L[0]);
-                const double py = wrap1(Y.get(a) - Y.get(b), m.box.L[1]);
-                const double pz = wrap1(Z.get(a) - Z.get(b), m.box.L[2]);
-                const double diff = len2 - (px * px + py * py + pz * pz);
-                if (fabs(diff) > len2 * tol2) {
-                    const double qx = wrap1(OX.get(a) - OX.get(b), m.box.L[0]);
-                    const double qy = wrap1(OY.get(a) - OY.get(b), m.box.L[1]);
-                    const double qz = wrap1(OZ.get(a) - OZ.get(b), m.box.L[2]);
-                    const double ma = IM.get(a), mb = IM.get(b);
-                    const double g = diff / (2.0 * (ma + mb) * (qx * px + qy * py + qz * pz));
-                    double dx = qx * g, dy = qy * g, dz = qz * g;
-                    X.add(a, ma * dx); Y.add(a, ma * dy); Z.add(a, ma * dz);
-                    X.add(b, -(mb * dx)); Y.add(b, -(mb * dy)); Z.add(b, -(mb * dz));
-                    dx *= inv_dt; dy *= inv_dt; dz *= inv_dt;
-                    VX.add(a, ma * dx); VY.add(a, ma * dy); VZ.add(a, ma * dz);
-                    VX.add(b, -(mb * dx)); VY.add(b, -(mb * dy)); VZ.add(b, -(mb * dz));
+                const double diff = len2[k] - (p[k][0] * p[k][0] + p[k][1] * p[k][1] + p[k][2] * p[k][2]);
+                if (fabs(diff) > len2[k] * tol2) {
+                    const double g = diff / (scale[k] * (B.d[k][0] * p[k][0] + B.d[k][1] * p[k][1] + B.d[k][2] * p[k][2]));
+                    G[k] += g;
+#pragma unroll
+                    for (int l = 0; l < 3; ++l) {
+                        const double wg = w[l][k] * g;
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) p[l][a] = fma(wg, B.d[k][a], p[l][a]);
+                    }
                     done = 0;
                 }
             }
             if (++iter > kMaxIter) break;
         }
-        X.store(rx, first); Y.store(ry, first); Z.store(rz, first);
-        VX.store(vx, first); VY.store(vy, first); VZ.store(vz, first);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            const double g0 = B.move(t, 0) * G[0], g1 = B.move(t, 1) * G[1], g2 = B.move(t, 2) * G[2];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const double dx = fma(g0, B.d[0][a], fma(g1, B.d[1][a], g2 * B.d[2][a]));
+                r[a][first + t] = x[a][t] + dx;
+                v[a][first + t] += dx * inv_dt;
+            }
+        }
         if (!done) atomicOr(&flags[2], 1);
         return;
     }
@@ -269,7 +341,7 @@ __global__ void __launch_bounds__(256, 2) k_rattle1(MdParams m, CstrView cv, dou
 
 // rattle_2nd, force.c:2004-2090: one thread per molecule; the constraint
 // virial goes to per-block partials.
-__global__ void __launch_bounds__(256) k_rattle2(MdParams m, CstrView cv, const double *rx, const double *ry,
+__global__ void __launch_bounds__(kRattleBlock) k_rattle2(MdParams m, CstrView cv, const double *rx, const double *ry,
                                                  const double *rz, double *vx, double *vy, double *vz,
                                                  int *flags, double *partials)
 {
@@ -287,46 +359,61 @@ __global__ void __launch_bounds__(256) k_rattle2(MdParams m, CstrView cv, const 
         int iter = 0, done = nc == 0;
         const bool fast = !done && cv.mol_atoms[mt] == 3 && nc <= 3;
         if (fast) {
-            Mol3 X, Y, Z, VX, VY, VZ, IM;
-            X.load(rx, first); Y.load(ry, first); Z.load(rz, first);
-            VX.load(vx, first); VY.load(vy, first); VZ.load(vz, first);
-            IM.load(cv.inv_mass, first);
-            int ca[3] = {0, 0, 0}, cb[3] = {0, 0, 0};
-            double inv_den[3] = {0.0, 0.0, 0.0};
+            Bonds3 B;
+            B.load(cv, first, c0, nc);
+            const double *const r[3] = {rx, ry, rz};
+            double *const v[3] = {vx, vy, vz};
+            double u[3][3], c[3] = {0.0, 0.0, 0.0}, inv_den[3], C[3][3], G[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-            for (int k = 0; k < 3; ++k)
-                if (k < nc) {
-                    ca[k] = cv.ci[c0 + k];
-                    cb[k] = cv.cj[c0 + k];
-                    const double len = cv.len[c0 + k];
-                    inv_den[k] = 1.0 / ((IM.get(ca[k]) + IM.get(cb[k])) * (len * len));
+            for (int a = 0; a < 3; ++a) {
+                double x[3];
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    x[t] = r[a][first + t];
+                    u[a][t] = v[a][first + t];
                 }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    B.d[k][a] = wrap1(B.diff(x, k), m.box.L[a]);
+                    c[k] = fma(B.d[k][a], B.diff(u[a], k), c[k]);  // projected relative velocity
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double len = k < nc ? cv.len[c0 + k] : 1.0;
+                inv_den[k] = 1.0 / ((B.mass(B.ca[k]) + B.mass(B.cb[k])) * (len * len));
+#pragma unroll
+                for (int l = 0; l < 3; ++l)
+                    C[l][k] = B.weight(l, k) * (B.d[l][0] * B.d[k][0] + B.d[l][1] * B.d[k][1] + B.d[l][2] * B.d[k][2]);
+            }
             while (!done) {
                 done = 1;
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     if (k >= nc) continue;
-                    const int a = ca[k], b = cb[k];
-                    const double ux = VX.get(a) - VX.get(b), uy = VY.get(a) - VY.get(b), uz = VZ.get(a) - VZ.get(b);
-                    const double px = wrap1(X.get(a) - X.get(b), m.box.L[0]);
-                    const double py = wrap1(Y.get(a) - Y.get(b), m.box.L[1]);
-                    const double pz = wrap1(Z.get(a) - Z.get(b), m.box.L[2]);
-                    const double ma = IM.get(a), mb = IM.get(b);
-                    const double g = -(px * ux + py * uy + pz * uz) * inv_den[k];
+                    const double g = -c[k] * inv_den[k];
                     if (fabs(g) > tol) {
-                        double dx = px * g, dy = py * g, dz = pz * g;
-                        VX.add(a, ma * dx); VY.add(a, ma * dy); VZ.add(a, ma * dz);
-                        VX.add(b, -(mb * dx)); VY.add(b, -(mb * dy)); VZ.add(b, -(mb * dz));
-                        dx *= inv_hdt; dy *= inv_hdt; dz *= inv_hdt;
-                        vir[0] -= px * dx; vir[1] -= px * dy; vir[2] -= px * dz;
-                        vir[3] -= py * dx; vir[4] -= py * dy; vir[5] -= py * dz;
-                        vir[6] -= pz * dx; vir[7] -= pz * dy; vir[8] -= pz * dz;
+                        G[k] += g;
+#pragma unroll
+                        for (int l = 0; l < 3; ++l) c[l] = fma(C[l][k], g, c[l]);
                         done = 0;
                     }
                 }
                 if (++iter > kMaxIter) break;
             }
-            VX.store(vx, first); VY.store(vy, first); VZ.store(vz, first);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                const double g0 = B.move(t, 0) * G[0], g1 = B.move(t, 1) * G[1], g2 = B.move(t, 2) * G[2];
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    v[a][first + t] = u[a][t] + fma(g0, B.d[0][a], fma(g1, B.d[1][a], g2 * B.d[2][a]));
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) vir[3 * a + b] -= B.d[k][a] * (B.d[k][b] * G[k] * inv_hdt);
         }
         while (!fast && !done) {
             done = 1;
@@ -620,13 +707,13 @@ void launch_md_drift(capac_ctx *c)
 void launch_rattle(capac_ctx *c, int second)
 {
     if (!c->has_cstr) return;
-    const unsigned grid = grid_for(c->n_mols, 256);
+    const unsigned grid = grid_for(c->n_mols, kRattleBlock);
     if (!second) {
-        k_rattle1<<<grid, 256, 0, c->stream>>>(md_params(c), cstr_view(c), c->rx, c->ry, c->rz, c->ox, c->oy, c->oz,
+        k_rattle1<<<grid, kRattleBlock, 0, c->stream>>>(md_params(c), cstr_view(c), c->rx, c->ry, c->rz, c->ox, c->oy, c->oz,
                                                c->vx, c->vy, c->vz, c->flags);
         ++c->launches;
     } else {
-        k_rattle2<<<grid, 256, 0, c->stream>>>(md_params(c), cstr_view(c), c->rx, c->ry, c->rz, c->vx, c->vy, c->vz,
+        k_rattle2<<<grid, kRattleBlock, 0, c->stream>>>(md_params(c), cstr_view(c), c->rx, c->ry, c->rz, c->vx, c->vy, c->vz,
                                                c->flags, c->partials);
         ++c->launches;
         static const int pot_slots[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
