@@ -247,21 +247,27 @@ __device__ __forceinline__ int cluster_offsets(const int m[4], const double *__r
     return nk;
 }
 
-// The clusters of one cell (a thread per cell), and in flags[5] the largest
-// component of a member's offset from its cluster's centroid (float bits,
-// rounded up).
+// The clusters (a thread per cluster), and in flags[5] the largest component
+// of a member's offset from its cluster's centroid (float bits, rounded up).
+// A thread finds its cell by bisecting the cells' first clusters: boxes under
+// seven half-cell edges are one cell, whose clusters one thread per cell would
+// form one after the other (3,147 atoms in one cell: 802 us, here 6).
 // cl_of (half list, else null): the cluster of each atom.
 __global__ void k_make_clusters(int n_cells, const int *__restrict__ cell_start, const int *__restrict__ cl_start,
                                 const int *__restrict__ cell_atoms, const double *__restrict__ rx,
                                 const double *__restrict__ ry, const double *__restrict__ rz, InvBox B,
                                 int4 *cl_atoms, int *cl_of, int *flags)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_cells) return;
-    const int s = cell_start[c], e = cell_start[c + 1];
-    int cl = cl_start[c];
-    double emax = 0.0;
-    for (int p = s; p < e; p += 4, ++cl) {
+    const int cl = blockIdx.x * blockDim.x + threadIdx.x;
+    float emax = 0.f;
+    if (cl < cl_start[n_cells]) {
+        int lo = 0, hi = n_cells;  // cl_start[lo] <= cl < cl_start[hi]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (cl_start[mid] <= cl) lo = mid;
+            else hi = mid;
+        }
+        const int p = cell_start[lo] + 4 * (cl - cl_start[lo]), e = cell_start[lo + 1];
         int m[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) m[t] = p + t < e ? cell_atoms[p + t] : -1;
@@ -269,12 +275,14 @@ __global__ void k_make_clusters(int n_cells, const int *__restrict__ cell_start,
         if (cl_of)
             for (int t = 0; t < 4; ++t)
                 if (m[t] >= 0) cl_of[m[t]] = cl;
-        double o[4][3], cc[3];
+        double o[4][3], cc[3], ext = 0.0;
         const int nk = cluster_offsets(m, rx, ry, rz, B, o, cc);
         for (int k = 0; k < nk; ++k)
-            for (int a = 0; a < 3; ++a) emax = fmax(emax, fabs(o[k][a]));
+            for (int a = 0; a < 3; ++a) ext = fmax(ext, fabs(o[k][a]));
+        emax = __double2float_ru(ext);
     }
-    if (emax > 0.0) atomicMax(&flags[5], __float_as_int(__double2float_ru(emax)));
+    const int bits = __reduce_max_sync(0xffffffffu, __float_as_int(emax));  // non-negative: ordered as integers
+    if ((threadIdx.x & 31) == 0 && bits > 0) atomicMax(&flags[5], bits);
 }
 
 // One warp per cluster: the cluster list (see the file comment).
@@ -834,7 +842,7 @@ bool make_clusters(capac_ctx *c, int n_cells)
     }
     CAPAC_CUDA(cub::DeviceScan::ExclusiveSum(c->scan_tmp, need, c->cl_counts, c->cl_cell_start, n_cells + 1, s));
     CAPAC_CUDA(cudaMemsetAsync(c->flags + 5, 0, sizeof(int), s));
-    k_make_clusters<<<grid_for(n_cells, 128), 128, 0, s>>>(n_cells, c->cell_start, c->cl_cell_start, c->cell_atoms,
+    k_make_clusters<<<grid_for(c->cl_max, 128), 128, 0, s>>>(n_cells, c->cell_start, c->cl_cell_start, c->cell_atoms,
                                                            c->rx, c->ry, c->rz, inv_box(c), c->cl_atoms,
                                                            c->cl_half ? c->cl_of : nullptr, c->flags);
     c->launches += 3;
