@@ -33,25 +33,35 @@ namespace {
 
 constexpr int kG = 32;             // atoms per group
 constexpr int kN = 4 * kG;         // rows per block
-constexpr int kInvThreads = 256;
+constexpr int kInvThreads = 512;
+constexpr int kInvRows = kN * kN / kInvThreads / 4;  // rows of a warp
 
-// In-place Gauss-Jordan inversion with partial pivoting of the group's
-// block, FP64 in shared memory; one block per group.  A pivot below
-// 1e-13 of the block's largest entry falls back to the Jacobi inverse for
-// this group (never observed; it keeps a degenerate block harmless).
+// In-place Gauss-Jordan inversion with partial pivoting of the group's block
+// in FP64, one block per group.  The matrix lives in registers, warp w holding
+// rows 8 w .., lane l columns 4 l .. 4 l + 3: a pivot step then takes 4 reads of
+// column factors and 2 of the pivot row from shared memory for 32 multiply-adds
+// of a thread.  (Shared reads set the pace, a 16-byte one costing four cycles
+// even when all lanes read the same: 32 rows of one column per thread, 16 such
+// reads for the same 32, took 1.9 us a step; the whole matrix read and
+// rewritten in shared memory 4.4.  128 steps: 568 -> 247 -> 152 us a launch,
+// whatever the number of groups.)  Rows are not interchanged: row p_k serves as
+// pivot of column k and is marked used, and the result is stored permuted,
+// inverse[k][p_l] = B[p_k][l].  The pivot is the largest entry to 13 bits of
+// mantissa (the rest of a 32-bit key holds the row), which is as good a pivot.
+// A pivot below 1e-13 of the block's largest entry falls back to the Jacobi
+// inverse for this group (never observed; it keeps a degenerate block harmless).
 __global__ void __launch_bounds__(kInvThreads) k_block_inverse(DevParams P, const double4 *__restrict__ pos4,
                                                                const int *__restrict__ g_atoms, float *__restrict__ dinv)
 {
-    extern __shared__ double Dm[];  // kN * kN, row-major
-    __shared__ int piv[kN];
-    __shared__ double fcol[kN];
+    extern __shared__ __align__(16) double Dm[];  // kN * kN, row-major; then the inverse in FP32, rows of kN + 1
+    // the pivot column, twice: as it is, for the pivot search, and as the
+    // update's factors, where the pivot row's is replaced
+    __shared__ __align__(16) double colk[2][kN], fac[2][kN], prow[kN];
     __shared__ double wv[kInvThreads / 32];
-    __shared__ int wi[kInvThreads / 32];
-    __shared__ int bad;
-    __shared__ double amax;
-    const int G = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    __shared__ short piv[kN], row_of[kN];  // piv[k] = p_k, row_of[p_k] = k
+    const int G = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int w = __shfl_sync(0xffffffffu, tid >> 5, 0), row0 = w * kInvRows;
     const int *atoms = g_atoms + (size_t)G * kG;
-    if (tid == 0) bad = 0;
 
     // the block: diagonal terms and cpim_block for every ordered pair of the group
     for (int q = tid; q < kG * kG; q += blockDim.x) {
@@ -73,104 +83,112 @@ __global__ void __launch_bounds__(kInvThreads) k_block_inverse(DevParams P, cons
             for (int cc = 0; cc < 4; ++cc) Dm[(4 * a + r) * kN + 4 * b + cc] = e[4 * r + cc];
     }
     __syncthreads();
-    {
-        double m = 0.0;
-        for (int q = tid; q < kN * kN; q += blockDim.x) m = fmax(m, fabs(Dm[q]));
+    double a[kInvRows][4], amax = 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) wv[wid] = m;
-        __syncthreads();
-        if (tid == 0) {
-            double mm = 0.0;
-            for (int w = 0; w < kInvThreads / 32; ++w) mm = fmax(mm, wv[w]);
-            amax = mm;
+    for (int r = 0; r < kInvRows; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; c += 2) {
+            const double2 v = *reinterpret_cast<const double2 *>(Dm + (row0 + r) * kN + 4 * lane + c);
+            a[r][c] = v.x;
+            a[r][c + 1] = v.y;
+            amax = fmax(amax, fmax(fabs(v.x), fabs(v.y)));
         }
-        __syncthreads();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) {
+        wv[w] = amax;
+        double2 *u = reinterpret_cast<double2 *>(colk[0] + row0), *v = reinterpret_cast<double2 *>(fac[0] + row0);
+#pragma unroll
+        for (int r = 0; r < kInvRows; r += 2) u[r / 2] = v[r / 2] = make_double2(a[r][0], a[r + 1][0]);
     }
+    __syncthreads();
+    for (int q = 0; q < kInvThreads / 32; ++q) amax = fmax(amax, wv[q]);
     const double tiny = 1e-13 * amax;
 
-    for (int k = 0; k < kN; ++k) {
-        // pivot: largest |D[i][k]|, i >= k (lowest i on ties)
-        double v = -1.0;
-        int vi = kN;
-        if (tid >= k && tid < kN) {
-            v = fabs(Dm[tid * kN + k]);
-            vi = tid;
-        }
+    bool bad = false;
+    unsigned used = 0;  // of rows lane, lane + 32, ..: every warp keeps its own copy
+    for (int k4 = 0; k4 < kN && !bad; k4 += 4) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-            const int i2 = __shfl_xor_sync(0xffffffffu, vi, o);
-            if (v2 > v || (v2 == v && i2 < vi)) {
-                v = v2;
-                vi = i2;
+        for (int kk = 0; kk < 4; ++kk) {  // column kk of lane k4 / 4
+            const int k = k4 + kk;
+            const double *col = colk[kk & 1];
+            double *f = fac[kk & 1];
+            unsigned key = 0;
+#pragma unroll
+            for (int q = 0; q < kN / 32; ++q) {
+                const int i = lane + 32 * q;
+                const unsigned h = (unsigned)__double2hiint(fabs(col[i]));
+                if (!((used >> q) & 1u)) key = max(key, (h & ~(unsigned)(kN - 1)) | (unsigned)(kN - 1 - i));
             }
-        }
-        if (lane == 0) {
-            wv[wid] = v;
-            wi[wid] = vi;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double bv = -1.0;
-            int bi = kN;
-            for (int w = 0; w < kInvThreads / 32; ++w)
-                if (wv[w] > bv || (wv[w] == bv && wi[w] < bi)) {
-                    bv = wv[w];
-                    bi = wi[w];
+            const int p = kN - 1 - (int)(__reduce_max_sync(0xffffffffu, key) & (unsigned)(kN - 1));
+            const double d = col[p];
+            bad = !(fabs(d) > tiny);  // the same in every thread
+            if (bad) break;
+            if ((p & 31) == lane) used |= 1u << (p >> 5);
+            const int pl = p - row0;  // the pivot row among this warp's
+            // the pivot column becomes the unit vector of the pivot row
+            if (lane == k4 / 4)
+#pragma unroll
+                for (int r = 0; r < kInvRows; ++r) a[r][kk] = r == pl ? 1.0 : 0.0;
+            if ((unsigned)pl < (unsigned)kInvRows) {
+                // the pivot row, before its division, from the warp that holds it
+                double v[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    v[c] = a[0][c];
+#pragma unroll
+                    for (int r = 1; r < kInvRows; ++r) v[c] = r == pl ? a[r][c] : v[c];
                 }
-            piv[k] = bi;
-            if (!(bv > tiny) || bi >= kN) bad = 1;
-        }
-        __syncthreads();
-        if (bad) break;
-        const int p = piv[k];
-        if (p != k)
-            for (int j = tid; j < kN; j += blockDim.x) {
-                const double t = Dm[k * kN + j];
-                Dm[k * kN + j] = Dm[p * kN + j];
-                Dm[p * kN + j] = t;
+                double2 *u = reinterpret_cast<double2 *>(prow + 4 * lane);
+                u[0] = make_double2(v[0], v[1]);
+                u[1] = make_double2(v[2], v[3]);
+                if (lane == 0) {
+                    piv[k] = (short)p;
+                    row_of[p] = (short)k;
+                    f[p] = d - 1.0;  // v - (d - 1) v / d = v / d
+                }
             }
-        __syncthreads();
-        const double inv = 1.0 / Dm[k * kN + k];
-        for (int i = tid; i < kN; i += blockDim.x) fcol[i] = i == k ? 0.0 : Dm[i * kN + k];
-        __syncthreads();
-        for (int j = tid; j < kN; j += blockDim.x) Dm[k * kN + j] = (j == k ? 1.0 : Dm[k * kN + j]) * inv;
-        __syncthreads();
-        for (int q = tid; q < kN * kN; q += blockDim.x) {
-            const int i = q / kN, j = q % kN;
-            if (i == k) continue;
-            const double base = j == k ? 0.0 : Dm[q];
-            Dm[q] = fma(-fcol[i], Dm[k * kN + j], base);
-        }
-        __syncthreads();
-    }
-    if (!bad) {
-        // undo the row interchanges as column interchanges, last first
-        for (int k = kN - 1; k >= 0; --k) {
-            const int p = piv[k];
-            if (p != k)
-                for (int i = tid; i < kN; i += blockDim.x) {
-                    const double t = Dm[i * kN + k];
-                    Dm[i * kN + k] = Dm[i * kN + p];
-                    Dm[i * kN + p] = t;
+            const double inv = 1.0 / d;
+            __syncthreads();
+            const double2 p0 = *reinterpret_cast<const double2 *>(prow + 4 * lane);
+            const double2 p1 = *reinterpret_cast<const double2 *>(prow + 4 * lane + 2);
+            const double rj[4] = {p0.x * inv, p0.y * inv, p1.x * inv, p1.y * inv};
+#pragma unroll
+            for (int r = 0; r < kInvRows; r += 2) {
+                const double2 g = *reinterpret_cast<const double2 *>(f + row0 + r);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    a[r][c] = fma(-g.x, rj[c], a[r][c]);
+                    a[r + 1][c] = fma(-g.y, rj[c], a[r + 1][c]);
                 }
+            }
+            if (k + 1 < kN && lane == (k + 1) / 4) {
+                double2 *u = reinterpret_cast<double2 *>(colk[(kk + 1) & 1] + row0);
+                double2 *v = reinterpret_cast<double2 *>(fac[(kk + 1) & 1] + row0);
+#pragma unroll
+                for (int r = 0; r < kInvRows; r += 2)
+                    u[r / 2] = v[r / 2] = make_double2(a[r][(kk + 1) & 3], a[r + 1][(kk + 1) & 3]);
+            }
             __syncthreads();
         }
     }
-    float *out = dinv + (size_t)G * kN * kN;
-    for (int q = tid; q < kN * kN; q += blockDim.x) {
-        const int c = q / kN, o = q % kN;  // out[c][o] = inverse[o][c]
-        float val;
-        if (!bad) {
-            val = (float)Dm[o * kN + c];
-        } else {  // Jacobi for this group
-            const int a = o >> 2, comp = o & 3;
-            const double d = atoms[a] < 0 ? 1.0 : (comp < 3 ? P.inv_polar : -P.inv_capac);
-            val = c == o ? (float)(1.0 / d) : 0.0f;
+    float *S = reinterpret_cast<float *>(Dm);
+    __syncthreads();
+    if (!bad) {
+#pragma unroll
+        for (int r = 0; r < kInvRows; ++r)  // out[c][o] = inverse[o][c], o = row_of[i], c = piv[j]
+#pragma unroll
+            for (int c = 0; c < 4; ++c) S[piv[4 * lane + c] * (kN + 1) + row_of[row0 + r]] = (float)a[r][c];
+    } else {  // Jacobi for this group
+        for (int q = tid; q < kN * kN; q += blockDim.x) {
+            const int c = q / kN, o = q % kN, at = o >> 2, comp = o & 3;
+            const double d = atoms[at] < 0 ? 1.0 : (comp < 3 ? P.inv_polar : -P.inv_capac);
+            S[c * (kN + 1) + o] = c == o ? (float)(1.0 / d) : 0.0f;
         }
-        out[q] = val;
     }
+    __syncthreads();
+    float *out = dinv + (size_t)G * kN * kN;
+    for (int q = tid; q < kN * kN; q += blockDim.x) out[q] = S[q / kN * (kN + 1) + q % kN];
 }
 
 // Interleave the low 21 bits of v with two zero bits after each (Morton key).
