@@ -245,10 +245,11 @@ struct capac_ctx {
     int cz_nc = 0;               // coarse columns: cz_modes per group and one per nanoparticle
     int cz_modes = 1;            // 1: the group's charge sum; 4: its dipole sums and charge sum
     float *cz_az = nullptr;      // A Z
-    float *cz_w = nullptr;       // (A Z) E^-1
+    float *cz_w = nullptr;       // W = (A Z) E^-1
+    float *cz_kw = nullptr;      // K W, with the current inverse blocks
     float *cz_einv = nullptr;    // E^-1
     double *cz_aug = nullptr;    // [E | I] workspace of the inversion
-    double *cz_zbuf = nullptr;   // Z^T v inside the solver
+    double *cz_zbuf = nullptr;   // Z^T v inside the solver, by quarters of the groups
     int cz_cluster = 0;          // CTAs of the last inversion's cluster (1: one block)
     bool cz_one_block = false;   // invert in one block (CAPAC_COARSE_ONE_BLOCK at creation)
     long inner_stalls = 0;       // inner solves ended that way
@@ -364,6 +365,7 @@ int coarse_columns(int M, int n_nps, int modes);
 int coarse_columns_max();  // the most coarse columns the solver holds
 size_t coarse_az_floats(int M, int n_nps, int modes);
 void launch_coarse_refresh(capac_ctx *c);
+void launch_coarse_kw(capac_ctx *c);  // K W, after either of K and W has changed
 size_t group_rows(int M, int n_nps);
 int group_grid_size(int device, bool hold);
 int group_blocks_per_sm(int device, bool hold);

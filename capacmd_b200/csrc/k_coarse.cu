@@ -19,7 +19,8 @@
 // couplings.  E sums A Z over each group's rows; E^-1 by Gauss-Jordan with
 // partial pivoting in FP64 in one block.
 //
-// W = (A Z) E^-1, in the layout of A Z, is what the solver reads.
+// W = (A Z) E^-1 and K W, in the layout of A Z, are what the solver reads (K W
+// is formed again with every refresh of the inverse blocks).
 // Layout (group g's columns at nm g ..): az[(g * nc + j) * 128 + r] for internal row 128 g + r (column
 // j contiguous over the group's rows), then az[128 nG nc + k * nc + j] for
 // constraint row k; einv[j * nc + i] = (E^-1)[i][j] (E is symmetric).
@@ -452,6 +453,36 @@ __global__ void __launch_bounds__(128) k_coarse_w(int nG, int nc, int n_nps, con
     }
 }
 
+// K W (the layout of W), K the inverse blocks dinv[g][c][o]: block (g, 32
+// columns), thread r one row of group g, the columns of W staged in shared
+// memory 32 rows at a time.
+__global__ void __launch_bounds__(128) k_coarse_kw(int nc, const float *__restrict__ dinv, const float *__restrict__ w,
+                                                   float *__restrict__ kw)
+{
+    __shared__ float ws[32][33];  // [column][row of the chunk]
+    const int g = blockIdx.x, j0 = blockIdx.y * 32, r = threadIdx.x;
+    float acc[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) acc[q] = 0.f;
+    for (int c0 = 0; c0 < kRows; c0 += 32) {
+        __syncthreads();
+        for (int q = threadIdx.x; q < 32 * 32; q += blockDim.x) {
+            const int jj = q >> 5, cc = q & 31;
+            ws[jj][cc] = j0 + jj < nc ? w[((size_t)g * nc + j0 + jj) * kRows + c0 + cc] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int cc = 0; cc < 32; ++cc) {
+            const float k = dinv[((size_t)g * kRows + c0 + cc) * kRows + r];
+#pragma unroll
+            for (int q = 0; q < 32; ++q) acc[q] = fmaf(k, ws[q][cc], acc[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 32; ++q)
+        if (j0 + q < nc) kw[((size_t)g * nc + j0 + q) * kRows + r] = acc[q];
+}
+
 }  // namespace
 
 int coarse_columns(int M, int n_nps, int nm) { return nm * precond_groups(M) + n_nps; }
@@ -504,6 +535,14 @@ void launch_coarse_invert(capac_ctx *c, int nc)
     }
     c->cz_cluster = 1;
     k_coarse_invert<<<1, kInvThreads, 0, c->stream>>>(nc, c->cz_aug, c->cz_einv, c->flags + 6);
+}
+
+void launch_coarse_kw(capac_ctx *c)
+{
+    const int nG = precond_groups(c->M), nc = coarse_columns(c->M, c->n_nps, c->cz_modes);
+    ProfScope ps(c, K_MATRIX);
+    k_coarse_kw<<<dim3(nG, (nc + 31) / 32), kRows, 0, c->stream>>>(nc, c->dinv, c->cz_w, c->cz_kw);
+    ++c->launches;
 }
 
 void launch_coarse_refresh(capac_ctx *c)

@@ -271,6 +271,7 @@ void launch_cpim_matrix(capac_ctx *c)
             launch_block_inverse(c);
             if (c->twolevel && c->precond_age <= 1) c->coarse_age = 0;  // fresh positions: fresh coarse part
             if (c->twolevel && c->coarse_age++ % kCoarseEvery == 0) launch_coarse_refresh(c);
+            if (c->twolevel && !c->dense_ex) launch_coarse_kw(c);
         }
         return;
     }

@@ -1009,8 +1009,8 @@ struct GroupArgs {
     int stall;                   // > 0: stop (status 1) after this many iterations without halving (r, r)
     int nc;                      // > 0: the two-level operator with nc coarse columns (k_coarse.cu)
     int nm;                      // coarse columns per group: 1 (charge) or 4 (dipole x, y, z, charge)
-    const float *w, *einv;       // (A Z) E^-1 and E^-1 of the coarse space
-    double *zbuf;                // Z^T of the vector being preconditioned (nc)
+    const float *w, *kw, *einv;  // W = (A Z) E^-1, K W and E^-1 of the coarse space
+    double *zbuf;                // Z^T of the vector being preconditioned, by quarters of the groups (4 nc)
     long spin_limit;
     double inv_polar, inv_capac;
     const int *g_atoms;          // [32 nG] metal-local atom of each slot, -1 padding
@@ -1370,65 +1370,75 @@ __device__ void reduce_group(const GroupArgs &A, const PassScalars &S, double *b
 constexpr int kCoarseMax = 384;  // coarse columns the solver's shared buffer holds
 
 // The reductions of reduce_group with the two-level operator of k_coarse.cu
-// in place of the block-Jacobi K alone: first every group's rows of `out`
-// (v, t or r), the dots that do not involve K out, and the group's four mode
-// sums (and the constraint rows) into zbuf; a grid barrier; then in every
-// block c = E^-1 zbuf, and for its groups K out = Z c + K (out - (A Z) c)
-// with the dots of K out.  Returns false when the grid barrier gave up.
-// scratch: 256 + 2 kCoarseMax doubles of shared memory (the pass inputs'
-// buffer, idle between passes).
+// in place of the block-Jacobi K alone: first the rows of `out` (v, t or r),
+// the dots that do not involve K out, and the mode sums (and the constraint
+// rows) into zbuf; a grid barrier; then K out = Z c + K out - (K W) zbuf,
+// c = E^-1 zbuf, with the dots of K out.  Returns false when the grid barrier
+// gave up.  scratch: 256 + 2 kCoarseMax doubles of shared memory (the pass
+// inputs' buffer, idle between passes).
+//
+// A work item is a quarter of a group, 32 rows, so that 4 nG blocks share
+// the two steps (36 groups, 144 of 148 blocks; 65 groups, 260 of 296): they are
+// chains of loads from L2 whose length is what a block reads.  K W is formed
+// with the preconditioner (k_coarse.cu), since a quarter cannot form K (out -
+// W zbuf) of its rows without the whole group's.  The second step took 7.1 and
+// 7.5 us of 40.8 per iteration with one block per group (1,122 atoms), 9.7 and
+// 10.3 of 69.5 (2,057); now 4.5 and 5.0, 5.4 and 6.4.
 template <int RED>
 __device__ bool reduce_group2(const GroupArgs &A, const PassScalars &S, double *bp, bool products, double *scratch,
                               int iter = 0, int mark = -1)
 {
-    double *vrow = scratch, *hsum = scratch + 128, *cc = scratch + 256, *zs = scratch + 256 + kCoarseMax;
-    const int nG = A.nG, nc = A.nc, tid = threadIdx.x;
+    // vq: mode sums of the step's 8 atoms; vs: the group's rows of out; ps:
+    // partial sums of the warps; cc, zs: c of the group's columns, Z^T out
+    double *vq = scratch, *vs = scratch + 32, *ps = scratch + 160, *cc = scratch + 416, *zs = scratch + 420;
+    static_assert(420 + kCoarseMax <= 256 + 2 * kCoarseMax, "the scratch holds the step's arrays");
+    const int nG = A.nG, nc = A.nc, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const double *in = RED == RED_START ? A.xi : (RED == RED_V ? A.yb[S.cur ^ 1] : A.z);
     double *outv = RED == RED_START ? A.r : (RED == RED_V ? A.v : A.t);
     double *kout = RED == RED_START ? A.Kr : (RED == RED_V ? A.Kv : A.Kt);
     double d[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int G = blockIdx.x; G < nG; G += gridDim.x) {
-        const int o = tid & 127, h = tid >> 7;
+    for (int it = blockIdx.x; it < 4 * nG; it += gridDim.x) {
+        // warp wid: one atom; lane: component lane / 8, every eighth partial
+        const int G = it >> 2, quarter = it & 3, o = 32 * quarter + 4 * wid + (lane >> 3), part = lane & 7;
+        const int row = 128 * G + o, comp = lane >> 3;
+        // the row's other operands, loaded beside the partials
+        const double xin = products ? __ldcg(in + row) : 0.0;
+        const double r0 = RED == RED_START ? 0.0 : __ldcg(A.r0 + row);
+        const double sr = RED == RED_T ? __ldcg(A.s + row) : 0.0;
+        const bool valid = A.g_atoms[row >> 2] >= 0;
         double sum = 0.0;
         if (products) {
             const double *src = A.part + (size_t)G * nG * (kT * 4) + o;
-            for (int K0 = h; K0 < nG; K0 += 2 * kBatch) {
+            for (int K0 = part; K0 < nG; K0 += 8 * kBatch) {
                 double vals[kBatch];
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) {
-                    const int Kk = K0 + 2 * u;
+                    const int Kk = K0 + 8 * u;
                     vals[u] = Kk < nG ? __ldcg(src + (size_t)Kk * (kT * 4)) : 0.0;
                 }
 #pragma unroll
                 for (int u = 0; u < kBatch; ++u) sum += vals[u];
             }
         }
-        if (h == 1) hsum[o] = sum;
-        __syncthreads();
-        if (h == 0) {
-            const int row = 128 * G + o;
-            sum += hsum[o];
-            const double xin = products ? __ldcg(in + row) : 0.0;
-            if ((o & 3) < 3) {
+#pragma unroll
+        for (int m = 1; m < 8; m *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+        if (part == 0) {
+            if (comp < 3) {
                 sum += A.inv_polar * xin;
             } else {
                 sum += -A.inv_capac * xin;
                 const int k = A.slot_np[row >> 2];
                 if (products && k >= 0) sum += __ldcg(in + 128 * nG + k);
             }
-            double out;
+            double out = sum;
             if (RED == RED_START) {
                 const int rr = g_ref_row(A, row);
-                const double bk = rr >= 0 ? A.b[rr] : 0.0;
-                out = bk - sum;
+                out = (rr >= 0 ? A.b[rr] : 0.0) - sum;
                 A.r0[row] = out;
                 d[0] += out * out;
             } else if (RED == RED_V) {
-                out = sum;
-                d[0] += __ldcg(A.r0 + row) * out;
+                d[0] += r0 * out;
             } else {
-                out = sum;
-                const double sr = __ldcg(A.s + row), r0 = __ldcg(A.r0 + row);
                 d[2] += r0 * sr;
                 d[3] += r0 * out;
                 d[4] += sr * sr;
@@ -1436,14 +1446,15 @@ __device__ bool reduce_group2(const GroupArgs &A, const PassScalars &S, double *
                 d[6] += out * out;
             }
             outv[row] = out;
-            vrow[o] = A.g_atoms[row >> 2] >= 0 ? out : 0.0;
+            vq[4 * wid + comp] = valid ? out : 0.0;
         }
         __syncthreads();
-        if (tid < A.nm) {  // the group's mode sums (padding rows hold zero)
+        if (tid < A.nm) {  // the quarter's mode sums (padding rows hold zero)
             const int c = A.nm == 4 ? tid : 3;
-            double zs = 0.0;
-            for (int a = 0; a < kT; ++a) zs += vrow[4 * a + c];
-            A.zbuf[A.nm * G + tid] = zs;
+            double z = 0.0;
+#pragma unroll
+            for (int a = 0; a < kWarps; ++a) z += vq[4 * a + c];
+            A.zbuf[quarter * nc + A.nm * G + tid] = z;
         }
         __syncthreads();
     }
@@ -1473,70 +1484,73 @@ __device__ bool reduce_group2(const GroupArgs &A, const PassScalars &S, double *
             }
             outv[row] = out;
             A.zbuf[A.nm * nG + k] = out;
+            for (int q = 1; q < 4; ++q) A.zbuf[q * nc + A.nm * nG + k] = 0.0;
         }
         __syncthreads();
     }
     if (!grid_barrier(A.sync, A.spin_limit)) return false;
     if (mark >= 0) g_phase_mark(A, iter, mark);  // the phase timer splits the two steps
 
-    const int lane = tid & 31, wid = tid >> 5;
-    const bool mine = (int)blockIdx.x < nG || (int)gridDim.x - 1 - (int)blockIdx.x < A.n_nps;
+    const bool mine = (int)blockIdx.x < 4 * nG || (int)gridDim.x - 1 - (int)blockIdx.x < A.n_nps;
     if (mine) {
-        for (int j = tid; j < nc; j += blockDim.x) zs[j] = __ldcg(A.zbuf + j);
-        __syncthreads();
+        for (int j = tid; j < nc; j += blockDim.x)
+            zs[j] = (__ldcg(A.zbuf + j) + __ldcg(A.zbuf + nc + j)) +
+                    (__ldcg(A.zbuf + 2 * nc + j) + __ldcg(A.zbuf + 3 * nc + j));
     }
-    for (int G = blockIdx.x; G < nG; G += gridDim.x) {
-        const int o = tid & 127, h = tid >> 7;
+    for (int it = blockIdx.x; it < 4 * nG; it += gridDim.x) {
+        const int G = it >> 2, quarter = it & 3, o = 32 * quarter + lane, row = 128 * G + o;
+        // warp wid: 16 of K's columns and every eighth column of K W, for the 32
+        // rows of the quarter (lane)
+        const float *col = A.dinv + ((size_t)G * 128 + 16 * wid) * 128 + o;
+        float kv[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) kv[c] = __ldg(col + (size_t)c * 128);
+        if (tid < 128) vs[tid] = __ldcg(outv + 128 * G + tid);
+        __syncthreads();  // zs, vs
         // c of the group's own columns: warp m, lanes over the columns of
         // row nm G + m of E^-1
         if (wid < A.nm) {
             const float *er = A.einv + (size_t)(A.nm * G + wid) * nc;
             double s = 0.0;
             for (int j = lane; j < nc; j += 32) s = fma((double)__ldg(er + j), zs[j], s);
-#pragma unroll
-            for (int m = 16; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+            s = warp_sum(s);
             if (lane == 0) cc[wid] = s;
         }
-        // (A Z c) of the group's rows = W zbuf: two halves of the columns
-        const float *wg = A.w + (size_t)G * nc * 128 + o;
+        const float *kw = A.kw + (size_t)G * nc * 128 + o;
         double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        int j = h;
-        for (; j + 6 < nc; j += 8) {
-            s0 = fma((double)__ldg(wg + (size_t)j * 128), zs[j], s0);
-            s1 = fma((double)__ldg(wg + (size_t)(j + 2) * 128), zs[j + 2], s1);
-            s2 = fma((double)__ldg(wg + (size_t)(j + 4) * 128), zs[j + 4], s2);
-            s3 = fma((double)__ldg(wg + (size_t)(j + 6) * 128), zs[j + 6], s3);
+        int j = wid;
+        for (; j + 7 * kWarps < nc; j += 8 * kWarps) {
+            float q[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) q[u] = __ldg(kw + (size_t)(j + u * kWarps) * 128);
+#pragma unroll
+            for (int u = 0; u < 8; u += 2) {
+                s0 = fma((double)q[u], zs[j + u * kWarps], s0);
+                s1 = fma((double)q[u + 1], zs[j + (u + 1) * kWarps], s1);
+            }
         }
-        for (; j < nc; j += 2) s0 = fma((double)__ldg(wg + (size_t)j * 128), zs[j], s0);
-        const double s = (s0 + s1) + (s2 + s3);
-        if (h == 1) hsum[o] = s;
-        __syncthreads();
-        if (h == 0) {
-            const int row = 128 * G + o;
-            const bool valid = A.g_atoms[row >> 2] >= 0;
-            vrow[o] = valid ? __ldcg(outv + row) - (s + hsum[o]) : 0.0;
+        for (; j < nc; j += kWarps) s0 = fma((double)__ldg(kw + (size_t)j * 128), zs[j], s0);
+#pragma unroll
+        for (int c = 0; c < 16; c += 2) {
+            s2 = fma((double)kv[c], vs[16 * wid + c], s2);
+            s3 = fma((double)kv[c + 1], vs[16 * wid + c + 1], s3);
         }
+        ps[32 * wid + lane] = (s2 + s3) - (s0 + s1);
         __syncthreads();
-        // K w with the group's inverse block, plus Z c
-        {
-            const int o2 = tid >> 1, half = tid & 1;
-            const float *col = A.dinv + (size_t)G * 128 * 128 + (size_t)(64 * half) * 128 + o2;
+        if (wid == 0) {
             double acc = 0.0;
-#pragma unroll 16
-            for (int c = 0; c < 64; ++c) acc = fma((double)__ldg(col + (size_t)c * 128), vrow[64 * half + c], acc);
-            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-            if (half == 0) {
-                const int row = 128 * G + o2;
-                if (A.g_atoms[row >> 2] >= 0 && (A.nm == 4 || (o2 & 3) == 3)) acc += cc[A.nm == 4 ? (o2 & 3) : 0];
-                kout[row] = acc;
-                if (RED == RED_T) {
-                    d[0] += acc * __ldcg(A.z + row);
-                    d[1] += acc * acc;
-                }
+#pragma unroll
+            for (int q = 0; q < kWarps; ++q) acc += ps[32 * q + lane];
+            if (A.g_atoms[row >> 2] >= 0 && (A.nm == 4 || (o & 3) == 3)) acc += cc[A.nm == 4 ? (o & 3) : 0];
+            kout[row] = acc;
+            if (RED == RED_T) {
+                d[0] += acc * __ldcg(A.z + row);
+                d[1] += acc * acc;
             }
         }
         __syncthreads();
     }
+    if (mine) __syncthreads();  // zs, for a block without a quarter
     for (int k = (int)gridDim.x - 1 - (int)blockIdx.x; k < A.n_nps; k += gridDim.x) {
         // the whole block over the coarse columns, two per thread at most
         __shared__ double shc[2 * kWarps];
@@ -1941,6 +1955,7 @@ int bicgstab_group(capac_ctx *c, const double *b, double *x, double tol, double 
     A.nc = c->twolevel ? c->cz_nc : 0;
     A.nm = c->cz_modes;
     A.w = c->cz_w;
+    A.kw = c->cz_kw;
     A.einv = c->cz_einv;
     A.zbuf = c->cz_zbuf;
     A.spin_limit = c->opt.wait_polls > 0 ? c->opt.wait_polls : kSpinLimit;
