@@ -36,51 +36,70 @@ void check_ctx(capac_ctx *c)
     if (!c) throw Error(CAPAC_ERR_INVALID, "null context");
 }
 
+// Throws when a solve whose status has landed did not converge.
+void settle(capac_ctx *c)
+{
+    const int st = settle_solve(c);
+    if (st == CAPAC_OK) return;
+    c->grad_ready = false;
+    char msg[160];
+    snprintf(msg, sizeof msg, "Error: bicg_stab not converged. rTr= %e, bTb= %e", c->h_ss->rTr, c->h_ss->bTb);
+    throw Error(st, msg);
+}
+
+// Waits for the stream; throws the failures of RATTLE and of a pending solve.
 void check_flags(capac_ctx *c)
 {
     CAPAC_CUDA(cudaMemcpyAsync(c->h_flags, c->flags, sizeof(int) * 4, cudaMemcpyDeviceToHost, c->stream));
     CAPAC_CUDA(cudaStreamSynchronize(c->stream));
-    if (c->h_flags[2]) {
-        const bool first = c->h_flags[2] & 1;
-        CAPAC_CUDA(cudaMemsetAsync(c->flags + 2, 0, sizeof(int), c->stream));
-        throw Error(CAPAC_ERR_RATTLE, first ? "RATTLE_1 not converged!" : "RATTLE_2 not converged!");
-    }
+    settle(c);
+    check_rattle(c);
 }
 
 void record(capac_ctx *c, int k) { CAPAC_CUDA(cudaEventRecord(c->ev[k], c->stream)); }
 
 // One mpi_force equivalent on the device state; solve = false keeps the
-// induced vector as it is.
+// induced vector as it is.  The host waits once, for the displacement check
+// (and the previous call's solve, whose status is read there): the Sutton-Chen
+// and matrix kernels, which need no list, are queued before.  The caller waits
+// for this call's own status (check_flags) unless another force call follows.
 void force(capac_ctx *c, bool solve = true)
 {
     cudaStream_t s = c->stream;
     c->grad_ready = false;
+    struct Defer {  // the launches' sums are left to launch_force_sums
+        capac_ctx *c;
+        explicit Defer(capac_ctx *cc) : c(cc)
+        {
+            c->defer = true;
+            c->fs = ForceSums{};
+        }
+        ~Defer() { c->defer = false; }
+    } defer(c);
     record(c, 0);
     launch_build_vsites(c);  // build_vsites before everything (force.c:2124-2129)
-    launch_list_maintenance(c, false);
-    launch_pack_positions(c);
-    CAPAC_CUDA(cudaMemsetAsync(c->fx, 0, sizeof(double) * c->N, s));
-    CAPAC_CUDA(cudaMemsetAsync(c->fy, 0, sizeof(double) * c->N, s));
-    CAPAC_CUDA(cudaMemsetAsync(c->fz, 0, sizeof(double) * c->N, s));
-    CAPAC_CUDA(cudaMemsetAsync(c->pot, 0, sizeof(double) * 15, s));
-    CAPAC_CUDA(cudaMemsetAsync(c->vir, 0, sizeof(double) * 9, s));
+    launch_begin_force(c);
     record(c, 1);
     const bool cpim = c->M > 0 && c->use_cpff;
     launch_bonded(c);
     if (c->M > 0) launch_qsc(c);
+    record(c, 2);
+    if (cpim) launch_cpim_matrix(c);
+    record(c, 3);
+    finish_begin_force(c);
+    settle(c);
     // the nonbonded pairs (their own stream) meanwhile with the CPIM stages
     const bool ovl = c->overlap && cpim && solve && c->clusters && c->cl_half;
     if (ovl) launch_pair_nonbonded_async(c);
-    record(c, 2);
+    record(c, 8);
     int st = CAPAC_OK;
     try {
         if (cpim) launch_cpim_rhs(c);
-        record(c, 3);
-        if (cpim) launch_cpim_matrix(c);
         record(c, 4);
-        if (cpim && solve) st = c->opt.precision == CAPAC_PREC_MIXED ? run_refined_solve(c) : run_bicgstab(c);
+        if (cpim && solve)
+            st = c->opt.precision == CAPAC_PREC_MIXED ? run_refined_solve(c, true) : run_bicgstab(c, true);
     } catch (...) {
-        if (ovl) cudaStreamWaitEvent(c->stream, c->ev_join, 0);  // nothing left running on stream2
+        if (ovl) cudaStreamWaitEvent(s, c->ev_join, 0);  // nothing left running on stream2
         throw;
     }
     record(c, 5);
@@ -91,6 +110,7 @@ void force(capac_ctx *c, bool solve = true)
     record(c, 6);
     if (cpim) launch_cpim_metal_forces(c);
     launch_external_field(c);
+    launch_force_sums(c);
     launch_vsite_forces(c);  // mpi_vsites after all force terms (force.c:2290-2296)
     record(c, 7);
     if (st != CAPAC_OK) {
@@ -105,26 +125,13 @@ void md_step(capac_ctx *c)
 {
     const long step = ++c->md_step;
     const bool nvt = c->ensemble == CAPAC_NVT;
-    launch_heating(c, step);
-    if (nvt) launch_nhc(c);
-    launch_md_half_kick(c, nvt);
-    launch_md_drift(c);
+    if (nvt) launch_nhc(c, step);
+    launch_md_kick_drift(c, nvt, step);
     launch_rattle(c, 0);
     force(c);
-    check_flags(c);
-    launch_sum_potential(c);
-    launch_md_half_kick(c, false);
-    launch_rattle(c, 1);
-    launch_kinetic(c);
-    if (nvt) {
-        launch_nhc(c);
-        launch_scale_velocities(c);
-    } else if (c->ensemble == CAPAC_BERENDSEN) {
-        launch_berendsen(c);
-        launch_scale_velocities(c);
-    }
-    launch_remove_com(c);
-    launch_kinetic(c);
+    launch_md_half_kick(c);
+    launch_rattle(c, 1, true);
+    launch_step_sums(c, c->ensemble, c->has_cstr);
     if (step % c->n_save == 0) {
         launch_apply_pbc(c);
         launch_fmax_rms(c);
@@ -158,6 +165,15 @@ double *state_array(capac_ctx *c, const std::string &n, int *count)
 }  // namespace
 
 void set_last_error(const std::string &msg) { g_last_error = msg; }
+
+void check_rattle(capac_ctx *c)
+{
+    if (!c->h_flags[2]) return;
+    const bool first = c->h_flags[2] & 1;
+    c->h_flags[2] = 0;
+    CAPAC_CUDA(cudaMemsetAsync(c->flags + 2, 0, sizeof(int), c->stream));
+    throw Error(CAPAC_ERR_RATTLE, first ? "RATTLE_1 not converged!" : "RATTLE_2 not converged!");
+}
 
 constexpr int kProfSlots = 4096;
 
@@ -587,6 +603,11 @@ int capac_create(const capac_desc *d, const capac_options *opt, capac_ctx **out)
 
             c->partials_cap = partials_needed(c);
             c->partials = dalloc<double>(c->partials_cap);
+            c->fpart = dalloc<double>(force_partial_areas(c, c->fpart_off));
+            c->spart = dalloc<double>((size_t)kSumBlocks * 8);
+            c->scount = dalloc<int>(2);
+            CAPAC_CUDA(cudaMemsetAsync(c->scount, 0, sizeof(int) * 2, s));
+            CAPAC_CUDA(cudaEventCreateWithFlags(&c->ev_flags, cudaEventDisableTiming));
             if (const char *ps = getenv("CAPAC_PAIR_SPLIT")) c->pair_split_force = ps[0] == '0' ? 0 : 1;
             if (o.precision == CAPAC_PREC_MIXED && d->n_metal > 0 && d->use_cpff && getenv("CAPAC_OVERLAP")) {
                 c->overlap = true;
@@ -644,7 +665,7 @@ int capac_destroy(capac_ctx *c)
                    c->cl_nbr, c->cl_nnb, c->cl_metal, c->cl_of, c->cl_next, c->cl_sel, c->n_cl_sel, c->partials2,
                    c->cp_list,
                    c->cp_n, c->cp_cent, c->cp_off, c->cp_ti, c->cz_az, c->cz_w, c->cz_kw, c->cz_einv, c->cz_aug, c->cz_zbuf, c->scan_tmp, c->isd, c->vec_ext, c->vec_pq,
-                   c->diag, c->mat, c->matf, c->msym, c->sympart, c->dense_ex, c->coop_bp, c->coop_bar, c->g_atoms, c->dinv, c->slot_np, c->np_off, c->np_rows, c->gvec, c->gw, c->em_buf, c->phase_buf, c->rres, c->dcorr, c->xprev, c->bw, c->bwf, c->ss, c->partials, c->pot, c->vir, c->th};
+                   c->diag, c->mat, c->matf, c->msym, c->sympart, c->dense_ex, c->coop_bp, c->coop_bar, c->g_atoms, c->dinv, c->slot_np, c->np_off, c->np_rows, c->gvec, c->gw, c->em_buf, c->phase_buf, c->rres, c->dcorr, c->xprev, c->bw, c->bwf, c->ss, c->partials, c->fpart, c->spart, c->scount, c->pot, c->vir, c->th};
     for (void *p : dev)
         if (p) cudaFree(p);
     for (void *p : c->bonded_buffers)
@@ -661,6 +682,7 @@ int capac_destroy(capac_ctx *c)
         for (auto &e : g.ev)
             if (e) cudaEventDestroy(e);
     }
+    if (c->ev_flags) cudaEventDestroy(c->ev_flags);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->stream2) cudaStreamDestroy(c->stream2);
@@ -888,9 +910,7 @@ int capac_md_init(capac_ctx *c)
         check_ctx(c);
         force(c);
         check_flags(c);
-        launch_sum_potential(c);
-        launch_remove_com(c);
-        launch_kinetic(c);
+        launch_step_sums(c, CAPAC_NVE, false);
         CAPAC_CUDA(cudaMemcpyAsync(c->h_th, c->th, sizeof(ThermoState), cudaMemcpyDeviceToHost, c->stream));
         CAPAC_CUDA(cudaStreamSynchronize(c->stream));
         c->h_th->first_temp = c->h_th->inst_temp;
@@ -1279,10 +1299,10 @@ int capac_phase_times(capac_ctx *c, double out_ms[15])
             if (cudaEventElapsedTime(&ms, c->ev[a], c->ev[b]) != cudaSuccess) return 0.0;
             return (double)ms;
         };
-        out_ms[10] = span(0, 1);  // list maintenance and packing
+        out_ms[10] = span(0, 1) + span(3, 8);  // packing and list maintenance
         out_ms[1] = span(1, 2);   // Sutton-Chen density + force
-        out_ms[6] = span(2, 3);   // CPIM vector
-        out_ms[5] = span(3, 4);   // CPIM matrix
+        out_ms[5] = span(2, 3);   // CPIM matrix
+        out_ms[6] = span(8, 4);   // CPIM vector
         out_ms[7] = span(4, 5);   // CPIM solve
         out_ms[4] = span(5, 6);   // nonbonded (+ water side of CPIM)
         out_ms[8] = span(6, 7);   // CPIM force, external field

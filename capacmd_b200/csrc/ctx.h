@@ -58,6 +58,13 @@ struct DevParams {
     int metal_by_type;
 };
 
+// Block partials of one force call, summed together at its end: per source
+// the first partial and the number of blocks (0: not launched).
+struct ForceSums {
+    const double *qsc, *pair, *metal, *field;
+    int n_qsc, n_pair, n_metal, n_field;
+};
+
 // Bonded terms and virtual sites per molecule type (capac_desc bt_*, vs_*).
 struct BondedView {
     int n_mols;
@@ -289,6 +296,18 @@ struct capac_ctx {
     // reductions and outputs
     double *partials = nullptr;
     size_t partials_cap = 0;     // doubles
+    // a force call's own block partials (areas of each source), kept until its
+    // end; `defer`: the launches of a force call leave their sums to that end
+    double *fpart = nullptr;
+    size_t fpart_off[4] = {};    // areas: Sutton-Chen, pairs, CPIM metal, external field
+    bool defer = false;
+    capac::ForceSums fs{};
+    double *spart = nullptr;     // block partials of the step's velocity sums
+    int *scount = nullptr;       // their arrival counters (the last block finishes the sums)
+    int disp_tag = 0;            // flags[0] == disp_tag: an atom has moved half the skin (one tag per check)
+    cudaEvent_t ev_flags = nullptr;
+    bool pending_solve = false;  // the last solve's status is not read yet (settle_solve)
+    double pending_tol = 0.0;
     double *pot = nullptr, *vir = nullptr;  // [15], [9]
     capac::ThermoState *th = nullptr;
     capac::ThermoState *h_th = nullptr;
@@ -315,6 +334,12 @@ void launch_cluster_frames(capac_ctx *c, bool statics);
 void launch_pair_nonbonded_async(capac_ctx *c);
 void launch_pair_join(capac_ctx *c);
 void launch_list_maintenance(capac_ctx *c, bool force_rebuild);
+// start of a force call: packed positions, zeroed forces, energies and virial,
+// and the displacement check, whose answer finish_begin_force waits for (and
+// rebuilds the list); what needs no list may be launched in between
+void launch_begin_force(capac_ctx *c);
+void finish_begin_force(capac_ctx *c);
+void check_rattle(capac_ctx *c);  // throws when h_flags tells of a RATTLE failure
 // Rebuild the lists with an atom-list row for every atom, now and at every
 // later build (the gradient kernels walk all rows).
 void ensure_full_atom_list(capac_ctx *c);
@@ -322,8 +347,11 @@ void launch_pair_forces(capac_ctx *c, int mode);  // mode: 0 full, 1 CPIM water 
 void launch_qsc(capac_ctx *c);
 void launch_cpim_rhs(capac_ctx *c);
 void launch_cpim_matrix(capac_ctx *c);
-int run_bicgstab(capac_ctx *c);  // returns status
-int run_refined_solve(capac_ctx *c);  // mixed path: FP64 refinement around FP32-matrix BiCGSTAB
+// solve, with `defer` (dense solver only) without waiting for the status, which
+// settle_solve reads at the next wait; both return the status
+int run_bicgstab(capac_ctx *c, bool defer = false);
+int run_refined_solve(capac_ctx *c, bool defer = false);  // mixed path: FP64 refinement around FP32-matrix BiCGSTAB
+int settle_solve(capac_ctx *c);  // once the stream's work is done
 void launch_cpim_spmv(capac_ctx *c, const double *x, double *y);  // plain y = A x
 void launch_cpim_block_rows(capac_ctx *c, int i0, int rows, double *out);  // dense FP64 blocks of some rows
 // the symmetric FP64 tiles from a matrix in the reference's COO form (k_cpim_sym.cu)
@@ -358,7 +386,8 @@ int bicgstab_coop(capac_ctx *c, const double *b, double *x, double tol, double s
 bool dense_fits(int device, int n, bool mixed);
 size_t dense_exchange_bytes(int n);
 int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double skip, double *hist = nullptr,
-                   int order = 0);
+                   int order = 0, bool defer = false);
+int dense_status(capac_ctx *c, double skip);  // after the launch has ended and h_ss has landed
 // group-ordered solver (k_solve_coop.cu): internal vector length, blocks
 int group_tmem_tiles();
 int coarse_columns(int M, int n_nps, int modes);
@@ -371,23 +400,26 @@ int group_grid_size(int device, bool hold);
 int group_blocks_per_sm(int device, bool hold);
 void launch_cpim_metal_forces(capac_ctx *c);
 void launch_external_field(capac_ctx *c);
+// where source `area` of a force call writes its block partials
+inline double *force_partials(capac_ctx *c, int area) { return c->defer ? c->fpart + c->fpart_off[area] : c->partials; }
+enum { FP_QSC = 0, FP_PAIR, FP_METAL, FP_FIELD };
+void launch_force_sums(capac_ctx *c);  // the deferred partials into energy and virial slots
 // per-block partials (src, default c->partials) summed into energy and virial slots
 void launch_finalize(capac_ctx *c, int nblocks, int K, const int *slots_pot, const int *slots_vir,
                      const double *src = nullptr);
 void launch_pair_fingerprint(capac_ctx *c, int from_list, long *count, unsigned long long *hash);
 
 // integrator
-void launch_md_half_kick(capac_ctx *c, bool with_nhc_scale);
-void launch_md_drift(capac_ctx *c);
-void launch_rattle(capac_ctx *c, int second);
-void launch_kinetic(capac_ctx *c);
-void launch_nhc(capac_ctx *c);
-void launch_berendsen(capac_ctx *c);
-void launch_scale_velocities(capac_ctx *c);
-void launch_remove_com(capac_ctx *c);
+void launch_nhc(capac_ctx *c, long step);                // with the heating ramp
+void launch_md_kick_drift(capac_ctx *c, bool nvt, long step);  // scale (nvt) or heating ramp; half kick; drift
+void launch_md_half_kick(capac_ctx *c);
+// stage 2 in an MD step (in_step) leaves its virial to launch_step_sums
+void launch_rattle(capac_ctx *c, int second, bool in_step = false);
+// kinetic energy and momentum, thermostat (CAPAC_NVT, CAPAC_BERENDSEN; CAPAC_NVE none), COM
+// removal, kinetic energy again, sum_potential
+void launch_step_sums(capac_ctx *c, int thermostat, bool rattle_virial);
 void launch_apply_pbc(capac_ctx *c);
 void launch_fmax_rms(capac_ctx *c);
-void launch_heating(capac_ctx *c, long step);
 void launch_sum_potential(capac_ctx *c);
 void launch_build_vsites(capac_ctx *c);   // k_bonded.cu
 void launch_bonded(capac_ctx *c);
@@ -397,6 +429,8 @@ void launch_em_direction(capac_ctx *c, double gamma);  // s = F + gamma s; old F
 void launch_em_dots(capac_ctx *c);                 // partials of (F,F), (F_old,F), (F_old,F_old)
 
 size_t partials_needed(const capac_ctx *c);
+size_t force_partial_areas(const capac_ctx *c, size_t off[4]);
+constexpr int kSumBlocks = 592;  // most blocks of the step's velocity sums
 
 // Profiler hooks: a ProfScope brackets the launches issued in its lifetime.
 void prof_begin(capac_ctx *c, int cls);

@@ -2,6 +2,8 @@
 // Nose-Hoover chain, half kicks, drift, RATTLE, kinetic energy, COM-velocity
 // removal, apply_pbc and the force diagnostics.  Scalars (thermostat chain,
 // kinetic energy, temperature) stay in device memory.
+#include <algorithm>
+
 #include "ctx.h"
 
 namespace capac {
@@ -29,10 +31,14 @@ MdParams md_params(const capac_ctx *c)
 }
 
 // Heating ramp of the reference temperature (mpi-main.c:879-891).
-__global__ void k_heating(ThermoState *th, long step, int n_heating)
+struct Heating {
+    long step;
+    int n;
+};
+__device__ __forceinline__ void heat(ThermoState *th, Heating h)
 {
-    if (step < n_heating)
-        th->ref_temp = th->first_temp + (th->ext_temp - th->first_temp) * step / n_heating;
+    if (h.step < h.n)
+        th->ref_temp = th->first_temp + (th->ext_temp - th->first_temp) * h.step / h.n;
     else
         th->ref_temp = th->ext_temp;
     th->kT = kBoltz * th->ref_temp;
@@ -102,7 +108,7 @@ __device__ __forceinline__ double nhc_chain(double (&vQ)[kNhc], double (&aQ)[kNh
 // library's); on the way up they are those of velocities the way down left
 // final, so only a multiply-add pair waits; the divisions by Q are folded into
 // kT / Q.  41 us a launch with the library's exp and the divisions, 14.6 so.
-__global__ void k_nhc(ThermoState *th, MdParams m)
+__device__ void nhc(ThermoState *th, const MdParams &m)
 {
     const double Q = m.q_mass, kT = th->kT, NkT = kT * m.ndf, ek = th->eksum, inv_q = 1.0 / Q;
     // the chain in registers (every index is fixed once the loops unroll),
@@ -126,12 +132,19 @@ __global__ void k_nhc(ThermoState *th, MdParams m)
     th->inst_temp *= scale * scale;
 }
 
+// The first chain of a step, after the heating ramp.
+__global__ void k_nhc(ThermoState *th, MdParams m, Heating h)
+{
+    heat(th, h);
+    nhc(th, m);
+}
+
 // Berendsen weak coupling (no counterpart in the reference, whose only
 // thermostat is the Nose-Hoover chain): lambda = sqrt(1 + dt/tau (T0/T - 1))
 // from the temperature after the second RATTLE (Berendsen et al., J. Chem.
 // Phys. 81, 3684 (1984)), lambda^2 held to [0.64, 1.5625] and lambda = 1 at
-// T = 0; the scale is left in th->scale for k_scale_velocities.
-__global__ void k_berendsen(ThermoState *th, double dt_over_tau)
+// T = 0; the scale is left in th->scale.
+__device__ void berendsen(ThermoState *th, double dt_over_tau)
 {
     const double T = th->inst_temp;
     double s2 = 1.0;
@@ -142,47 +155,45 @@ __global__ void k_berendsen(ThermoState *th, double dt_over_tau)
     th->inst_temp *= s * s;
 }
 
-// Optional thermostat scaling of every velocity, then v += dt/2 F/m for
-// atoms that move (mpi-main.c:900-913).
-__global__ void k_half_kick(MdParams m, const unsigned char *is_metal, const double *inv_mass,
-                            const double *fx, const double *fy, const double *fz, double *vx, double *vy,
-                            double *vz, const ThermoState *th, int apply_scale)
+// First half of a step: the thermostat's scale (nvt; else the heating ramp is
+// done here), v += dt/2 F/m, old_r = r, r += dt v, the last three for atoms
+// that move (mpi-main.c:900-932).
+__global__ void k_kick_drift(MdParams m, const unsigned char *is_metal, const double *inv_mass, const double *fx,
+                             const double *fy, const double *fz, double *vx, double *vy, double *vz, double *rx,
+                             double *ry, double *rz, double *ox, double *oy, double *oz, ThermoState *th, int nvt,
+                             Heating h)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (!nvt && i == 0) heat(th, h);
     if (i >= m.N) return;
     double a = vx[i], b = vy[i], c = vz[i];
-    if (apply_scale) {
+    if (nvt) {
         const double s = th->scale;
         a *= s; b *= s; c *= s;
     }
     if (!(m.fix_metal == 1 && is_metal[i])) {
-        const double im = inv_mass[i];
+        const double im = inv_mass[i], x = rx[i], y = ry[i], z = rz[i];
         a += m.dt_2 * fx[i] * im;
         b += m.dt_2 * fy[i] * im;
         c += m.dt_2 * fz[i] * im;
+        ox[i] = x; oy[i] = y; oz[i] = z;
+        rx[i] = x + m.dt * a;
+        ry[i] = y + m.dt * b;
+        rz[i] = z + m.dt * c;
     }
     vx[i] = a; vy[i] = b; vz[i] = c;
 }
 
-__global__ void k_scale_velocities(int N, const ThermoState *th, double *vx, double *vy, double *vz)
+// v += dt/2 F/m for atoms that move.
+__global__ void k_half_kick(MdParams m, const unsigned char *is_metal, const double *inv_mass, const double *fx,
+                            const double *fy, const double *fz, double *vx, double *vy, double *vz)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const double s = th->scale;
-    vx[i] *= s; vy[i] *= s; vz[i] *= s;
-}
-
-// old_r = r; r += dt v (mpi-main.c:917-932).
-__global__ void k_drift(MdParams m, const unsigned char *is_metal, double *rx, double *ry, double *rz,
-                        const double *vx, const double *vy, const double *vz, double *ox, double *oy, double *oz)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.N) return;
-    if (m.fix_metal == 1 && is_metal[i]) return;
-    ox[i] = rx[i]; oy[i] = ry[i]; oz[i] = rz[i];
-    rx[i] += m.dt * vx[i];
-    ry[i] += m.dt * vy[i];
-    rz[i] += m.dt * vz[i];
+    if (i >= m.N || (m.fix_metal == 1 && is_metal[i])) return;
+    const double im = inv_mass[i];
+    vx[i] += m.dt_2 * fx[i] * im;
+    vy[i] += m.dt_2 * fy[i] * im;
+    vz[i] += m.dt_2 * fz[i] * im;
 }
 
 struct CstrView {
@@ -444,81 +455,107 @@ __global__ void __launch_bounds__(kRattleBlock) k_rattle2(MdParams m, CstrView c
     block_partials<9>(vir, sh, partials);
 }
 
-// partials of sum m v^2 per axis (kinetic_energy, thermostat.c:34-63)
-__global__ void __launch_bounds__(256) k_kinetic(int N, const double *mass, const double *vx, const double *vy,
-                                                 const double *vz, double *partials)
+// A block's K partial sums stored; true in the block that finds all others'
+// stored (the last to arrive), which then sums them in block order.  The
+// counter is left at zero for the next launch.
+template <int K>
+__device__ bool last_block_sum(double (&v)[K], double *sh, double *partials, int *count)
 {
-    __shared__ double sh[32 * 3];
-    double v[3] = {0.0, 0.0, 0.0};
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < N) {
-        const double mm = mass[i];
-        if (mm > 0.0) {
-            v[0] = mm * vx[i] * vx[i];
-            v[1] = mm * vy[i] * vy[i];
-            v[2] = mm * vz[i] * vz[i];
-        }
+    __shared__ int last;
+    block_partials<K>(v, sh, partials);
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(count, 1) == (int)gridDim.x - 1;
     }
-    block_partials<3>(v, sh, partials);
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] += __ldcg(partials + (size_t)K * b + k);
+    block_sum<K>(v, sh);
+    if (threadIdx.x == 0) *count = 0;
+    return true;
 }
 
-__global__ void k_kinetic_final(const double *partials, int nb, int ndf, ThermoState *th)
+// The velocity sums after the second half kick, kinetic_energy
+// (thermostat.c:34-63) and remove_comm's momentum (:69-108), in one pass; the
+// last block finishes them, runs the thermostat and leaves in th the scale and
+// the scaled momentum's velocity for k_step_apply, and adds RATTLE's block
+// partials of the virial.
+__global__ void __launch_bounds__(256) k_step_sums(MdParams m, const double *__restrict__ mass,
+                                                   const double *__restrict__ vx, const double *__restrict__ vy,
+                                                   const double *__restrict__ vz, int thermostat, double dt_over_tau,
+                                                   ThermoState *th, double *partials, int *count,
+                                                   const double *__restrict__ rattle, int n_rattle, double *vir)
 {
-    __shared__ double sh[32 * 3];
-    double v[3] = {0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-        v[0] += partials[3 * b];
-        v[1] += partials[3 * b + 1];
-        v[2] += partials[3 * b + 2];
+    __shared__ double sh[32 * 9];
+    double v[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.N; i += gridDim.x * blockDim.x) {
+        const double mm = mass[i];
+        if (!(mm > 0.0)) continue;
+        const double a = vx[i], b = vy[i], c = vz[i];
+        v[0] += mm * a * a;
+        v[1] += mm * b * b;
+        v[2] += mm * c * c;
+        v[3] += a * mm;
+        v[4] += b * mm;
+        v[5] += c * mm;
+        v[6] += mm;
     }
-    block_sum<3>(v, sh);
+    if (!last_block_sum<7>(v, sh, partials, count)) return;
     if (threadIdx.x == 0) {
         th->eksum = v[0] + v[1] + v[2];
-        th->inst_temp = th->eksum / (kBoltz * ndf);
+        th->inst_temp = th->eksum / (kBoltz * m.ndf);
+        if (thermostat == CAPAC_NVT) nhc(th, m);
+        else if (thermostat == CAPAC_BERENDSEN) berendsen(th, dt_over_tau);
+        else th->scale = 1.0;
+        for (int a = 0; a < 3; ++a) th->vcom[a] = th->scale * v[3 + a] / v[6];
+        th->vcom[3] = v[6];
+    }
+    if (n_rattle > 0) {
+        double w[9] = {0.0};
+        for (int b = threadIdx.x; b < n_rattle; b += blockDim.x)
+#pragma unroll
+            for (int k = 0; k < 9; ++k) w[k] += rattle[(size_t)9 * b + k];
+        __syncthreads();
+        block_sum<9>(w, sh);
+        if (threadIdx.x == 0)
+            for (int k = 0; k < 9; ++k) vir[k] += w[k];
     }
 }
 
-// remove_comm, thermostat.c:69-108
-__global__ void __launch_bounds__(256) k_momentum(int N, const double *mass, const double *vx, const double *vy,
-                                                  const double *vz, double *partials)
+// v = scale v - v_com and the kinetic energy of the result (the last block
+// finishes it), with sum_potential (force.c:322-331).
+__global__ void __launch_bounds__(256) k_step_apply(MdParams m, const double *__restrict__ mass, double *vx, double *vy,
+                                                    double *vz, ThermoState *th, double *partials, int *count,
+                                                    double *pot)
 {
-    __shared__ double sh[32 * 4];
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < N) {
+    __shared__ double sh[32 * 3];
+    const double s = th->scale, c0 = th->vcom[0], c1 = th->vcom[1], c2 = th->vcom[2];
+    double v[3] = {0.0, 0.0, 0.0};
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.N; i += gridDim.x * blockDim.x) {
         const double mm = mass[i];
-        if (mm > 0.0) {
-            v[0] = vx[i] * mm;
-            v[1] = vy[i] * mm;
-            v[2] = vz[i] * mm;
-            v[3] = mm;
+        const bool real = mm > 0.0;
+        const double a = s * vx[i] - (real ? c0 : 0.0), b = s * vy[i] - (real ? c1 : 0.0),
+                     c = s * vz[i] - (real ? c2 : 0.0);
+        vx[i] = a; vy[i] = b; vz[i] = c;
+        if (real) {
+            v[0] += mm * a * a;
+            v[1] += mm * b * b;
+            v[2] += mm * c * c;
         }
     }
-    block_partials<4>(v, sh, partials);
-}
-
-__global__ void k_momentum_final(const double *partials, int nb, ThermoState *th)
-{
-    __shared__ double sh[32 * 4];
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
-        for (int k = 0; k < 4; ++k) v[k] += partials[4 * b + k];
-    block_sum<4>(v, sh);
+    if (!last_block_sum<3>(v, sh, partials, count)) return;
     if (threadIdx.x == 0) {
-        th->vcom[0] = v[0] / v[3];
-        th->vcom[1] = v[1] / v[3];
-        th->vcom[2] = v[2] / v[3];
-        th->vcom[3] = v[3];
+        th->eksum = v[0] + v[1] + v[2];
+        th->inst_temp = th->eksum / (kBoltz * m.ndf);
+        double e = 0.0;
+        for (int k = 1; k < 15; ++k) e += pot[k];
+        pot[0] = e;
     }
-}
-
-__global__ void k_sub_com(int N, const double *mass, const ThermoState *th, double *vx, double *vy, double *vz)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N || !(mass[i] > 0.0)) return;
-    vx[i] -= th->vcom[0];
-    vy[i] -= th->vcom[1];
-    vz[i] -= th->vcom[2];
 }
 
 // apply_pbc, force.c:127-165: one thread per molecule.
@@ -665,46 +702,39 @@ CstrView cstr_view(const capac_ctx *c)
 
 }  // namespace
 
-void launch_heating(capac_ctx *c, long step)
+void launch_nhc(capac_ctx *c, long step)
 {
-    k_heating<<<1, 1, 0, c->stream>>>(c->th, step, c->n_heating);
+    k_nhc<<<1, 1, 0, c->stream>>>(c->th, md_params(c), Heating{step, c->n_heating});
     ++c->launches;
 }
 
-void launch_nhc(capac_ctx *c)
+void launch_md_kick_drift(capac_ctx *c, bool nvt, long step)
 {
-    k_nhc<<<1, 1, 0, c->stream>>>(c->th, md_params(c));
+    k_kick_drift<<<grid_for(c->N, 256), 256, 0, c->stream>>>(
+        md_params(c), c->is_metal, c->inv_mass, c->fx, c->fy, c->fz, c->vx, c->vy, c->vz, c->rx, c->ry, c->rz, c->ox,
+        c->oy, c->oz, c->th, nvt ? 1 : 0, Heating{step, c->n_heating});
     ++c->launches;
 }
 
-void launch_berendsen(capac_ctx *c)
-{
-    k_berendsen<<<1, 1, 0, c->stream>>>(c->th, c->dt_over_tau);
-    ++c->launches;
-}
-
-void launch_md_half_kick(capac_ctx *c, bool with_nhc_scale)
+void launch_md_half_kick(capac_ctx *c)
 {
     k_half_kick<<<grid_for(c->N, 256), 256, 0, c->stream>>>(md_params(c), c->is_metal, c->inv_mass, c->fx, c->fy,
-                                                           c->fz, c->vx, c->vy, c->vz, c->th,
-                                                           with_nhc_scale ? 1 : 0);
+                                                           c->fz, c->vx, c->vy, c->vz);
     ++c->launches;
 }
 
-void launch_scale_velocities(capac_ctx *c)
+void launch_step_sums(capac_ctx *c, int thermostat, bool rattle_virial)
 {
-    k_scale_velocities<<<grid_for(c->N, 256), 256, 0, c->stream>>>(c->N, c->th, c->vx, c->vy, c->vz);
-    ++c->launches;
+    const unsigned grid = std::min(grid_for(c->N, 256), (unsigned)kSumBlocks);
+    const int nr = rattle_virial ? (int)grid_for(c->n_mols, kRattleBlock) : 0;
+    k_step_sums<<<grid, 256, 0, c->stream>>>(md_params(c), c->mass, c->vx, c->vy, c->vz, thermostat, c->dt_over_tau,
+                                             c->th, c->spart, c->scount, c->partials, nr, c->vir);
+    k_step_apply<<<grid, 256, 0, c->stream>>>(md_params(c), c->mass, c->vx, c->vy, c->vz, c->th, c->spart,
+                                              c->scount + 1, c->pot);
+    c->launches += 2;
 }
 
-void launch_md_drift(capac_ctx *c)
-{
-    k_drift<<<grid_for(c->N, 256), 256, 0, c->stream>>>(md_params(c), c->is_metal, c->rx, c->ry, c->rz, c->vx,
-                                                       c->vy, c->vz, c->ox, c->oy, c->oz);
-    ++c->launches;
-}
-
-void launch_rattle(capac_ctx *c, int second)
+void launch_rattle(capac_ctx *c, int second, bool in_step)
 {
     if (!c->has_cstr) return;
     const unsigned grid = grid_for(c->n_mols, kRattleBlock);
@@ -716,27 +746,11 @@ void launch_rattle(capac_ctx *c, int second)
         k_rattle2<<<grid, kRattleBlock, 0, c->stream>>>(md_params(c), cstr_view(c), c->rx, c->ry, c->rz, c->vx, c->vy, c->vz,
                                                c->flags, c->partials);
         ++c->launches;
+        if (in_step) return;
         static const int pot_slots[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};
         static const int vir_slots[9] = {0, 1, 2, 3, 4, 5, 6, 7, 8};
         launch_finalize(c, (int)grid, 9, pot_slots, vir_slots);
     }
-}
-
-void launch_kinetic(capac_ctx *c)
-{
-    const unsigned grid = grid_for(c->N, 256);
-    k_kinetic<<<grid, 256, 0, c->stream>>>(c->N, c->mass, c->vx, c->vy, c->vz, c->partials);
-    k_kinetic_final<<<1, 256, 0, c->stream>>>(c->partials, (int)grid, c->c.ndf, c->th);
-    c->launches += 2;
-}
-
-void launch_remove_com(capac_ctx *c)
-{
-    const unsigned grid = grid_for(c->N, 256);
-    k_momentum<<<grid, 256, 0, c->stream>>>(c->N, c->mass, c->vx, c->vy, c->vz, c->partials);
-    k_momentum_final<<<1, 256, 0, c->stream>>>(c->partials, (int)grid, c->th);
-    k_sub_com<<<grid, 256, 0, c->stream>>>(c->N, c->mass, c->th, c->vx, c->vy, c->vz);
-    c->launches += 3;
 }
 
 void launch_apply_pbc(capac_ctx *c)

@@ -1071,16 +1071,17 @@ void launch_pair_t(capac_ctx *c, int mode, unsigned grid)
 {
     const PairConstsF K = pair_consts_f(c);
     const bool cpim = c->M > 0 && c->use_cpff;
+    double *part = force_partials(c, FP_PAIR);
     ProfScope ps(c, K_PAIR);
     if (mode == 0 && cpim)
         k_pair<Real, true, true><<<grid, kPairWarps * 32, 0, c->stream>>>(c->P, K, c->pos4, c->nbr, c->nnb, c->cap,
-                                                                          c->vec_pq, c->fx, c->fy, c->fz, c->partials);
+                                                                          c->vec_pq, c->fx, c->fy, c->fz, part);
     else if (mode == 0)
         k_pair<Real, true, false><<<grid, kPairWarps * 32, 0, c->stream>>>(c->P, K, c->pos4, c->nbr, c->nnb, c->cap,
-                                                                           c->vec_pq, c->fx, c->fy, c->fz, c->partials);
+                                                                           c->vec_pq, c->fx, c->fy, c->fz, part);
     else
         k_pair<Real, false, true><<<grid, kPairWarps * 32, 0, c->stream>>>(c->P, K, c->pos4, c->nbr, c->nnb, c->cap,
-                                                                           c->vec_pq, c->fx, c->fy, c->fz, c->partials);
+                                                                           c->vec_pq, c->fx, c->fy, c->fz, part);
     ++c->launches;
 }
 
@@ -1105,7 +1106,7 @@ void launch_pair_cp_t(capac_ctx *c, unsigned grid)
     CAPAC_CUDA(cudaMemsetAsync(c->cl_next, 0, sizeof(int), c->stream));
     k_pair_cp<NONBONDED, CPIM><<<grid, kCpWarps * 32, 0, c->stream>>>(
         c->P, pair_consts_f(c), c->cp_cent, c->cp_off, c->cp_ti, c->cp_list, c->cp_n, c->cp_cap, c->n_clusters,
-        c->vec_pq, c->fx, c->fy, c->fz, c->partials, c->cl_next);
+        c->vec_pq, c->fx, c->fy, c->fz, force_partials(c, FP_PAIR), c->cl_next);
 }
 
 // The cluster frames of the current positions, then the cluster-pair kernel.
@@ -1126,26 +1127,27 @@ void launch_pair_cpairs(capac_ctx *c, int mode, unsigned grid)
 void launch_pair_clusters(capac_ctx *c, int mode, unsigned grid)
 {
     const bool cpim = c->M > 0 && c->use_cpff;
+    double *part = force_partials(c, FP_PAIR);
     ProfScope ps(c, K_PAIR);
     if (c->cl_half) {
         if (mode == 0 && cpim && c->pair_split) {
             // the pair terms without the CPIM branches, then the water-side
             // CPIM term over the clusters with a metal member or neighbour
-            launch_pair_cl_t<true, false, true>(c, grid, c->stream, c->partials, false);
-            launch_pair_cl_t<false, true, true>(c, grid, c->stream, c->partials, true);
+            launch_pair_cl_t<true, false, true>(c, grid, c->stream, part, false);
+            launch_pair_cl_t<false, true, true>(c, grid, c->stream, part, true);
             ++c->launches;
         } else if (mode == 0 && cpim)
-            launch_pair_cl_t<true, true, true>(c, grid, c->stream, c->partials, false);
+            launch_pair_cl_t<true, true, true>(c, grid, c->stream, part, false);
         else if (mode == 0)
-            launch_pair_cl_t<true, false, true>(c, grid, c->stream, c->partials, false);
+            launch_pair_cl_t<true, false, true>(c, grid, c->stream, part, false);
         else
-            launch_pair_cl_t<false, true, true>(c, grid, c->stream, c->partials, false);
+            launch_pair_cl_t<false, true, true>(c, grid, c->stream, part, false);
     } else if (mode == 0 && cpim)
-        launch_pair_cl_t<true, true, false>(c, grid, c->stream, c->partials, false);
+        launch_pair_cl_t<true, true, false>(c, grid, c->stream, part, false);
     else if (mode == 0)
-        launch_pair_cl_t<true, false, false>(c, grid, c->stream, c->partials, false);
+        launch_pair_cl_t<true, false, false>(c, grid, c->stream, part, false);
     else
-        launch_pair_cl_t<false, true, false>(c, grid, c->stream, c->partials, false);
+        launch_pair_cl_t<false, true, false>(c, grid, c->stream, part, false);
     ++c->launches;
 }
 
@@ -1213,7 +1215,10 @@ void launch_pair_forces(capac_ctx *c, int mode)
         launch_pair_t<float>(c, mode, grid);
     else
         launch_pair_t<double>(c, mode, grid);
-    if (mode == 0) {
+    if (mode == 0 && c->defer) {
+        c->fs.pair = force_partials(c, FP_PAIR);
+        c->fs.n_pair = (int)grid;
+    } else if (mode == 0) {
         static const int pot_slots[11] = {7, 8, -1, -1, -1, -1, -1, -1, -1, -1, -1};
         static const int vir_slots[11] = {-1, -1, 0, 1, 2, 3, 4, 5, 6, 7, 8};
         launch_finalize(c, (int)grid, 11, pot_slots, vir_slots);

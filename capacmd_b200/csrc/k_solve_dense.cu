@@ -72,6 +72,7 @@ constexpr long kPollLimit = 1L << 24;
 constexpr int kFirstRead = 600; // cycles from a block's store to its first read
 constexpr int kStall = 60;      // iterations without a halving of (r, r) that end a sweep
 constexpr int kSweeps = 12;
+constexpr int kStarts = 8;      // FP64 path: starts after breakdowns
 constexpr int kStageRows = 8;   // ring of inverse-block rows: stages(C) x 2 groups x 8 rows
 constexpr int kStepsPerPair = kGroup / kStageRows;
 constexpr long kWaitPolls = 1L << 20;
@@ -476,7 +477,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_bicgstab_dense(const __grid_const
         rTr = rr0 = rho;
         if (BJ ? rTr <= crit : rho < A.skip) done = true;  // warm start already converged (bicg_stab.c:368)
     }
-    while (ok && !done) {  // sweeps: one on the FP64 path
+    while (ok && !done) {  // sweeps; on the FP64 path starts, a second one only after a breakdown
         const double goal = BJ ? 0.25 * crit : crit;
         double rho_old = 1.0, alpha = 1.0, omega = 1.0, mark = rTr;
         int it = 0, gain = 0;
@@ -567,7 +568,32 @@ __global__ void __launch_bounds__(kBlock, 1) k_bicgstab_dense(const __grid_const
                 }
             }
         }
-        if (!BJ || !ok) break;
+        if (!ok) break;
+        if (!BJ) {
+            // a breakdown leaves x at its last finite value: start again from
+            // there with a fresh shadow residual (the reference would carry the
+            // NaN to MAX_ITER); only an exact zero now ends it early
+            ++sweep;
+            if (!broke || status != -2 || sweep == kStarts) break;
+            broke = false;
+            status = 0;
+#pragma unroll
+            for (int m = 0; m < C; ++m) y[m] = xs[m][tid];
+            product(y, true, since);
+            const bool bad = receive<C>(A, y, seq, since);
+            ++seq;
+            double s[1] = {0.0};
+#pragma unroll
+            for (int m = 0; m < C; ++m) {
+                const int e = tid + kBlock * m, rr = e < n ? ref_row(e) : -1;
+                r[m] = rr >= 0 ? A.b[rr] - y[m] : 0.0;
+                s[0] = fma(r[m], r[m], s[0]);
+            }
+            ok = sum_all<1>(s, tsh, bad);
+            rTr = rho = s[0];
+            done = rho < 1.0e-300;
+            continue;
+        }
         // x += K u: the block's rows of K u, one warp per row, then the new x
         // to every block and its residual from the matrix itself
         if (it == 0) break;  // no progress possible
@@ -702,7 +728,9 @@ size_t dense_exchange_bytes(int n) { return (size_t)2 * ((n + kR - 1) / kR) * kS
 // refined solve (hist set: with the warm-start predictor) to (r, r) <= tol
 // (b, b), the residual from the positions.  The status as bicgstab_core
 // returns it.
-int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double skip, double *hist, int order)
+// `defer`: without waiting for it (dense_status reads it later).
+int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double skip, double *hist, int order,
+                   bool defer)
 {
     const bool mixed = c->opt.precision == CAPAC_PREC_MIXED;
     DenseArgs A;
@@ -732,10 +760,10 @@ int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double 
     A.nG = mixed ? precond_groups(c->M) : 0;
     A.hist = hist;
     A.order = order;
-    // two exchanges per iteration, two per sweep and one for the start; the
+    // two exchanges per iteration, two per sweep or start; the
     // numbers of a launch are not used again until they wrap, when the buffers
     // are cleared
-    const unsigned long long need = 2ull * ((unsigned long long)A.max_iter + 4) * (mixed ? kSweeps : 1) + 2;
+    const unsigned long long need = 2ull * ((unsigned long long)A.max_iter + 4) * (mixed ? kSweeps : kStarts) + 2;
     if (c->dense_seq + need > 0xffffffffull) {
         CAPAC_CUDA(cudaMemsetAsync(c->dense_ex, 0, dense_exchange_bytes(A.n), c->stream));
         c->dense_seq = 1;
@@ -750,7 +778,13 @@ int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double 
     }
     ++c->launches;
     CAPAC_CUDA(cudaMemcpyAsync(c->h_ss, c->ss, sizeof(SolverScalars), cudaMemcpyDeviceToHost, c->stream));
+    if (defer) return CAPAC_OK;
     CAPAC_CUDA(cudaStreamSynchronize(c->stream));
+    return dense_status(c, skip);
+}
+
+int dense_status(capac_ctx *c, double skip)
+{
     if (c->h_ss->error) {
         CAPAC_CUDA(cudaMemsetAsync(&c->ss->error, 0, sizeof(int), c->stream));
         throw Error(CAPAC_ERR_CUDA, "persistent solver: a bounded wait timed out");
