@@ -50,13 +50,17 @@ void settle(capac_ctx *c)
 // Waits for the stream; throws the failures of RATTLE and of a pending solve.
 void check_flags(capac_ctx *c)
 {
-    CAPAC_CUDA(cudaMemcpyAsync(c->h_flags, c->flags, sizeof(int) * 4, cudaMemcpyDeviceToHost, c->stream));
     CAPAC_CUDA(cudaStreamSynchronize(c->stream));
     settle(c);
     check_rattle(c);
 }
 
-void record(capac_ctx *c, int k) { CAPAC_CUDA(cudaEventRecord(c->ev[k], c->stream)); }
+// A timed event costs the stream ~4 us, so only the last force call of a run of
+// MD steps records its phases.
+void record(capac_ctx *c, int k)
+{
+    if (c->phases) CAPAC_CUDA(cudaEventRecord(c->ev[k], c->stream));
+}
 
 // One mpi_force equivalent on the device state; solve = false keeps the
 // induced vector as it is.  The host waits once, for the displacement check
@@ -121,14 +125,21 @@ void force(capac_ctx *c, bool solve = true)
     c->grad_ready = solve;
 }
 
-void md_step(capac_ctx *c)
+void md_step(capac_ctx *c, bool last)
 {
     const long step = ++c->md_step;
     const bool nvt = c->ensemble == CAPAC_NVT;
     if (nvt) launch_nhc(c, step);
     launch_md_kick_drift(c, nvt, step);
     launch_rattle(c, 0);
-    force(c);
+    {
+        struct Phases {
+            capac_ctx *c;
+            ~Phases() { c->phases = true; }
+        } phases{c};
+        c->phases = last;
+        force(c);
+    }
     launch_md_half_kick(c);
     launch_rattle(c, 1, true);
     launch_step_sums(c, c->ensemble, c->has_cstr);
@@ -168,10 +179,9 @@ void set_last_error(const std::string &msg) { g_last_error = msg; }
 
 void check_rattle(capac_ctx *c)
 {
-    if (!c->h_flags[2]) return;
-    const bool first = c->h_flags[2] & 1;
-    c->h_flags[2] = 0;
-    CAPAC_CUDA(cudaMemsetAsync(c->flags + 2, 0, sizeof(int), c->stream));
+    if (!c->sig[1] && !c->sig[2]) return;
+    const bool first = c->sig[1] != 0;
+    c->sig[1] = c->sig[2] = 0;
     throw Error(CAPAC_ERR_RATTLE, first ? "RATTLE_1 not converged!" : "RATTLE_2 not converged!");
 }
 
@@ -492,6 +502,12 @@ int capac_create(const capac_desc *d, const capac_options *opt, capac_ctx **out)
             c->flags = dalloc<int>(8);
             CAPAC_CUDA(cudaMemsetAsync(c->flags, 0, sizeof(int) * 8, s));
             CAPAC_CUDA(cudaMallocHost(&c->h_flags, sizeof(int) * 8));
+            {
+                void *sig = nullptr;
+                CAPAC_CUDA(cudaMallocHost(&sig, sizeof(int) * 4));
+                c->sig = static_cast<volatile int *>(sig);
+                for (int k = 0; k < 4; ++k) c->sig[k] = 0;
+            }
 
             // metal / CPIM
             if (c->M > 0) {
@@ -671,6 +687,7 @@ int capac_destroy(capac_ctx *c)
     for (void *p : c->bonded_buffers)
         if (p) cudaFree(p);
     if (c->h_flags) cudaFreeHost(c->h_flags);
+    if (c->sig) cudaFreeHost(const_cast<int *>(c->sig));
     if (c->h_ss) cudaFreeHost(c->h_ss);
     if (c->h_th) cudaFreeHost(c->h_th);
     for (auto &e : c->ev)
@@ -1133,8 +1150,7 @@ int capac_md_steps(capac_ctx *c, int n)
     return guard([&] {
         check_ctx(c);
         if (n < 0) throw Error(CAPAC_ERR_INVALID, "negative step count");
-        for (int k = 0; k < n; ++k) md_step(c);
-        CAPAC_CUDA(cudaStreamSynchronize(c->stream));
+        for (int k = 0; k < n; ++k) md_step(c, k == n - 1);
         check_flags(c);
     });
 }
@@ -1318,7 +1334,7 @@ int capac_time_md_steps(capac_ctx *c, int n, double *ms)
         check_ctx(c);
         if (!ms || n < 0) throw Error(CAPAC_ERR_INVALID, "bad argument");
         CAPAC_CUDA(cudaEventRecord(c->ev[14], c->stream));
-        for (int k = 0; k < n; ++k) md_step(c);
+        for (int k = 0; k < n; ++k) md_step(c, k == n - 1);
         CAPAC_CUDA(cudaEventRecord(c->ev[15], c->stream));
         CAPAC_CUDA(cudaEventSynchronize(c->ev[15]));
         float t = 0.f;

@@ -168,7 +168,7 @@ struct capac_ctx {
     double4 *spos = nullptr;     // [N] positions in cell order, atom index in w
     void *sort_tmp = nullptr;
     size_t sort_tmp_bytes = 0;
-    int *flags = nullptr;      // [0] rebuild needed, [1] list overflow max count, [2] rattle error,
+    int *flags = nullptr;      // [0] rebuild needed (stage calls), [1] list overflow max count,
                                // [4] cluster-list overflow max count, [5] cluster extent (float bits),
                                // [7] cluster-pair list overflow max count
     int *h_flags = nullptr;    // pinned mirror
@@ -304,7 +304,13 @@ struct capac_ctx {
     capac::ForceSums fs{};
     double *spart = nullptr;     // block partials of the step's velocity sums
     int *scount = nullptr;       // their arrival counters (the last block finishes the sums)
-    int disp_tag = 0;            // flags[0] == disp_tag: an atom has moved half the skin (one tag per check)
+    // words in pinned host memory that kernels write (posted, seen by the host
+    // after the wait for an event behind the kernel; a copy of its own took
+    // ~10 us of a step): [0] the tag of the displacement check that found an
+    // atom past half the skin, [1], [2] a molecule RATTLE's stage did not converge
+    volatile int *sig = nullptr;
+    int disp_tag = 0;            // tag of the last check
+    bool phases = true;          // record the phase events of force calls
     cudaEvent_t ev_flags = nullptr;
     bool pending_solve = false;  // the last solve's status is not read yet (settle_solve)
     double pending_tol = 0.0;
@@ -339,7 +345,7 @@ void launch_list_maintenance(capac_ctx *c, bool force_rebuild);
 // rebuilds the list); what needs no list may be launched in between
 void launch_begin_force(capac_ctx *c);
 void finish_begin_force(capac_ctx *c);
-void check_rattle(capac_ctx *c);  // throws when h_flags tells of a RATTLE failure
+void check_rattle(capac_ctx *c);  // throws when sig tells of a RATTLE failure
 // Rebuild the lists with an atom-list row for every atom, now and at every
 // later build (the gradient kernels walk all rows).
 void ensure_full_atom_list(capac_ctx *c);

@@ -62,7 +62,10 @@ __device__ __forceinline__ void load4(const double *p, double out[4])
     out[3] = v.y;
 }
 
-// Assembly: one block per tile, 256 threads, 4 pairs each.
+// Assembly: blockIdx.y of gridDim.y blocks per tile, 256 threads, 4 pairs each
+// where one block forms the tile.  A pair is a long chain of FP64 operations,
+// so a matrix of few tiles is spread over four blocks each (15 tiles: 10.4 ->
+// 5 us).
 template <typename T>
 // slots: null for the metal atoms in index order, else the atom of each
 // tile slot (-1 for padding): the group order of the grouped solver.
@@ -75,7 +78,7 @@ __global__ void __launch_bounds__(256) k_sym_assemble(DevParams P, const double4
     while (tile_index(I + 1, I + 1, nT) <= t && I + 1 < nT) ++I;
     const int J = I + (int)(t - tile_index(I, I, nT));
     T *tile = mat + t * kTileElems;
-    for (int q = threadIdx.x; q < kT * kT; q += blockDim.x) {
+    for (int q = blockIdx.y * blockDim.x + threadIdx.x; q < kT * kT; q += gridDim.y * blockDim.x) {
         const int a = q & (kT - 1), b = q >> 5;
         int i = I * kT + a, j = J * kT + b;
         if (slots) {
@@ -383,11 +386,12 @@ void launch_sym_assemble(capac_ctx *c)
     const int nT = sym_tiles(c->M);
     const unsigned tiles = (unsigned)(nT * (nT + 1) / 2);
     ProfScope ps(c, K_MATRIX);
+    const dim3 grid(tiles, tiles <= 2u * c->num_sms ? 4 : 1);
     if (c->opt.precision == CAPAC_PREC_MIXED)
-        k_sym_assemble<float><<<tiles, 256, 0, c->stream>>>(c->P, c->pos4, nT, c->grouped ? c->g_atoms : nullptr,
+        k_sym_assemble<float><<<grid, 256, 0, c->stream>>>(c->P, c->pos4, nT, c->grouped ? c->g_atoms : nullptr,
                                                              static_cast<float *>(c->msym));
     else
-        k_sym_assemble<double><<<tiles, 256, 0, c->stream>>>(c->P, c->pos4, nT, nullptr,
+        k_sym_assemble<double><<<grid, 256, 0, c->stream>>>(c->P, c->pos4, nT, nullptr,
                                                               static_cast<double *>(c->msym));
     ++c->launches;
 }

@@ -671,13 +671,13 @@ __global__ void k_displacement(int N, Box box, double half_skin2, const double *
 
 // Start of a force call, one pass over the atoms: the packed positions, zeroed
 // forces, energies and virial, and (rx0 not null) the displacement check, which
-// leaves `tag` in flags[0].
+// leaves `tag` in the host's word.
 __global__ void k_begin_force(int N, Box box, double half_skin2, const double *__restrict__ rx,
                               const double *__restrict__ ry, const double *__restrict__ rz,
                               const double *__restrict__ q, const double *__restrict__ rx0,
                               const double *__restrict__ ry0, const double *__restrict__ rz0, double4 *pos4,
-                              float4 *pos4f, double *fx, double *fy, double *fz, double *pot, double *vir, int *flags,
-                              int tag)
+                              float4 *pos4f, double *fx, double *fy, double *fz, double *pot, double *vir,
+                              volatile int *moved, int tag)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (blockIdx.x == 0 && threadIdx.x < 15) pot[threadIdx.x] = 0.0;
@@ -691,7 +691,7 @@ __global__ void k_begin_force(int N, Box box, double half_skin2, const double *_
     const double dx = wrap1(p.x - rx0[i], box.L[0]);
     const double dy = wrap1(p.y - ry0[i], box.L[1]);
     const double dz = wrap1(p.z - rz0[i], box.L[2]);
-    if (dx * dx + dy * dy + dz * dz > half_skin2) flags[0] = tag;
+    if (dx * dx + dy * dy + dz * dz > half_skin2) *moved = tag;
 }
 
 // Pair-set fingerprint over the list: the j < i entries inside the cut-off.
@@ -1127,9 +1127,8 @@ void launch_begin_force(capac_ctx *c)
     if (++c->disp_tag <= 0) c->disp_tag = 1;
     k_begin_force<<<grid_for(c->N, 256), 256, 0, c->stream>>>(
         c->N, c->P.box, hs * hs, c->rx, c->ry, c->rz, c->charge, check ? c->rx0 : nullptr, c->ry0, c->rz0, c->pos4,
-        c->pos4f, c->fx, c->fy, c->fz, c->pot, c->vir, c->flags, c->disp_tag);
+        c->pos4f, c->fx, c->fy, c->fz, c->pot, c->vir, c->sig, c->disp_tag);
     ++c->launches;
-    CAPAC_CUDA(cudaMemcpyAsync(c->h_flags, c->flags, sizeof(int) * 4, cudaMemcpyDeviceToHost, c->stream));
     CAPAC_CUDA(cudaEventRecord(c->ev_flags, c->stream));
 }
 
@@ -1137,7 +1136,7 @@ void finish_begin_force(capac_ctx *c)
 {
     CAPAC_CUDA(cudaEventSynchronize(c->ev_flags));
     check_rattle(c);
-    if (!c->list_valid || c->h_flags[0] == c->disp_tag) build_list(c);
+    if (!c->list_valid || c->sig[0] == c->disp_tag) build_list(c);
 }
 
 void launch_pair_fingerprint(capac_ctx *c, int from_list, long *count, unsigned long long *hash)

@@ -251,7 +251,7 @@ constexpr int kRattleBlock = 128;
 
 // rattle_1st, force.c:1907-1997: one thread per molecule.
 __global__ void __launch_bounds__(kRattleBlock) k_rattle1(MdParams m, CstrView cv, double *rx, double *ry, double *rz, const double *ox,
-                          const double *oy, const double *oz, double *vx, double *vy, double *vz, int *flags)
+                          const double *oy, const double *oz, double *vx, double *vy, double *vz, volatile int *failed)
 {
     const int im = blockIdx.x * blockDim.x + threadIdx.x;
     if (im >= m.n_mols) return;
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kRattleBlock) k_rattle1(MdParams m, CstrView c
                 v[a][first + t] += dx * inv_dt;
             }
         }
-        if (!done) atomicOr(&flags[2], 1);
+        if (!done) *failed = 1;
         return;
     }
     while (!done) {
@@ -347,14 +347,14 @@ __global__ void __launch_bounds__(kRattleBlock) k_rattle1(MdParams m, CstrView c
         }
         if (++iter > kMaxIter) break;
     }
-    if (!done) atomicOr(&flags[2], 1);
+    if (!done) *failed = 1;
 }
 
 // rattle_2nd, force.c:2004-2090: one thread per molecule; the constraint
 // virial goes to per-block partials.
 __global__ void __launch_bounds__(kRattleBlock) k_rattle2(MdParams m, CstrView cv, const double *rx, const double *ry,
                                                  const double *rz, double *vx, double *vy, double *vz,
-                                                 int *flags, double *partials)
+                                                 volatile int *failed, double *partials)
 {
     __shared__ double sh[32 * 9];
     double vir[9] = {0.0};
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kRattleBlock) k_rattle2(MdParams m, CstrView c
             }
             if (++iter > kMaxIter) break;
         }
-        if (!done) atomicOr(&flags[2], 2);
+        if (!done) *failed = 1;
     }
     block_partials<9>(vir, sh, partials);
 }
@@ -740,11 +740,11 @@ void launch_rattle(capac_ctx *c, int second, bool in_step)
     const unsigned grid = grid_for(c->n_mols, kRattleBlock);
     if (!second) {
         k_rattle1<<<grid, kRattleBlock, 0, c->stream>>>(md_params(c), cstr_view(c), c->rx, c->ry, c->rz, c->ox, c->oy, c->oz,
-                                               c->vx, c->vy, c->vz, c->flags);
+                                               c->vx, c->vy, c->vz, c->sig + 1);
         ++c->launches;
     } else {
         k_rattle2<<<grid, kRattleBlock, 0, c->stream>>>(md_params(c), cstr_view(c), c->rx, c->ry, c->rz, c->vx, c->vy, c->vz,
-                                               c->flags, c->partials);
+                                               c->sig + 2, c->partials);
         ++c->launches;
         if (in_step) return;
         static const int pot_slots[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};

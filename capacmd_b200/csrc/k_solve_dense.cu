@@ -89,7 +89,8 @@ struct DenseArgs {
     double *x;
     ulonglong2 *ex;       // two exchange buffers of kSeg slots per block
     unsigned seq;         // number of the first exchange of this launch
-    SolverScalars *ss;
+    SolverScalars *ss;    // the error word that ends all polls
+    SolverScalars *out;   // pinned host memory: the result's scalars
     // mixed path
     DevParams P;
     const double4 *pos4;
@@ -215,6 +216,13 @@ __device__ __forceinline__ bool sum_all(double (&v)[K], double (*sh)[8], bool ba
     return true;
 }
 
+// A bounded wait has run out: the other blocks' polls end, the host is told.
+__device__ __forceinline__ void give_up(const DenseArgs &A)
+{
+    atomicExch(&A.ss->error, 1);
+    *(volatile int *)&A.out->error = 1;
+}
+
 // Store the block's kR values (thread q < kR holds row q) for exchange seq.
 __device__ __forceinline__ void publish(const DenseArgs &A, double v, unsigned seq)
 {
@@ -269,7 +277,7 @@ __device__ __forceinline__ bool receive(const DenseArgs &A, double (&out)[C], un
         }
         if (!all) {
             if (++spins > A.spin_limit) {
-                atomicExch(&A.ss->error, 1);
+                give_up(A);
                 bad = true;
             } else if ((spins & 63) == 0 && *(volatile int *)&A.ss->error != 0) {
                 bad = true;
@@ -327,15 +335,19 @@ __global__ void __launch_bounds__(kBlock, 1) k_bicgstab_dense(const __grid_const
         p[m] = v[m] = 0.0;
         d2[0] += bk * bk;
         d2[1] += xk != 0.0 ? 1.0 : 0.0;
-#pragma unroll
-        for (int q = 0; q < kR; ++q)
-            a[q][m] = !BJ && e < n && row0 + q < n ? tile_entry(A, row0 + q, e) : 0.0;
     }
     sum_all<2>(d2, vsh, false);
     const double bTb = d2[0], crit = bTb * A.tol;
     double rTr = 0.0, rr0 = 0.0;
     int iter = 0, status = 0, sweep = 0;
     bool done = bTb < A.skip;  // zero right-hand side: x stays (bicg_stab.c:303-307)
+#pragma unroll
+    for (int m = 0; m < C; ++m) {
+        const int e = tid + kBlock * m;
+#pragma unroll
+        for (int q = 0; q < kR; ++q)
+            a[q][m] = !BJ && !done && e < n && row0 + q < n ? tile_entry(A, row0 + q, e) : 0.0;
+    }
 
     if (BJ && !done) {
         // K's blocks stream through a ring of kStages slots of kStageRows rows
@@ -413,7 +425,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_bicgstab_dense(const __grid_const
                     // the copies in flight land in this block's shared memory:
                     // wait for them (bounded) before leaving
                     if (tid == 0) {
-                        atomicExch(&A.ss->error, 1);
+                        give_up(A);
                         for (int u = t; u < min(t + kStages, steps); ++u) mbar_wait(bars + u % kStages, (u / kStages) & 1);
                     }
                     return;
@@ -668,7 +680,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_bicgstab_dense(const __grid_const
             if (moved || predicted) A.x[rr] = xs[m][tid];
         }
         if (tid == 0) {
-            SolverScalars *ss = A.ss;
+            volatile SolverScalars *ss = A.out;
             ss->bTb = bTb;
             ss->crit = crit;
             ss->rTr = rTr;
@@ -752,6 +764,7 @@ int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double 
     A.x = x;
     A.ex = static_cast<ulonglong2 *>(c->dense_ex);
     A.ss = c->ss;
+    A.out = c->h_ss;
     A.P = c->P;
     A.pos4 = c->pos4;
     A.g_atoms = c->g_atoms;
@@ -777,7 +790,6 @@ int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double 
                                                dim3(kBlock), args, dense_smem(A.n, mixed), c->stream));
     }
     ++c->launches;
-    CAPAC_CUDA(cudaMemcpyAsync(c->h_ss, c->ss, sizeof(SolverScalars), cudaMemcpyDeviceToHost, c->stream));
     if (defer) return CAPAC_OK;
     CAPAC_CUDA(cudaStreamSynchronize(c->stream));
     return dense_status(c, skip);
@@ -786,6 +798,7 @@ int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double 
 int dense_status(capac_ctx *c, double skip)
 {
     if (c->h_ss->error) {
+        c->h_ss->error = 0;
         CAPAC_CUDA(cudaMemsetAsync(&c->ss->error, 0, sizeof(int), c->stream));
         throw Error(CAPAC_ERR_CUDA, "persistent solver: a bounded wait timed out");
     }
