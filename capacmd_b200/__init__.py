@@ -46,6 +46,10 @@ BT_ANGLE_HARMONIC, BT_ANGLE_UB, BT_DIHEDRAL_RB = 5, 6, 7
 PARAMS = ("cpff_capac", "cpff_polar", "cpim_rq", "cpim_rp", "qsc_eps", "qsc_c", "qsc_a", "qsc_n", "qsc_m")
 
 
+# capac_get arrays of one value per atom; every other has at most n_mat or 16
+_ATOM_ARRAYS = frozenset(a + b for a in "rvf" for b in "xyz")
+
+
 class CapacError(RuntimeError):
     def __init__(self, code: int, msg: str):
         super().__init__(f"[{code}] {msg}")
@@ -108,6 +112,7 @@ def lib() -> ctypes.CDLL:
     L.capac_md_steps.argtypes = [vp, ip]
     L.capac_get.argtypes = [vp, cp, vp]
     L.capac_set.argtypes = [vp, cp, vp]
+    L.capac_get_xyz.argtypes = [vp, ctypes.c_char, vp]
     L.capac_get_stats.argtypes = [vp, ctypes.POINTER(Stats)]
     L.capac_pair_fingerprint.argtypes = [vp, ip, ctypes.POINTER(ctypes.c_long),
                                          ctypes.POINTER(ctypes.c_ulonglong)]
@@ -207,7 +212,7 @@ class Simulation:
         """mpi_force with host arrays in and out (drop-in mode)."""
         N = self.n_atoms
         rx, ry, rz = (np.ascontiguousarray(a, dtype=np.float64) for a in (rx, ry, rz))
-        out = {k: np.zeros(N) for k in ("fx", "fy", "fz")}
+        out = {k: np.empty(N) for k in ("fx", "fy", "fz")}
         out["potential"] = np.zeros(15)
         out["virial"] = np.zeros(9)
         n = max(self.n_mat, 1)
@@ -248,19 +253,24 @@ class Simulation:
 
     # --- state --------------------------------------------------------------
     def get(self, name: str) -> np.ndarray:
-        out = np.zeros(max(self.n_atoms, self.n_mat, 16))
+        out = np.empty(self.n_atoms if name in _ATOM_ARRAYS else max(self.n_mat, 16))
         n = _check(lib().capac_get(self._p, name.encode(), out.ctypes.data))
-        return out[:n].copy()
+        return out if n == len(out) else out[:n].copy()
+
+    def _xyz(self, what: bytes) -> np.ndarray:
+        out = np.empty((self.n_atoms, 3))
+        _check(lib().capac_get_xyz(self._p, what, out.ctypes.data))
+        return out
 
     def set(self, name: str, values) -> None:
         v = np.ascontiguousarray(values, dtype=np.float64)
         _check(lib().capac_set(self._p, name.encode(), v.ctypes.data))
 
     def forces(self) -> np.ndarray:
-        return np.stack([self.get("fx"), self.get("fy"), self.get("fz")], 1)
+        return self._xyz(b"f")
 
     def positions(self) -> np.ndarray:
-        return np.stack([self.get("rx"), self.get("ry"), self.get("rz")], 1)
+        return self._xyz(b"r")
 
     def stats(self) -> Stats:
         s = Stats()

@@ -312,6 +312,12 @@ struct capac_ctx {
     int disp_tag = 0;            // tag of the last check
     bool phases = true;          // record the phase events of force calls
     cudaEvent_t ev_flags = nullptr;
+    // state transfer (see fetch): pinned staging, its chunk events, and the
+    // interleaved copy of capac_get_xyz, allocated on first use
+    unsigned char *stage = nullptr;
+    size_t stage_bytes = 0;
+    cudaEvent_t ev_stage[8] = {};
+    double *xyz = nullptr;
     bool pending_solve = false;  // the last solve's status is not read yet (settle_solve)
     double pending_tol = 0.0;
     double *pot = nullptr, *vir = nullptr;  // [15], [9]
@@ -426,6 +432,7 @@ void launch_rattle(capac_ctx *c, int second, bool in_step = false);
 void launch_step_sums(capac_ctx *c, int thermostat, bool rattle_virial);
 void launch_apply_pbc(capac_ctx *c);
 void launch_fmax_rms(capac_ctx *c);
+void launch_interleave(capac_ctx *c, const double *x, const double *y, const double *z, double *out);
 void launch_sum_potential(capac_ctx *c);
 void launch_build_vsites(capac_ctx *c);   // k_bonded.cu
 void launch_bonded(capac_ctx *c);

@@ -626,6 +626,17 @@ __global__ void k_fmax_final(const double *partials, int nb, int N, ThermoState 
     }
 }
 
+// (x, y, z) of each atom side by side.
+__global__ void k_interleave(int N, const double *__restrict__ x, const double *__restrict__ y,
+                             const double *__restrict__ z, double *__restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    out[3 * (size_t)i] = x[i];
+    out[3 * (size_t)i + 1] = y[i];
+    out[3 * (size_t)i + 2] = z[i];
+}
+
 // Energy minimisation step (mpi-main.c:730-756): old_r = r for every atom;
 // r += s / f_max * em_length except for fixed metal atoms.
 __global__ void k_em_move(MdParams m, const unsigned char *is_metal, const ThermoState *th, double em_length,
@@ -757,6 +768,12 @@ void launch_apply_pbc(capac_ctx *c)
 {
     k_apply_pbc<<<grid_for(c->n_mols, 256), 256, 0, c->stream>>>(md_params(c), c->mol_first, c->mol_last, c->rx,
                                                                 c->ry, c->rz);
+    ++c->launches;
+}
+
+void launch_interleave(capac_ctx *c, const double *x, const double *y, const double *z, double *out)
+{
+    k_interleave<<<grid_for(c->N, 256), 256, 0, c->stream>>>(c->N, x, y, z, out);
     ++c->launches;
 }
 

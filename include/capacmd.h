@@ -373,6 +373,9 @@ int capac_checkpoint_load(capac_ctx *ctx, const char *path);
  * returns the count written, <0 on error. */
 int capac_get(capac_ctx *ctx, const char *name, double *out);
 int capac_set(capac_ctx *ctx, const char *name, const double *in);
+/* Positions ('r'), velocities ('v') or forces ('f') of all atoms as x, y, z
+ * side by side: 3 n_atoms doubles. */
+int capac_get_xyz(capac_ctx *ctx, char what, double *out);
 
 /* Statistics of the last force call: BiCGSTAB iterations, neighbour-list
  * rebuilds so far, list entries, pairs inside the cut-off.  list_entries,
