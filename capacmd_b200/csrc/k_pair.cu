@@ -33,7 +33,9 @@ constexpr int kPairWarps = 8;  // warps per block
 // FP32 constants of the run.
 struct PairConstsF {
     float rc, inv_rc, inv_rc12, inv_rc6, alpha, a2_sqrtpi, w_const, w_erfc_arcut, fqq, rc2;
+    float gauss2;  // -alpha^2 log2(e)
     int use_vdw, use_coulomb;
+    double iL[3];  // 1 / box edge
 };
 
 // One type pair in FP32, with the shifted-force constants of funct 1
@@ -73,9 +75,8 @@ __device__ __forceinline__ float rcp_approx(float x)
 // (relative error of R below 4e-8 in exact arithmetic, 3e-7 in FP32).  The
 // caller has exp(-x^2) already, for the Gaussian term of the same pair.
 // Beyond x = 5 the library erfcf.
-__device__ __forceinline__ float erfc_from_gauss_f(float x, float gauss)
+__device__ __forceinline__ float erfc_near_f(float x, float gauss)
 {
-    if (x >= 5.0f) return erfcf(x);
     const float t = rcp_approx(fmaf(0.5f, x, 1.0f));
     float r = -3.71903017e-02f;
     r = fmaf(r, t, 1.64898831e-01f);
@@ -88,6 +89,10 @@ __device__ __forceinline__ float erfc_from_gauss_f(float x, float gauss)
     r = fmaf(r, t, 2.83852814e-01f);
     r = fmaf(r, t, -9.64172679e-05f);
     return gauss * r;
+}
+__device__ __forceinline__ float erfc_from_gauss_f(float x, float gauss)
+{
+    return x >= 5.0f ? erfcf(x) : erfc_near_f(x, gauss);
 }
 
 // FP64 pair term (force on j = f * rvec), reference formulas with the
@@ -492,16 +497,10 @@ __global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 3 : 2) k_
 // 128 pairs to the warp's queue (dynamic shared memory, kClQueue entries);
 // full flushes of 32 follow at one site, which keeps the pair terms in the
 // code once.
-//
-// HALF (pair_list 0, the default, or 2): the list holds every pair once (k_list.cu), so each
-// survivor's force goes to both ends: the member's slot as above, the
-// neighbour's by FP64 atomic adds, and energies and virial count in full.
-// The CPIM force on a charged water atom from a metal atom is taken from
-// whichever end holds the metal.  The atomic adds make the order of the
-// neighbour-side sums vary from run to run (FP64 rounding of FP32 terms).
 constexpr int kClQueue = 160;  // < 32 left over + 4 x 32 appended
 constexpr int kClWarps = 8;      // warps per block of the cluster kernel
 constexpr int kClMinBlocks = 2;  // resident blocks per SM the register budget allows
+constexpr int kHalfWarps = 4, kHalfBlocks = 5;  // the same for k_pair_half
 constexpr size_t kClQueueBytes = (size_t)kClWarps * kClQueue * (sizeof(float4) + sizeof(uint32_t));
 // A warp's queue as two arrays: the neighbour's FP32 difference from the
 // cluster centroid with its charge, and the list entry with the member
@@ -513,7 +512,7 @@ struct ClQueue {
     float4 *a;
     uint32_t *b;
 };
-template <bool NONBONDED, bool CPIM, bool HALF>
+template <bool NONBONDED, bool CPIM>
 __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevParams P, PairConstsF K, const double4 *__restrict__ pos4,
                                                               const int4 *__restrict__ cl_atoms,
                                                               const int *__restrict__ n_cl,
@@ -522,15 +521,13 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
                                                               const unsigned char *__restrict__ cl_metal, int cap,
                                                               const double *__restrict__ vec_pq,
                                                               double *__restrict__ fx, double *__restrict__ fy,
-                                                              double *__restrict__ fz, double *__restrict__ partials,
-                                                              int *__restrict__ next, const int *__restrict__ sel)
+                                                              double *__restrict__ fz, double *__restrict__ partials)
 {
     constexpr int NB = 2;
     extern __shared__ __align__(16) unsigned char s_dyn[];  // the warps' queues
     __shared__ float4 s_mem[kClWarps][4];  // member offset from the centroid, charge
     __shared__ int s_trow[kClWarps][4];    // member type * n_types
     __shared__ unsigned char s_cpim[kClWarps][4];  // the member takes the CPIM force of metal neighbours
-    __shared__ int s_mmetal[kClWarps][4];          // half list: the member's metal index, -1 not metal
     __shared__ double s_acc[kClWarps][12][32];  // force on (member, axis) per lane slot
     __shared__ double sh[32 * 11];
     __shared__ double wacc[kClWarps][8];
@@ -553,20 +550,9 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
     const double L[3] = {P.box.L[0], P.box.L[1], P.box.L[2]};
     const double iL[3] = {1.0 / L[0], 1.0 / L[1], 1.0 / L[2]};
     const int ncl = *n_cl;
-    // next (the half list): a resident grid whose warps take the next cluster
-    // from the counter (zeroed before the launch) until none is left, so
-    // list lengths that differ from cluster to cluster leave no warp idle at
-    // the end; else the fixed grid-stride order, which keeps the energy and
-    // virial sums in the same order from run to run
-    // sel: only the listed clusters (n_cl then counts them)
-    for (int k = 0;; ++k) {
-        int ci = blockIdx.x * kClWarps + wib + k * gridDim.x * kClWarps;
-        if (next) {
-            if (lane == 0) ci = atomicAdd(next, 1);
-            ci = __shfl_sync(0xffffffffu, ci, 0);
-        }
-        if (ci >= ncl) break;
-        const int cl = sel ? __ldg(sel + ci) : ci;
+    // fixed grid-stride order, which keeps the energy and virial sums in the
+    // same order from run to run
+    for (int cl = blockIdx.x * kClWarps + wib; cl < ncl; cl += gridDim.x * kClWarps) {
         const int4 A = cl_atoms[cl];
         const int nk = 1 + (A.y >= 0) + (A.z >= 0) + (A.w >= 0);
         const int mine = lane == 0 ? A.x : lane == 1 ? A.y : lane == 2 ? A.z : A.w;
@@ -596,7 +582,6 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
             s_mem[wib][lane] = make_float4((float)(ox - mx), (float)(oy - my), (float)(oz - mz), (float)pm.w);
             s_trow[wib][lane] = P.type[mine] * P.n_types;
             s_cpim[wib][lane] = CPIM && P.is_metal[mine] == 0 && pm.w != 0.0;
-            s_mmetal[wib][lane] = HALF && P.is_metal[mine] != 0 ? mine - P.metal_min : -1;
         }
 #pragma unroll
         for (int q = 0; q < 12; ++q) s_acc[wib][q][lane] = 0.0;
@@ -612,11 +597,8 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
         // pair terms of the queue entries head .. head + cnt - 1 into the
         // lanes' slots
         auto flush = [&](int head, int cnt) {
-            float hj0 = 0.f, hj1 = 0.f, hj2 = 0.f;  // half list: the neighbour's force of this lane's pair
-            int jj = -1;
             if (lane < cnt) {
                 float g0 = 0.f, g1 = 0.f, g2 = 0.f;
-                float n0 = 0.f, n1 = 0.f, n2 = 0.f;  // the pair force on the member (reversed on the half list)
                 const float4 bq4 = Q.a[head + lane];
                 Cand<float> c;
                 c.e = Q.b[head + lane];
@@ -636,9 +618,9 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
                     e_qq += (double)eq;
                     e_vdw += (double)ev;
                     const float gx = f * c.dx, gy = f * c.dy, gz = f * c.dz;
-                    g0 = n0 = -gx;
-                    g1 = n1 = -gy;
-                    g2 = n2 = -gz;
+                    g0 = -gx;
+                    g1 = -gy;
+                    g2 = -gz;
                     v[0] -= c.dx * gx; v[1] -= c.dx * gy; v[2] -= c.dx * gz;
                     v[3] -= c.dy * gy; v[4] -= c.dy * gz; v[5] -= c.dz * gz;
                 }
@@ -660,53 +642,6 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
                 s_acc[wib][3 * k][lane] += (double)g0;
                 s_acc[wib][3 * k + 1][lane] += (double)g1;
                 s_acc[wib][3 * k + 2][lane] += (double)g2;
-                if (HALF) {
-                    // the neighbour's side: the pair force reversed, and the
-                    // CPIM force on it when the member is the metal atom
-                    float h0 = -n0, h1 = -n1, h2 = -n2;
-                    const int mm = s_mmetal[wib][k];
-                    if (CPIM && cpim_cl && mm >= 0 && c.qj != 0.f) {
-                        const int j = (int)(c.e & kClIdxMask);
-                        const bool mj = metal_by_type ? s_metal[tj] != 0 : P.is_metal[j] != 0;
-                        if (!mj) {
-                            const float r[3] = {-c.dx, -c.dy, -c.dz};  // metal - atom
-                            const float p[3] = {(float)vec_pq[3 * mm], (float)vec_pq[3 * mm + 1],
-                                                (float)vec_pq[3 * mm + 2]};
-                            float g[3];
-                            cpim_charge_pair_f(K, r, c.r2, c.qj, (float)vec_pq[3 * P.M + mm], p, g);
-                            h0 -= g[0];
-                            h1 -= g[1];
-                            h2 -= g[2];
-                        }
-                    }
-                    hj0 = h0;
-                    hj1 = h1;
-                    hj2 = h2;
-                    jj = (int)(c.e & kClIdxMask);
-                }
-            }
-            if (HALF) {
-                // a neighbour's pairs are adjacent (at most four): sum them
-                // into the first lane of the run, which adds them to the atom
-                const int jl = lane < cnt ? jj : -1 - lane;
-#pragma unroll
-                for (int o = 1; o < 4; o <<= 1) {
-                    const float t0 = __shfl_down_sync(0xffffffffu, hj0, o);
-                    const float t1 = __shfl_down_sync(0xffffffffu, hj1, o);
-                    const float t2 = __shfl_down_sync(0xffffffffu, hj2, o);
-                    const int tj = __shfl_down_sync(0xffffffffu, jl, o);
-                    if (lane + o < 32 && tj == jl) {
-                        hj0 += t0;
-                        hj1 += t1;
-                        hj2 += t2;
-                    }
-                }
-                const int prev = __shfl_up_sync(0xffffffffu, jl, 1);
-                if (lane < cnt && (lane == 0 || prev != jl) && (hj0 != 0.f || hj1 != 0.f || hj2 != 0.f)) {
-                    atomicAdd(fx + jl, (double)hj0);
-                    atomicAdd(fy + jl, (double)hj1);
-                    atomicAdd(fz + jl, (double)hj2);
-                }
             }
         };
 
@@ -758,51 +693,19 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
                 const float bq = hi ? qj[1] : qj[0];
                 const unsigned bm = hi ? mask[1] : mask[0];
                 const uint32_t bk = hi ? keep[1] : keep[0];
-                if (HALF) {
-                    // each entry's survivors appended next to each other (the
-                    // flush sums a neighbour's pairs before its atomic adds)
-                    unsigned smask = 0;
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const float4 mk = s_mem[wib][kk];
-                        const float dx = bx - mk.x, dy = by - mk.y, dz = bz - mk.z;
-                        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                        if (((bm >> kk) & 1u) && r2 < K.rc2) smask |= 1u << kk;
+                for (int kk = 0; kk < 4; ++kk) {
+                    const float4 mk = s_mem[wib][kk];
+                    const float dx = bx - mk.x, dy = by - mk.y, dz = bz - mk.z;
+                    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                    const bool ok = ((bm >> kk) & 1u) && r2 < K.rc2;
+                    const unsigned ballot = __ballot_sync(0xffffffffu, ok);
+                    if (ok) {
+                        const int at = qn + __popc(ballot & lt_mask);
+                        Q.a[at] = make_float4(bx, by, bz, bq);
+                        Q.b[at] = bk | ((uint32_t)kk << kClMaskShift);
                     }
-                    const int cnt = __popc(smask);
-                    int incl = cnt;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                        if (lane >= o) incl += t;
-                    }
-                    int pos = qn + incl - cnt;
-#pragma unroll
-                    const float4 b4 = make_float4(bx, by, bz, bq);
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        if ((smask >> kk) & 1u) {
-                            Q.a[pos] = b4;
-                            Q.b[pos] = bk | ((uint32_t)kk << kClMaskShift);
-                            ++pos;
-                        }
-                    }
-                    qn += __shfl_sync(0xffffffffu, incl, 31);
-                } else {
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const float4 mk = s_mem[wib][kk];
-                        const float dx = bx - mk.x, dy = by - mk.y, dz = bz - mk.z;
-                        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                        const bool ok = ((bm >> kk) & 1u) && r2 < K.rc2;
-                        const unsigned ballot = __ballot_sync(0xffffffffu, ok);
-                        if (ok) {
-                            const int at = qn + __popc(ballot & lt_mask);
-                            Q.a[at] = make_float4(bx, by, bz, bq);
-                            Q.b[at] = bk | ((uint32_t)kk << kClMaskShift);
-                        }
-                        qn += __popc(ballot);
-                    }
+                    qn += __popc(ballot);
                 }
                 __syncwarp();
                 int head = 0;
@@ -840,10 +743,7 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
             for (int q = 0; q < 32; ++q) s += s_acc[wib][lane][(q + lane) & 31];
             const int atom = k == 0 ? A.x : k == 1 ? A.y : k == 2 ? A.z : A.w;
             double *f = a == 0 ? fx : (a == 1 ? fy : fz);
-            if (HALF)
-                atomicAdd(f + atom, s);  // other clusters add to this atom as a neighbour
-            else
-                f[atom] += s;
+            f[atom] += s;
         }
         if (NONBONDED) {
             const double t[8] = {warp_sum(e_qq), warp_sum(e_vdw), warp_sum((double)v[0]),
@@ -851,7 +751,7 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
                                  warp_sum((double)v[4]), warp_sum((double)v[5])};
             if (lane == 0) {
 #pragma unroll
-                for (int q = 0; q < 8; ++q) wacc[wib][q] += (HALF ? 1.0 : 0.5) * t[q];
+                for (int q = 0; q < 8; ++q) wacc[wib][q] += 0.5 * t[q];
             }
         }
         __syncwarp();
@@ -860,6 +760,355 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
         __syncthreads();
         double acc[11] = {0.0};
         if (threadIdx.x < kClWarps) {
+            const double *w = wacc[threadIdx.x];
+            acc[0] = w[0];
+            acc[1] = w[1];
+            acc[2] = w[2]; acc[3] = w[3]; acc[4] = w[4];
+            acc[5] = w[3]; acc[6] = w[5]; acc[7] = w[6];
+            acc[8] = w[4]; acc[9] = w[6]; acc[10] = w[7];
+        }
+        block_partials<11>(acc, sh, partials);
+    }
+}
+
+// A float times 2^-896 as a double, in three integer operations: the conversion
+// instruction runs at an eighth of their rate, and the half-list kernel takes five
+// a pair.  Moving the bits without correcting the exponent's bias gives the scale;
+// it is exact, zero and subnormals included, so sums formed at this scale and
+// multiplied by 2^896 at the end have the bits of plain FP64 sums.  Infinities and
+// NaN are not preserved and take scaled_any.
+constexpr float kScaledLimit = 1e30f;
+__device__ __forceinline__ double scaled(float v)
+{
+    const int u = __float_as_int(v);
+    return __hiloint2double((u >> 3) & 0x8fffffff, u << 29);
+}
+__device__ __forceinline__ double scaled_any(float v) { return (double)v * 0x1p-896; }
+
+__device__ __forceinline__ float exp2_approx(float x)
+{
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// min_image with the rounding by an addition of 1.5 2^52 instead of the rounding
+// instruction, which runs at a fraction of the FP64 rate.
+__device__ __forceinline__ double min_image_fma(double d, double L, double inv_L)
+{
+    return d - L * (fma(d, inv_L, 0x1.8p52) - 0x1.8p52);
+}
+
+__device__ __forceinline__ float rsqrt_approx(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Mixed path on the half cluster list (pair_list 0, the default, or 2; every
+// pair listed once, k_list.cu): one warp per cluster of up to four atoms, a lane
+// per entry.  A lane forms its neighbour's minimum-image difference from the
+// centroid in FP64, rounds it once, and goes through the cluster's members: the
+// pair's difference, r^2 and cut-off in FP32 as on the full list, and the pair
+// terms in place for the lanes that pass.  The members' forces and the energies
+// accumulate in the lane in FP64 (summed over the lanes at the end of the
+// cluster); the neighbour's force over its at most four pairs in FP32, added to
+// the atom by FP64 atomic adds.  The atomic adds make the order of the
+// neighbour-side sums vary from run to run (FP64 rounding of FP32 terms).
+//
+// Bound by instruction issue (70% of the slots, 20 of 32 lanes active: about 45%
+// of the lanes pass a member test, ~75 instructions a test with survivors).
+// Queueing the survivors so that the pair terms run on full warps, as the full
+// list does, costs more than the idle lanes: scans, 20 bytes written and read per
+// pair in shared memory, the forces read and added in shared slots, shuffles for
+// the neighbour's sum; 2.31 ms a call at 452,057 atoms and 0.51 at 91,122.
+// Pairs in place 2.99 and 0.69 with the general terms in the four unrolled
+// members (instruction cache misses); 1.51 and 0.44 with the short route below;
+// 1.39 and 0.34 with the positions loaded a chunk ahead, the general terms in a
+// rolled loop and five blocks of four warps (96 registers, no spills).
+//
+// Routes, chosen per cluster: `plain` where every type pair that can occur (all
+// of them for a cluster next to metal, else those of non-metal types) has funct 1
+// and the options are the shifted-force van der Waals and the damped Coulomb
+// form with alpha rc < 5, the range of the fitted erfc; `general` otherwise
+// (pair_term_f, all forms; also with more types than the shared tables hold).
+// The short route takes the Gaussian as 2^(-alpha^2 log2(e) r^2) from r^2 itself
+// and sharpens 1/r by a Newton step.  Against 64 bits, alpha 2, r 0.12..1.2 nm: the
+// Gaussian within 4e-7 (expf of the rounded (alpha r)^2: 1.5e-6), the Coulomb
+// force's rms error 9.80e-6 (9.84e-6) nm^-2, the energy's mean error weighted by r^2
+// -0.8e-9 (1.2e-9) and its rms 7.3e-9 (8.5e-9) nm.  The virial from the entry's
+// summed force instead of per pair is 1% faster and 15% less accurate.
+//
+// The water-side CPIM term walks the entries a second time, only for clusters next
+// to metal; taken from whichever end holds the metal.
+template <bool NONBONDED, bool CPIM>
+__global__ void __launch_bounds__(kHalfWarps * 32, kHalfBlocks) k_pair_half(
+    DevParams P, PairConstsF K, const double4 *__restrict__ pos4, const int4 *__restrict__ cl_atoms,
+    const int *__restrict__ n_cl, const uint32_t *__restrict__ nbr, const int *__restrict__ nnb,
+    const unsigned char *__restrict__ cl_metal, int cap, const double *__restrict__ vec_pq, double *__restrict__ fx,
+    double *__restrict__ fy, double *__restrict__ fz, double *__restrict__ partials, int *__restrict__ next,
+    const int *__restrict__ sel)
+{
+    __shared__ float4 s_mem[kHalfWarps][4];  // member offset from the centroid, charge
+    __shared__ int s_type[kHalfWarps][4];    // member type * n_types
+    __shared__ int s_mmetal[kHalfWarps][4];  // the member's metal index, -1 not metal
+    __shared__ double sh[32 * 11];
+    __shared__ double wacc[kHalfWarps][8];
+    __shared__ __align__(16) TypePairF s_tpf[kSmemTypes * kSmemTypes];
+    __shared__ unsigned char s_metal[kSmemTypes], s_vdw[kSmemTypes];  // s_vdw: 1 with a non-metal type, 2 with a metal
+    __shared__ __align__(16) float4 s_lj[kSmemTypes * kSmemTypes];     // c6, c12, fc, es
+    bool plain_near = false, plain_far = false;  // all type pairs, or all of non-metal types, have funct 1
+    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane < 8) wacc[wib][lane] = 0.0;
+    const bool smem_types = P.n_types <= kSmemTypes;
+    const bool metal_by_type = smem_types && P.metal_by_type;
+    if (smem_types) {
+        const int nt = P.n_types;
+        for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) s_tpf[k] = make_type_pair_f(P, K, k);
+        for (int k = threadIdx.x; k < nt; k += blockDim.x) s_metal[k] = P.type_metal[k];
+        __syncthreads();
+        for (int k = threadIdx.x; k < nt; k += blockDim.x) {
+            int f = metal_by_type ? 0 : 3;
+            for (int j = 0; j < nt; ++j) {
+                const TypePairF &t = s_tpf[k * nt + j];
+                if (t.fn != 1 || t.c6 != 0.f || t.c12 != 0.f) f |= s_metal[j] ? 2 : 1;
+            }
+            s_vdw[k] = (unsigned char)f;
+        }
+        bool near = true, far = true;
+        for (int k = threadIdx.x; k < nt * nt; k += blockDim.x) {
+            const TypePairF &t = s_tpf[k];
+            s_lj[k] = make_float4(t.c6, t.c12, t.fc, t.es);
+            near = near && t.fn == 1;
+            far = far && (t.fn == 1 || (metal_by_type && (s_metal[k / nt] || s_metal[k % nt])));
+        }
+        const bool dsf = K.use_vdw == 1 && K.use_coulomb == 1 && K.alpha * K.rc < 5.0f;
+        plain_near = __syncthreads_and(near) && dsf;
+        plain_far = __syncthreads_and(far) && dsf;
+    }
+    __syncthreads();
+    const double L[3] = {P.box.L[0], P.box.L[1], P.box.L[2]};
+    const double iL[3] = {K.iL[0], K.iL[1], K.iL[2]};
+    const int ncl = *n_cl;
+    const float rc2 = K.rc2;
+    // a resident grid whose warps take the next cluster from the counter
+    // (zeroed before the launch), so list lengths that differ from cluster to
+    // cluster leave no warp idle at the end; sel: only the listed clusters
+    for (;;) {
+        int ci = 0;
+        if (lane == 0) ci = atomicAdd(next, 1);
+        ci = __shfl_sync(0xffffffffu, ci, 0);
+        if (ci >= ncl) break;
+        const int cl = sel ? __ldg(sel + ci) : ci;
+        const int n = nnb[cl];
+        const uint32_t *row = nbr + (size_t)cl * cap;
+        const uint32_t first = lane < n ? __ldcs(row + lane) : 0u;
+        const int4 A = cl_atoms[cl];
+        const int nk = 1 + (A.y >= 0) + (A.z >= 0) + (A.w >= 0);
+        const int mine = lane == 0 ? A.x : lane == 1 ? A.y : lane == 2 ? A.z : A.w;
+        double4 pm = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (lane < nk) pm = pos4[mine];
+        const double x0 = __shfl_sync(0xffffffffu, pm.x, 0), y0 = __shfl_sync(0xffffffffu, pm.y, 0),
+                     z0 = __shfl_sync(0xffffffffu, pm.z, 0);
+        double ox = 0.0, oy = 0.0, oz = 0.0;
+        if (lane < nk) {
+            ox = min_image(pm.x - x0, L[0], iL[0]);
+            oy = min_image(pm.y - y0, L[1], iL[1]);
+            oz = min_image(pm.z - z0, L[2], iL[2]);
+        }
+        // member mean offset: lanes 0..3 hold the offsets, the others zero
+        double sx = ox, sy = oy, sz = oz;
+#pragma unroll
+        for (int o = 1; o <= 2; o <<= 1) {
+            sx += __shfl_xor_sync(0xffffffffu, sx, o);
+            sy += __shfl_xor_sync(0xffffffffu, sy, o);
+            sz += __shfl_xor_sync(0xffffffffu, sz, o);
+        }
+        const double inv_nk = 1.0 / nk;
+        const double mx = __shfl_sync(0xffffffffu, sx, 0) * inv_nk, my = __shfl_sync(0xffffffffu, sy, 0) * inv_nk,
+                     mz = __shfl_sync(0xffffffffu, sz, 0) * inv_nk;
+        const double cx = x0 + mx, cy = y0 + my, cz = z0 + mz;
+        const bool near_metal = cl_metal[cl] != 0, cpim_cl = CPIM && near_metal;
+        bool vdw = false;
+        __syncwarp();
+        if (lane < nk) {
+            const int ty = P.type[mine];
+            s_mem[wib][lane] = make_float4((float)(ox - mx), (float)(oy - my), (float)(oz - mz), (float)pm.w);
+            s_type[wib][lane] = ty * P.n_types;
+            vdw = smem_types && (s_vdw[ty] & (near_metal ? 3 : 1)) != 0;
+            s_mmetal[wib][lane] = P.is_metal[mine] != 0 ? mine - P.metal_min : -1;
+        }
+        const unsigned vmask = __ballot_sync(0xffffffffu, vdw);
+        const bool plain = NONBONDED && (near_metal ? plain_near : plain_far);
+        __syncwarp();
+        double f[16];  // force on member k, axis a at 3 k + a
+#pragma unroll
+        for (int q = 0; q < 16; ++q) f[q] = 0.0;
+        double e_qq = 0.0, e_vdw = 0.0;
+        float v[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) v[q] = 0.f;
+
+        // the entries of the row, `pairs` with each one's difference from the centroid
+        auto walk = [&](auto pairs) {
+            // the next chunk's positions are loaded while this one is computed, the
+            // entries one further ahead
+            uint32_t e = first, nxt = 32 + lane < n ? __ldcs(row + 32 + lane) : 0u;
+            double4 pj = pos4[e & kClIdxMask];
+            for (int base = 0; base < n; base += 32) {
+                const float bx = (float)min_image_fma(pj.x - cx, L[0], iL[0]);
+                const float by = (float)min_image_fma(pj.y - cy, L[1], iL[1]);
+                const float bz = (float)min_image_fma(pj.z - cz, L[2], iL[2]);
+                const float bq = (float)pj.w;
+                pj = pos4[nxt & kClIdxMask];
+                const uint32_t cur = e;
+                e = nxt;
+                const int k = base + 64 + lane;
+                nxt = k < n ? __ldcs(row + k) : 0u;
+                const int j = (int)(cur & kClIdxMask);
+                float h[3] = {0.f, 0.f, 0.f};  // force on the neighbour
+                // lanes past the end hold a zero entry: no mask bits
+                pairs(j, (int)(cur >> kClTypeShift), (cur >> kClMaskShift) & 15u, bx, by, bz, bq, h);
+                if (h[0] != 0.f || h[1] != 0.f || h[2] != 0.f) {
+                    atomicAdd(fx + j, (double)h[0]);
+                    atomicAdd(fy + j, (double)h[1]);
+                    atomicAdd(fz + j, (double)h[2]);
+                }
+            }
+        };
+        // pairs of any form with the members in `mask`; h null: only the sums that `scaled` takes
+        auto general = [&](int tj, unsigned mask, float bx, float by, float bz, float bq, float *h) {
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k) {
+                const float4 mk = s_mem[wib][k];
+                const float dx = bx - mk.x, dy = by - mk.y, dz = bz - mk.z;
+                const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                if (!(((mask >> k) & 1u) && r2 < rc2)) continue;
+                const int tp = s_type[wib][k] + tj;
+                float eq = 0.f, ev = 0.f;
+                const float fp = pair_term_f(K, smem_types ? s_tpf[tp] : make_type_pair_f(P, K, tp), mk.w, bq, r2, eq,
+                                             ev);
+                const float gx = fp * dx, gy = fp * dy, gz = fp * dz;
+                const double sx = scaled_any(gx), sy = scaled_any(gy), sz = scaled_any(gz);
+#pragma unroll
+                for (int m = 0; m < 4; ++m)
+                    if (m == k) {
+                        f[3 * m] -= sx;
+                        f[3 * m + 1] -= sy;
+                        f[3 * m + 2] -= sz;
+                    }
+                e_qq += scaled_any(eq);
+                e_vdw += scaled_any(ev);
+                if (h) {
+                    h[0] += gx;
+                    h[1] += gy;
+                    h[2] += gz;
+                    v[0] -= dx * gx; v[1] -= dx * gy; v[2] -= dx * gz;
+                    v[3] -= dy * gy; v[4] -= dy * gz; v[5] -= dz * gz;
+                }
+            }
+        };
+        if (plain) {
+            walk([&](int, int tj, unsigned mask, float bx, float by, float bz, float bq, float *h) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float4 mk = s_mem[wib][k];
+                    const float dx = bx - mk.x, dy = by - mk.y, dz = bz - mk.z;
+                    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                    if (!(((mask >> k) & 1u) && r2 < rc2)) continue;
+                    const float y = rsqrt_approx(r2), rinv = fmaf(0.5f * y, fmaf(-(r2 * y), y, 1.0f), y), r = r2 * rinv,
+                                r2inv = rinv * rinv;
+                    float fp = 0.f, eq = 0.f, ev = 0.f;
+                    if ((vmask >> k) & 1u) {
+                        const float4 t = s_lj[s_type[wib][k] + tj];
+                        if (t.x != 0.f || t.y != 0.f) {
+                            const float r6inv = r2inv * r2inv * r2inv, a6 = t.x * r6inv, a12 = t.y * (r6inv * r6inv);
+                            fp = (12.f * a12 - 6.f * a6 - t.z) * r2inv;
+                            ev = (a12 - a6) + (r - K.rc) * t.z * K.inv_rc - t.w;
+                        }
+                    }
+                    if (mk.w != 0.f && bq != 0.f) {
+                        const float qq = K.fqq * mk.w * bq, eg = exp2_approx(K.gauss2 * r2),
+                                    ec = erfc_near_f(K.alpha * r, eg);
+                        fp += qq * ((ec * r2inv + K.a2_sqrtpi * eg * rinv) - K.w_const) * rinv;
+                        eq = qq * (ec * rinv - K.w_erfc_arcut + K.w_const * (r - K.rc));
+                    }
+                    const float gx = fp * dx, gy = fp * dy, gz = fp * dz;
+                    if (fabsf(fp) < kScaledLimit) {
+                        f[3 * k] -= scaled(gx);
+                        f[3 * k + 1] -= scaled(gy);
+                        f[3 * k + 2] -= scaled(gz);
+                        e_qq += scaled(eq);
+                        e_vdw += scaled(ev);
+                    } else {
+                        f[3 * k] -= scaled_any(gx);
+                        f[3 * k + 1] -= scaled_any(gy);
+                        f[3 * k + 2] -= scaled_any(gz);
+                        e_qq += scaled_any(eq);
+                        e_vdw += scaled_any(ev);
+                    }
+                    h[0] += gx;
+                    h[1] += gy;
+                    h[2] += gz;
+                    v[0] -= dx * gx; v[1] -= dx * gy; v[2] -= dx * gz;
+                    v[3] -= dy * gy; v[4] -= dy * gz; v[5] -= dz * gz;
+                }
+            });
+        } else if (NONBONDED) {
+            walk([&](int, int tj, unsigned mask, float bx, float by, float bz, float bq, float *h) {
+                general(tj, mask, bx, by, bz, bq, h);
+            });
+        }
+        if (NONBONDED) {
+            double t[8] = {0x1p896 * e_qq, 0x1p896 * e_vdw, (double)v[0], (double)v[1], (double)v[2], (double)v[3],
+                           (double)v[4], (double)v[5]};
+            const double w = warp_sum_halving<8>(t, lane);
+            if ((lane & 3) == 0) wacc[wib][lane >> 2] += w;
+        }
+        if (cpim_cl) {
+            walk([&](int j, int tj, unsigned mask, float bx, float by, float bz, float bq, float *h) {
+                const bool mj = metal_by_type ? s_metal[tj] != 0 : mask != 0 && P.is_metal[j] != 0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float4 mk = s_mem[wib][k];
+                    const float dx = bx - mk.x, dy = by - mk.y, dz = bz - mk.z;
+                    const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                    const int mm = s_mmetal[wib][k];
+                    if (!(((mask >> k) & 1u) && r2 < rc2) || mj == (mm >= 0)) continue;
+                    // one of the two is metal
+                    const int m = mj ? j - P.metal_min : mm;
+                    const float q = mj ? mk.w : bq, sgn = mj ? 1.f : -1.f;
+                    if (q == 0.f) continue;
+                    const float r[3] = {sgn * dx, sgn * dy, sgn * dz};  // metal - atom
+                    const float p[3] = {(float)vec_pq[3 * m], (float)vec_pq[3 * m + 1], (float)vec_pq[3 * m + 2]};
+                    float g[3];
+                    cpim_charge_pair_f(K, r, r2, q, (float)vec_pq[3 * P.M + m], p, g);
+                    if (mj) {
+                        f[3 * k] -= scaled_any(g[0]);
+                        f[3 * k + 1] -= scaled_any(g[1]);
+                        f[3 * k + 2] -= scaled_any(g[2]);
+                    } else {
+                        h[0] -= g[0];
+                        h[1] -= g[1];
+                        h[2] -= g[2];
+                    }
+                }
+            });
+        }
+
+        // member forces: summed over the lanes, value q = 3 k + a in lane 2 q
+        const double sum = 0x1p896 * warp_sum_halving<16>(f, lane);
+        const int q = lane >> 1, k = q / 3, a = q - 3 * k;
+        if ((lane & 1) == 0 && k < nk) {
+            const int atom = k == 0 ? A.x : k == 1 ? A.y : k == 2 ? A.z : A.w;
+            double *out = a == 0 ? fx : (a == 1 ? fy : fz);
+            atomicAdd(out + atom, sum);  // other clusters add to this atom as a neighbour
+        }
+    }
+    if (NONBONDED) {
+        __syncthreads();
+        double acc[11] = {0.0};
+        if (threadIdx.x < kHalfWarps) {
             const double *w = wacc[threadIdx.x];
             acc[0] = w[0];
             acc[1] = w[1];
@@ -1061,8 +1310,10 @@ PairConstsF pair_consts_f(const capac_ctx *c)
     K.w_erfc_arcut = (float)c->P.w_erfc_arcut;
     K.fqq = (float)kFQQ;
     K.rc2 = (float)c->P.rc2;
+    K.gauss2 = (float)(-c->P.w_alpha * c->P.w_alpha * 1.4426950408889634074);
     K.use_vdw = c->P.use_vdw;
     K.use_coulomb = c->P.use_coulomb;
+    for (int a = 0; a < 3; ++a) K.iL[a] = 1.0 / c->P.box.L[a];
     return K;
 }
 
@@ -1085,18 +1336,27 @@ void launch_pair_t(capac_ctx *c, int mode, unsigned grid)
     ++c->launches;
 }
 
-// The cluster pair kernel on stream st, its block partials to `partials`;
-// sel: only the clusters with a metal member or neighbour.
-template <bool NONBONDED, bool CPIM, bool HALF>
-void launch_pair_cl_t(capac_ctx *c, unsigned grid, cudaStream_t st, double *partials, bool sel)
+// The full-list cluster kernel.
+template <bool NONBONDED, bool CPIM>
+void launch_pair_cl_t(capac_ctx *c, unsigned grid, double *partials)
 {
     // the queues and the static arrays together exceed the default 48 KB
-    CAPAC_CUDA(cudaFuncSetAttribute(k_pair_cl<NONBONDED, CPIM, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CAPAC_CUDA(cudaFuncSetAttribute(k_pair_cl<NONBONDED, CPIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kClQueueBytes));
-    if (HALF) CAPAC_CUDA(cudaMemsetAsync(c->cl_next, 0, sizeof(int), st));
-    k_pair_cl<NONBONDED, CPIM, HALF><<<grid, kClWarps * 32, kClQueueBytes, st>>>(
+    k_pair_cl<NONBONDED, CPIM><<<grid, kClWarps * 32, kClQueueBytes, c->stream>>>(
+        c->P, pair_consts_f(c), c->pos4, c->cl_atoms, c->cl_cell_start + c->n_cells, c->cl_nbr, c->cl_nnb, c->cl_metal,
+        c->cl_cap, c->vec_pq, c->fx, c->fy, c->fz, partials);
+}
+
+// The half-list cluster kernel on stream st, its block partials to `partials`;
+// sel: only the clusters with a metal member or neighbour.
+template <bool NONBONDED, bool CPIM>
+void launch_pair_half_t(capac_ctx *c, unsigned grid, cudaStream_t st, double *partials, bool sel)
+{
+    CAPAC_CUDA(cudaMemsetAsync(c->cl_next, 0, sizeof(int), st));
+    k_pair_half<NONBONDED, CPIM><<<grid, kHalfWarps * 32, 0, st>>>(
         c->P, pair_consts_f(c), c->pos4, c->cl_atoms, sel ? c->n_cl_sel : c->cl_cell_start + c->n_cells, c->cl_nbr,
-        c->cl_nnb, c->cl_metal, c->cl_cap, c->vec_pq, c->fx, c->fy, c->fz, partials, HALF ? c->cl_next : nullptr,
+        c->cl_nnb, c->cl_metal, c->cl_cap, c->vec_pq, c->fx, c->fy, c->fz, partials, c->cl_next,
         sel ? c->cl_sel : nullptr);
 }
 
@@ -1133,21 +1393,21 @@ void launch_pair_clusters(capac_ctx *c, int mode, unsigned grid)
         if (mode == 0 && cpim && c->pair_split) {
             // the pair terms without the CPIM branches, then the water-side
             // CPIM term over the clusters with a metal member or neighbour
-            launch_pair_cl_t<true, false, true>(c, grid, c->stream, part, false);
-            launch_pair_cl_t<false, true, true>(c, grid, c->stream, part, true);
+            launch_pair_half_t<true, false>(c, grid, c->stream, part, false);
+            launch_pair_half_t<false, true>(c, grid, c->stream, part, true);
             ++c->launches;
         } else if (mode == 0 && cpim)
-            launch_pair_cl_t<true, true, true>(c, grid, c->stream, part, false);
+            launch_pair_half_t<true, true>(c, grid, c->stream, part, false);
         else if (mode == 0)
-            launch_pair_cl_t<true, false, true>(c, grid, c->stream, part, false);
+            launch_pair_half_t<true, false>(c, grid, c->stream, part, false);
         else
-            launch_pair_cl_t<false, true, true>(c, grid, c->stream, part, false);
+            launch_pair_half_t<false, true>(c, grid, c->stream, part, false);
     } else if (mode == 0 && cpim)
-        launch_pair_cl_t<true, true, false>(c, grid, c->stream, part, false);
+        launch_pair_cl_t<true, true>(c, grid, part);
     else if (mode == 0)
-        launch_pair_cl_t<true, false, false>(c, grid, c->stream, part, false);
+        launch_pair_cl_t<true, false>(c, grid, part);
     else
-        launch_pair_cl_t<false, true, false>(c, grid, c->stream, part, false);
+        launch_pair_cl_t<false, true>(c, grid, part);
     ++c->launches;
 }
 
@@ -1160,14 +1420,14 @@ unsigned pair_grid(const capac_ctx *c)
 {
     if (c->cpairs) return (unsigned)c->num_sms * kCpMinBlocks;
     const long units = c->clusters ? c->n_clusters : c->N;
-    const int warps = c->clusters ? kClWarps : kPairWarps;
+    const int warps = c->clusters ? (c->cl_half ? kHalfWarps : kClWarps) : kPairWarps;
     const long need = (units + warps - 1) / warps;
-    const long cap = (long)c->num_sms * (c->clusters && c->cl_half ? kClMinBlocks : 16);
+    const long cap = (long)c->num_sms * (c->clusters && c->cl_half ? kHalfBlocks : 16);
     return (unsigned)std::max(1L, std::min(need, cap));
 }
 
 // Overlap, first half (on stream2, once `stream` has reached this point):
-// the nonbonded terms of the half cluster list, one block per SM so that the
+// the nonbonded terms of the half cluster list, two blocks per SM so that the
 // CPIM solve's blocks find room beside it; energies and virial into
 // partials2.  The forces go to fx, fy, fz by atomic adds only, so the
 // kernels that run meanwhile on `stream` must leave them alone (the CPIM
@@ -1179,9 +1439,9 @@ void launch_pair_nonbonded_async(capac_ctx *c)
     c->work_stream = c->stream2;
     {
         ProfScope ps(c, K_PAIR);
-        // one block per SM, and no more blocks than warps have clusters to take
-        c->async_grid = std::min((unsigned)c->num_sms, pair_grid(c));
-        launch_pair_cl_t<true, false, true>(c, c->async_grid, c->stream2, c->partials2, false);
+        // two blocks (eight warps) per SM, and no more blocks than warps have clusters to take
+        c->async_grid = std::min(2u * (unsigned)c->num_sms, pair_grid(c));
+        launch_pair_half_t<true, false>(c, c->async_grid, c->stream2, c->partials2, false);
     }
     c->work_stream = nullptr;
     ++c->launches;
@@ -1199,7 +1459,7 @@ void launch_pair_join(capac_ctx *c)
     launch_finalize(c, (int)c->async_grid, 11, pot_slots, vir_slots, c->partials2);
     {
         ProfScope ps(c, K_PAIR);
-        launch_pair_cl_t<false, true, true>(c, pair_grid(c), c->stream, c->partials, true);
+        launch_pair_half_t<false, true>(c, pair_grid(c), c->stream, c->partials, true);
     }
     ++c->launches;
 }
