@@ -312,8 +312,10 @@ struct capac_ctx {
     int disp_tag = 0;            // tag of the last check
     bool phases = true;          // record the phase events of force calls
     cudaEvent_t ev_flags = nullptr;
-    // state transfer (see fetch): pinned staging, its chunk events, and the
-    // interleaved copy of capac_get_xyz, allocated on first use
+    // state transfer (see fetch): pinned staging (in the block that also holds
+    // h_flags, sig, h_ss and h_th), its chunk events, and the interleaved copy of
+    // capac_get_xyz (behind fx, fy, fz)
+    void *pinned = nullptr;
     unsigned char *stage = nullptr;
     size_t stage_bytes = 0;
     cudaEvent_t ev_stage[8] = {};
