@@ -386,7 +386,8 @@ int capac_create(const capac_desc *d, const capac_options *opt, capac_ctx **out)
             }
             c->ox = dalloc<double>(N); c->oy = dalloc<double>(N); c->oz = dalloc<double>(N);
             c->rx0 = dalloc<double>(N); c->ry0 = dalloc<double>(N); c->rz0 = dalloc<double>(N);
-            c->pos4 = dalloc<double4>(N);
+            c->pos4 = dalloc<double4>(N + (N + 1) / 2);
+            c->pos4f = reinterpret_cast<float4 *>(c->pos4 + N);
 
             // topology
             c->type = dupload(d->atom_type, N, s);
@@ -718,7 +719,7 @@ int capac_destroy(capac_ctx *c)
     if (!c) return CAPAC_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
     void *dev[] = {c->rx, c->ry, c->rz, c->vx, c->vy, c->vz, c->fx, c->ox, c->oy, c->oz,
-                   c->rx0, c->ry0, c->rz0, c->pos4, c->pos4f, c->type, c->mol_id, c->mol_type,
+                   c->rx0, c->ry0, c->rz0, c->pos4, c->type, c->mol_id, c->mol_type,
                    c->atom_in_mol, c->is_metal, c->type_metal, c->charge, c->mass, c->inv_mass, c->mol_atoms,
                    c->excl_offset, c->excl, c->nb_funct, c->nb_par, c->mol_first, c->mol_last, c->cstr_off,
                    c->cstr_cnt, c->cstr_i, c->cstr_j, c->cstr_r, c->np_start, c->np_end, c->np_charge,

@@ -139,7 +139,7 @@ struct capac_ctx {
     double *rx = nullptr, *ry = nullptr, *rz = nullptr, *vx = nullptr, *vy = nullptr, *vz = nullptr;
     double *fx = nullptr, *fy = nullptr, *fz = nullptr, *ox = nullptr, *oy = nullptr, *oz = nullptr;
     double4 *pos4 = nullptr;  // (x, y, z, q) packed for gathers
-    float4 *pos4f = nullptr;  // mixed path: FP32 copy
+    float4 *pos4f = nullptr;  // its FP32 copy, behind it: k_pair's candidate test (not kept on the cluster lists)
     // topology
     int *type = nullptr, *mol_id = nullptr, *mol_type = nullptr, *atom_in_mol = nullptr;
     unsigned char *is_metal = nullptr;

@@ -1127,7 +1127,7 @@ void launch_begin_force(capac_ctx *c)
     if (++c->disp_tag <= 0) c->disp_tag = 1;
     k_begin_force<<<grid_for(c->N, 256), 256, 0, c->stream>>>(
         c->N, c->P.box, hs * hs, c->rx, c->ry, c->rz, c->charge, check ? c->rx0 : nullptr, c->ry0, c->rz0, c->pos4,
-        c->pos4f, c->fx, c->fy, c->fz, c->pot, c->vir, c->sig, c->disp_tag);
+        c->clusters || c->cpairs ? nullptr : c->pos4f, c->fx, c->fy, c->fz, c->pot, c->vir, c->sig, c->disp_tag);
     ++c->launches;
     CAPAC_CUDA(cudaEventRecord(c->ev_flags, c->stream));
 }
@@ -1136,7 +1136,11 @@ void finish_begin_force(capac_ctx *c)
 {
     CAPAC_CUDA(cudaEventSynchronize(c->ev_flags));
     check_rattle(c);
-    if (!c->list_valid || c->sig[0] == c->disp_tag) build_list(c);
+    if (!c->list_valid || c->sig[0] == c->disp_tag) {
+        const bool cl = c->clusters || c->cpairs;
+        build_list(c);
+        if (cl && !(c->clusters || c->cpairs)) launch_pack_positions(c);  // the FP32 copy too
+    }
 }
 
 void launch_pair_fingerprint(capac_ctx *c, int from_list, long *count, unsigned long long *hash)

@@ -9,8 +9,12 @@
 // list; every pair is visited from both ends, so forces need no atomics and
 // each end adds half of the pair energy and virial.  The cut-off test is done
 // in FP64 with the reference's r^2 rounding, so both precisions keep exactly
-// the reference's pair set.  Candidates that pass it are compacted into a
-// per-warp queue in shared memory and the pair math runs on full warps.
+// the reference's pair set.  Two passes: candidates (63% of the entries are
+// inside rc at a skin of 0.2) are first tested in FP32, with a margin that keeps
+// every pair the FP64 test accepts, and the entries that pass are compacted in
+// shared memory, 4 bytes each; then full warps form the FP64 difference, test it
+// and compute, their positions loaded one set ahead.  In FP64 the terms of an
+// ordinary pair are dsf_terms' ~55 operations.
 //
 // The same traversal adds, on each charged non-metal atom, the force from the
 // induced charges and dipoles of metal neighbours inside the cut-off: the
@@ -261,61 +265,80 @@ struct Acc<float> {
     __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
-// A candidate inside the cut-off, parked in the warp's queue: FP64 record
-// (48 B) for the FP64 path, FP32 record (24 B) for the mixed path.
-template <typename Real>
-struct Cand;
-template <>
-struct Cand<double> {
-    double dx, dy, dz, r2, qj;
-    uint32_t e;
-    int pad;
-};
-template <>
-struct Cand<float> {
-    float dx, dy, dz, r2, qj;
-    uint32_t e;
-};
-
 // Type-pair tables staged in shared memory when the type count allows.
 constexpr int kSmemTypes = 16;
 
-// Candidate chunks of 32 whose list entries and positions are loaded before
-// any is tested: more loads in flight per warp.
-template <typename Real>
-struct Batch {
-    static constexpr int N = 2;
-};
+// FP64 terms of a shifted-force Lennard-Jones and damped Coulomb pair (funct 1,
+// use_vdw = use_coulomb = 1, alpha rc < kDsfMaxX); t: c6, c12 and the type pair's
+// shifts of force and energy.
+__device__ __forceinline__ double pair_term_short(const DevParams &P, double inv_rc, const double4 &t, bool vdw, double qq,
+                                                  double r2, double &e_qq, double &e_vdw)
+{
+    const Dsf d = dsf_terms(P.w_alpha, r2);
+    const double r2inv = d.rinv * d.rinv;
+    double f = 0.0;
+    if (qq != 0.0) {
+        f = qq * (fma(d.ec, r2inv, P.w_a2_sqrtpi * d.eg * d.rinv) - P.w_const) * d.rinv;
+        e_qq = fma(qq, fma(d.ec, d.rinv, -P.w_erfc_arcut) + P.w_const * (d.r - P.rc), e_qq);
+    }
+    if (vdw && (t.x != 0.0 || t.y != 0.0)) {
+        const double r6inv = r2inv * r2inv * r2inv, a6 = t.x * r6inv, a12 = t.y * (r6inv * r6inv);
+        f += (12.0 * a12 - 6.0 * a6 - t.z) * r2inv;
+        e_vdw += (a12 - a6) + (d.r - P.rc) * (t.z * inv_rc) - t.w;
+    }
+    return f;
+}
+
+// The FP32 cut-off of the candidates of an atom at p (see k_pair): a pair whose
+// FP64 difference is inside rc has an FP32 r^2 below it.  Its coordinates are at
+// most A = max |p| + L + rc, so each FP32 coordinate is off by 2^-24 A, the
+// difference by less than 2^-21 (A + L) with the shift and its roundings; where the
+// shift itself is decided otherwise, the two images are equally far within that.
+__device__ __forceinline__ float candidate_cut(const DevParams &P, const double4 &p)
+{
+    const double L = fmax(P.box.L[0], fmax(P.box.L[1], P.box.L[2]));
+    const double A = fmax(fabs(p.x), fmax(fabs(p.y), fabs(p.z))) + 2.0 * L + P.rc;
+    const double r = P.rc + 0x1p-19 * A;
+    return __double2float_ru(r * r * 1.000001);
+}
+__device__ __forceinline__ float image1_f(float d, float L, float H) { return fabsf(d) > H ? d - copysignf(L, d) : d; }
+// pbc_12's single conditional shift of one axis (image)
+__device__ __forceinline__ double image1(double d, double L, double H) { return fabs(d) > H ? d - copysign(L, d) : d; }
 
 // One warp per atom i (grid-stride); see the file comment.
 template <typename Real, bool NONBONDED, bool CPIM>
-__global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 3 : 2) k_pair(DevParams P, PairConstsF K, const double4 *__restrict__ pos4,
-                                                           const uint32_t *__restrict__ nbr,
-                                                           const int *__restrict__ nnb, int cap,
-                                                           const double *__restrict__ vec_pq, double *__restrict__ fx,
-                                                           double *__restrict__ fy, double *__restrict__ fz,
-                                                           double *__restrict__ partials)
+__global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 3 : 2) k_pair(
+    DevParams P, PairConstsF K, const double4 *__restrict__ pos4, const float4 *__restrict__ pos4f,
+    const uint32_t *__restrict__ nbr, const int *__restrict__ nnb, int cap, const double *__restrict__ vec_pq,
+    double *__restrict__ fx, double *__restrict__ fy, double *__restrict__ fz, double *__restrict__ partials)
 {
-    constexpr int NB = Batch<Real>::N;
-    __shared__ Cand<Real> queue[kPairWarps][64];
+    constexpr int NB = 2;                            // chunks of 32 candidates tested together
+    __shared__ uint32_t queue[kPairWarps][32 * (NB + 1)];  // < 32 left over and NB x 32 appended
     __shared__ double sh[32 * 11];
     __shared__ double wacc[kPairWarps][8];  // per warp: e_qq, e_vdw, virial xx xy xz yy yz zz
     // type-pair table: double4 parameters (FP64) or TypePairF records (mixed), 32 B each
     __shared__ __align__(16) unsigned char s_tab[kSmemTypes * kSmemTypes * 32];
+    __shared__ double4 s_lj[sizeof(Real) == 8 ? kSmemTypes * kSmemTypes : 1];  // c6, c12 and pair_term's shift constants
     __shared__ int s_fn[kSmemTypes * kSmemTypes];
     __shared__ unsigned char s_metal[kSmemTypes];
     double4 *s_par = reinterpret_cast<double4 *>(s_tab);
     TypePairF *s_tpf = reinterpret_cast<TypePairF *>(s_tab);
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
-    Cand<Real> *Q = queue[wib];
+    uint32_t *Q = queue[wib];
     if (lane < 8) wacc[wib][lane] = 0.0;
     const bool smem_types = P.n_types <= kSmemTypes;
     if (smem_types) {
         const int nt2 = P.n_types * P.n_types;
         for (int k = threadIdx.x; k < nt2; k += blockDim.x) {
-            if constexpr (sizeof(Real) == 8) s_par[k] = P.nb_par[k];
-            else s_tpf[k] = make_type_pair_f(P, K, k);
+            if constexpr (sizeof(Real) == 8) {
+                const double4 t = P.nb_par[k];
+                s_par[k] = t;
+                s_lj[k] = make_double4(t.x, t.y, 12.0 * t.y * P.inv_rc12 - 6.0 * t.x * P.inv_rc6,
+                                       t.y * P.inv_rc12 - t.x * P.inv_rc6);
+            } else {
+                s_tpf[k] = make_type_pair_f(P, K, k);
+            }
             s_fn[k] = P.nb_funct[k];
         }
         for (int k = threadIdx.x; k < P.n_types; k += blockDim.x) s_metal[k] = P.type_metal[k];
@@ -328,11 +351,21 @@ __global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 3 : 2) k_
         Pt.nb_funct = s_fn;
     }
     const bool metal_by_type = smem_types && P.metal_by_type;
+    const bool damped = P.use_coulomb == 1 && P.w_alpha * P.rc < kDsfMaxX;
+    const bool shrt = smem_types && P.use_vdw == 1 && damped;
+    const double inv_rc = 1.0 / P.rc;
+    const float Lf[3] = {(float)P.box.L[0], (float)P.box.L[1], (float)P.box.L[2]};
+    const float Hf[3] = {(float)P.box.H[0], (float)P.box.H[1], (float)P.box.H[2]};
     const int stride = gridDim.x * kPairWarps;
     for (int i = blockIdx.x * kPairWarps + wib; i < P.N; i += stride) {
         const double4 pi = pos4[i];
+        const float xf = (float)pi.x, yf = (float)pi.y, zf = (float)pi.z, cut = candidate_cut(P, pi);
         const int trow = P.type[i] * P.n_types;
         const bool cpim_i = CPIM && P.is_metal[i] == 0 && pi.w != 0.0;
+        bool vdw_i = false;  // a type pair of this atom has Lennard-Jones terms
+        if (shrt)
+            for (int t = 0; t < P.n_types; ++t) vdw_i = vdw_i || s_par[trow + t].x != 0.0 || s_par[trow + t].y != 0.0;
+        const double qi = kFQQ * pi.w;
         const int n = nnb[i];
         const uint32_t *row = nbr + (size_t)i * cap;
         Acc<Real> f0, f1, f2;
@@ -341,15 +374,37 @@ __global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 3 : 2) k_
 #pragma unroll
         for (int q = 0; q < 6; ++q) v[q] = 0;
 
-        auto process = [&](const Cand<Real> &c) {
-            const Real dx = c.dx, dy = c.dy, dz = c.dz;
+        auto process = [&](uint32_t e, const double4 &pj, bool valid) {
+            const double ddx = image1(pj.x - pi.x, P.box.L[0], P.box.H[0]);
+            const double ddy = image1(pj.y - pi.y, P.box.L[1], P.box.H[1]);
+            const double ddz = image1(pj.z - pi.z, P.box.L[2], P.box.H[2]);
+            const Real dx = (Real)ddx, dy = (Real)ddy, dz = (Real)ddz;
+            Real r2;
+            bool ok;
+            if constexpr (sizeof(Real) == 8) {
+                // the reference's rounding of r^2: the FP64 pair set is the reference's
+                r2 = norm2_exact(ddx, ddy, ddz);
+                ok = valid && r2 < P.rc2;
+            } else {
+                // mixed: r^2 and the cut-off in FP32 from the FP64 minimum-image
+                // difference; pairs within rounding of the cut-off contribute
+                // nothing (shifted force and energy vanish there)
+                r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                ok = valid && r2 < K.rc2;
+            }
+            if (!ok) return;
+            const int tj = nb_type(e);
             if (NONBONDED) {
                 Real f;
-                if constexpr (sizeof(Real) == 8)
-                    f = pair_term(Pt, trow + nb_type(c.e), pi.w, c.qj, c.r2, e_qq, e_vdw);
-                else
-                    f = pair_term_f(K, smem_types ? s_tpf[trow + nb_type(c.e)] : make_type_pair_f(P, K, trow + nb_type(c.e)),
-                                    (float)pi.w, c.qj, c.r2, e_qq, e_vdw);
+                if constexpr (sizeof(Real) == 8) {
+                    if (shrt && s_fn[trow + tj] == 1)
+                        f = pair_term_short(P, inv_rc, s_lj[trow + tj], vdw_i, qi * pj.w, r2, e_qq, e_vdw);
+                    else
+                        f = pair_term(Pt, trow + tj, pi.w, pj.w, r2, e_qq, e_vdw);
+                } else {
+                    f = pair_term_f(K, smem_types ? s_tpf[trow + tj] : make_type_pair_f(P, K, trow + tj), (float)pi.w,
+                                    (float)pj.w, r2, e_qq, e_vdw);
+                }
                 const Real gx = f * dx, gy = f * dy, gz = f * dz;
                 f0.add(-gx);
                 f1.add(-gy);
@@ -358,97 +413,82 @@ __global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 3 : 2) k_
                 v[3] -= dy * gy; v[4] -= dy * gz; v[5] -= dz * gz;
             }
             if (cpim_i) {
-                const int j = nb_index(c.e);
-                const bool mj = metal_by_type ? s_metal[nb_type(c.e)] != 0 : P.is_metal[j] != 0;
+                const int j = nb_index(e);
+                const bool mj = metal_by_type ? s_metal[tj] != 0 : P.is_metal[j] != 0;
                 if (mj) {
                     const int jm = j - P.metal_min;
+                    Real g[3];
+                    const Real r[3] = {dx, dy, dz};  // metal - atom
+                    const Real p[3] = {(Real)vec_pq[3 * jm], (Real)vec_pq[3 * jm + 1], (Real)vec_pq[3 * jm + 2]};
+                    const Real q = (Real)vec_pq[3 * P.M + jm];
                     if constexpr (sizeof(Real) == 8) {
-                        const double r[3] = {c.dx, c.dy, c.dz};  // metal - atom
-                        const double p[3] = {vec_pq[3 * jm], vec_pq[3 * jm + 1], vec_pq[3 * jm + 2]};
-                        double g[3], a0, ec;
-                        cpim_charge_pair(P, r, c.r2, pi.w, vec_pq[3 * P.M + jm], p, g, a0, ec);
-                        f0.add(-g[0]);
-                        f1.add(-g[1]);
-                        f2.add(-g[2]);
+                        double a0, ec;
+                        if (damped)
+                            cpim_charge_pair_dsf(P, r, r2, pi.w, q, p, g);
+                        else
+                            cpim_charge_pair(P, r, r2, pi.w, q, p, g, a0, ec);
                     } else {
-                        const float r[3] = {c.dx, c.dy, c.dz};
-                        const float p[3] = {(float)vec_pq[3 * jm], (float)vec_pq[3 * jm + 1],
-                                            (float)vec_pq[3 * jm + 2]};
-                        float g[3];
-                        cpim_charge_pair_f(K, r, c.r2, (float)pi.w, (float)vec_pq[3 * P.M + jm], p, g);
-                        f0.add(-g[0]);
-                        f1.add(-g[1]);
-                        f2.add(-g[2]);
+                        cpim_charge_pair_f(K, r, r2, (float)pi.w, q, p, g);
                     }
+                    f0.add(-g[0]);
+                    f1.add(-g[1]);
+                    f2.add(-g[2]);
                 }
             }
         };
 
-        int qn = 0;  // queue fill, warp-uniform
-        // list entries are loaded one batch ahead (the list streams from
-        // HBM once per step, evict-first)
-        uint32_t nxt[NB];
+        // candidates: entries and FP32 positions of the next batch are loaded while
+        // this one is tested (the list streams from HBM once per step, evict-first)
+        uint32_t ev[NB], nxt[NB];
+        float4 pf[NB];
 #pragma unroll
         for (int u = 0; u < NB; ++u) {
-            const int k = u * 32 + lane;
-            nxt[u] = k < n ? __ldcs(row + k) : 0u;
+            const int k = u * 32 + lane, k2 = (NB + u) * 32 + lane;
+            ev[u] = k < n ? __ldcs(row + k) : 0u;
+            nxt[u] = k2 < n ? __ldcs(row + k2) : 0u;
         }
-        for (int base = 0; base < n; base += 32 * NB) {
-            uint32_t ev[NB];
-            bool valid[NB];
 #pragma unroll
-            for (int u = 0; u < NB; ++u) {
-                valid[u] = base + u * 32 + lane < n;
-                ev[u] = nxt[u];
-                const int k = base + (NB + u) * 32 + lane;
-                nxt[u] = k < n ? __ldcs(row + k) : 0u;
-            }
-            double4 pj[NB];
+        for (int u = 0; u < NB; ++u) pf[u] = pos4f[nb_index(ev[u])];
+        // survivors: popped 32 at a time, their FP64 positions loaded one pop ahead
+        int qn = 0, base = 0, cnt = -1;  // queue fill, next batch, size of the popped set (warp-uniform)
+        uint32_t ec = 0;
+        double4 pc = make_double4(0.0, 0.0, 0.0, 0.0);
+        for (;;) {
+            while (qn < 32 && base < n) {
 #pragma unroll
-            for (int u = 0; u < NB; ++u)
-                if (valid[u]) pj[u] = pos4[nb_index(ev[u])];
-#pragma unroll
-            for (int u = 0; u < NB; ++u) {
-                bool ok = false;
-                Cand<Real> c;
-                if (valid[u]) {
-                    double dx = pj[u].x - pi.x, dy = pj[u].y - pi.y, dz = pj[u].z - pi.z;
-                    image(dx, dy, dz, P.box);
-                    if constexpr (sizeof(Real) == 8) {
-                        // the reference's rounding of r^2: the FP64 pair set is the reference's
-                        const double r2 = norm2_exact(dx, dy, dz);
-                        ok = r2 < P.rc2;
-                        c.r2 = r2;
-                    } else {
-                        // mixed: r^2 and the cut-off in FP32 from the FP64 minimum-image
-                        // difference; pairs within rounding of the cut-off contribute
-                        // nothing (shifted force and energy vanish there)
-                        const float fx = (float)dx, fy = (float)dy, fz = (float)dz;
-                        const float r2 = fmaf(fz, fz, fmaf(fy, fy, fx * fx));
-                        ok = r2 < K.rc2;
-                        c.r2 = r2;
-                    }
-                    c.dx = (Real)dx;
-                    c.dy = (Real)dy;
-                    c.dz = (Real)dz;
-                    c.qj = (Real)pj[u].w;
-                    c.e = ev[u];
+                for (int u = 0; u < NB; ++u) {
+                    const float dx = image1_f(pf[u].x - xf, Lf[0], Hf[0]), dy = image1_f(pf[u].y - yf, Lf[1], Hf[1]),
+                                dz = image1_f(pf[u].z - zf, Lf[2], Hf[2]);
+                    const bool ok = base + u * 32 + lane < n && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < cut;
+                    const unsigned ballot = __ballot_sync(0xffffffffu, ok);
+                    if (ok) Q[qn + __popc(ballot & lt_mask)] = ev[u];
+                    qn += __popc(ballot);
                 }
-                const unsigned ballot = __ballot_sync(0xffffffffu, ok);
-                if (ok) Q[qn + __popc(ballot & lt_mask)] = c;
-                qn += __popc(ballot);
+                base += 32 * NB;
+#pragma unroll
+                for (int u = 0; u < NB; ++u) {
+                    ev[u] = nxt[u];
+                    pf[u] = pos4f[nb_index(ev[u])];
+                    const int k = base + (NB + u) * 32 + lane;
+                    nxt[u] = k < n ? __ldcs(row + k) : 0u;
+                }
                 __syncwarp();
-                if (qn >= 32) {
-                    process(Q[lane]);
-                    __syncwarp();
-                    if (lane < qn - 32) Q[lane] = Q[lane + 32];
-                    __syncwarp();
-                    qn -= 32;
-                }
             }
+            const int take = min(qn, 32);
+            uint32_t e2 = 0;
+            double4 p2 = pc;
+            if (lane < take) {
+                e2 = Q[qn - take + lane];
+                p2 = pos4[nb_index(e2)];
+            }
+            qn -= take;
+            __syncwarp();
+            if (cnt > 0) process(ec, pc, lane < cnt);
+            if (take == 0) break;
+            ec = e2;
+            pc = p2;
+            cnt = take;
         }
-        if (lane < qn) process(Q[lane]);
-        __syncwarp();
 
         const double s0 = warp_sum(f0.value()), s1 = warp_sum(f1.value()), s2 = warp_sum(f2.value());
         if (lane == 0) {
@@ -457,13 +497,10 @@ __global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 3 : 2) k_
             fz[i] += s2;
         }
         if (NONBONDED) {
-            const double t[8] = {warp_sum((double)e_qq), warp_sum((double)e_vdw), warp_sum((double)v[0]),
-                                 warp_sum((double)v[1]), warp_sum((double)v[2]), warp_sum((double)v[3]),
-                                 warp_sum((double)v[4]), warp_sum((double)v[5])};
-            if (lane == 0) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) wacc[wib][q] += 0.5 * t[q];
-            }
+            double t[8] = {(double)e_qq, (double)e_vdw, (double)v[0], (double)v[1], (double)v[2], (double)v[3],
+                           (double)v[4], (double)v[5]};
+            const double w = warp_sum_halving<8>(t, lane);
+            if ((lane & 3) == 0) wacc[wib][lane >> 2] += 0.5 * w;
         }
     }
     if (NONBONDED) {
@@ -511,6 +548,10 @@ constexpr size_t kClQueueBytes = (size_t)kClWarps * kClQueue * (sizeof(float4) +
 struct ClQueue {
     float4 *a;
     uint32_t *b;
+};
+struct ClPair {
+    float dx, dy, dz, r2, qj;
+    uint32_t e;
 };
 template <bool NONBONDED, bool CPIM>
 __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevParams P, PairConstsF K, const double4 *__restrict__ pos4,
@@ -600,7 +641,7 @@ __global__ void __launch_bounds__(kClWarps * 32, kClMinBlocks) k_pair_cl(DevPara
             if (lane < cnt) {
                 float g0 = 0.f, g1 = 0.f, g2 = 0.f;
                 const float4 bq4 = Q.a[head + lane];
-                Cand<float> c;
+                ClPair c;
                 c.e = Q.b[head + lane];
                 const int k = (int)((c.e >> kClMaskShift) & 3u);
                 const int tj = (int)(c.e >> kClTypeShift);
@@ -1325,13 +1366,13 @@ void launch_pair_t(capac_ctx *c, int mode, unsigned grid)
     double *part = force_partials(c, FP_PAIR);
     ProfScope ps(c, K_PAIR);
     if (mode == 0 && cpim)
-        k_pair<Real, true, true><<<grid, kPairWarps * 32, 0, c->stream>>>(c->P, K, c->pos4, c->nbr, c->nnb, c->cap,
+        k_pair<Real, true, true><<<grid, kPairWarps * 32, 0, c->stream>>>(c->P, K, c->pos4, c->pos4f, c->nbr, c->nnb, c->cap,
                                                                           c->vec_pq, c->fx, c->fy, c->fz, part);
     else if (mode == 0)
-        k_pair<Real, true, false><<<grid, kPairWarps * 32, 0, c->stream>>>(c->P, K, c->pos4, c->nbr, c->nnb, c->cap,
+        k_pair<Real, true, false><<<grid, kPairWarps * 32, 0, c->stream>>>(c->P, K, c->pos4, c->pos4f, c->nbr, c->nnb, c->cap,
                                                                            c->vec_pq, c->fx, c->fy, c->fz, part);
     else
-        k_pair<Real, false, true><<<grid, kPairWarps * 32, 0, c->stream>>>(c->P, K, c->pos4, c->nbr, c->nnb, c->cap,
+        k_pair<Real, false, true><<<grid, kPairWarps * 32, 0, c->stream>>>(c->P, K, c->pos4, c->pos4f, c->nbr, c->nnb, c->cap,
                                                                            c->vec_pq, c->fx, c->fy, c->fz, part);
     ++c->launches;
 }

@@ -5,6 +5,88 @@
 
 namespace capac {
 
+// exp(-x^2) and erfc(x) with x = alpha r, and 1/r, of one damped Coulomb pair,
+// for alpha r < kDsfMaxX: no branch and no call, ~55 FP64 operations where
+// sqrt, the division, exp and erfc take about 200.
+//
+// 1/r: the hardware approximation and one step of third order (remainder
+// 5/16 e^3 of an e below 2^-19).  exp(-x^2): x^2 with its rounding error, 2^n
+// split off, and 1 + f + f^2 q(f) on |f| <= ln2 / 2 with q a Chebyshev
+// interpolant (1.6e-17 of the result).  erfc(x) = exp(-x^2) R(x), R the scaled
+// complementary error function as a polynomial of degree 18 in
+// u = (x - 3.5) / (x + 3.5), Chebyshev interpolant on [0, 5] (3.7e-17 of R with
+// the rounded coefficients); both polynomials in two chains.
+constexpr double kDsfMaxX = 5.0;
+struct Dsf {
+    double rinv, r, eg, ec;
+};
+__device__ __forceinline__ Dsf dsf_terms(double alpha, double r2)
+{
+    Dsf d;
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+    double e = fma(-r2 * y, y, 1.0);
+    d.rinv = fma(y * e, fma(0.375, e, 0.5), y);
+    d.r = r2 * d.rinv;
+    const double x = alpha * d.r;
+    // exp(-x^2): n = round(-x^2 log2 e) from the low word of an addition to 1.5 2^52
+    const double x2 = x * x, lo = fma(x, x, -x2);
+    const double kd = fma(x2, -1.4426950408889634, 0x1.8p52), n = kd - 0x1.8p52;
+    const double f = fma(n, -0x1.473de6af278edp-34, fma(n, -0x1.62e42fef00000p-1, -x2)) - lo;
+    const double f2 = f * f;
+    double a = fma(2.51003759291859252e-08, f2, 2.75572684801069265e-06);
+    a = fma(a, f2, 1.98412698630406751e-04);
+    a = fma(a, f2, 8.33333333333006500e-03);
+    a = fma(a, f2, 1.66666666666666685e-01);
+    double b = fma(2.76200760056313823e-07, f2, 2.48015213221045905e-05);
+    b = fma(b, f2, 1.38888889171968899e-03);
+    b = fma(b, f2, 4.16666666666241636e-02);
+    b = fma(b, f2, 5.00000000000000111e-01);
+    const double g = 1.0 + fma(f2, fma(a, f, b), f);
+    d.eg = __hiloint2double(__double2hiint(g) + (__double2loint(kd) << 20), __double2loint(g));
+    // R(x)
+    const double z = x + 3.5;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(z));
+    e = fma(-z, y, 1.0);
+    const double u = fma(-7.0, fma(y, fma(e, e, e), y), 1.0), u2 = u * u;
+    a = fma(1.44851080807840048e-07, u2, 9.39502676422655287e-07);
+    a = fma(a, u2, -1.35300964606639283e-06);
+    a = fma(a, u2, -4.65943681772681595e-06);
+    a = fma(a, u2, 2.88553311039605571e-04);
+    a = fma(a, u2, -4.24223856269931136e-03);
+    a = fma(a, u2, -4.54367611836835258e-02);
+    a = fma(a, u2, -1.61338524764510272e-01);
+    a = fma(a, u2, -2.89265044832767437e-01);
+    b = fma(1.21445591197839242e-08, u2, 6.32563657300747914e-07);
+    b = fma(b, u2, -1.03347250494745519e-06);
+    b = fma(b, u2, 1.34428888195974961e-05);
+    b = fma(b, u2, -1.08088183803848795e-04);
+    b = fma(b, u2, 2.67384873232049400e-04);
+    b = fma(b, u2, 1.69767609425404628e-02);
+    b = fma(b, u2, 9.44278069090268707e-02);
+    b = fma(b, u2, 2.33130481600251627e-01);
+    b = fma(b, u2, 1.55293655608894299e-01);
+    d.ec = d.eg * fma(a, u, b);
+    return d;
+}
+
+// cpim_charge_pair with the damped form and alpha r < kDsfMaxX.
+__device__ __forceinline__ void cpim_charge_pair_dsf(const DevParams &P, const double r[3], double r2, double q_perm,
+                                                     double q_ind, const double p[3], double f[3])
+{
+    const Dsf d = dsf_terms(P.w_alpha, r2);
+    const double r2inv = d.rinv * d.rinv, ir3 = r2inv * d.rinv, al3 = P.w_alpha * P.w_alpha * P.w_alpha;
+    const double s = kFQQ * q_perm, sp = s / kNm2Bohr;
+    const double a0 = fma(d.ec, r2inv, P.w_a2_sqrtpi * d.eg * d.rinv) - P.w_const;
+    const double a1 = ir3 * r2inv * fma(P.w_a2_sqrtpi * d.r, d.eg, d.ec), b1 = 4.0 * kInvSqrtPi * al3 * r2inv * d.eg,
+                 c1 = P.w_const * ir3;
+    const double pr = p[0] * r[0] + p[1] * r[1] + p[2] * r[2];
+    // sum_a T_ab p_a, T_ab = a1 (3 r_a r_b - d_ab r^2) + b1 r_a r_b - c1 (r_a r_b - d_ab r^2)
+    const double along = fma(a0 * d.rinv, s * q_ind, -(3.0 * a1 + b1 - c1) * pr * sp), off = (a1 - c1) * r2 * sp;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) f[b] = fma(along, r[b], off * p[b]);
+}
+
 // Force on the metal atom from the permanent charge q of a non-metal atom at
 // metal - atom separation r (nm); the atom receives the opposite force.
 // cpff.c:604-702.  Returns through f[3]; also gives const_a0 for energy [11].
