@@ -165,7 +165,7 @@ struct capac_ctx {
     int n_cells = 1;
     int *cell_key = nullptr, *cell_key_sorted = nullptr, *atom_ids = nullptr, *cell_atoms = nullptr;
     int *cell_start = nullptr;   // [n_cells + 1] first sorted position of each cell
-    double4 *spos = nullptr;     // [N] positions in cell order, atom index in w
+    float4 *spos = nullptr;      // [N] wrapped positions in cell order, list entry (atom, type) in w
     void *sort_tmp = nullptr;
     size_t sort_tmp_bytes = 0;
     int *flags = nullptr;      // [0] rebuild needed (stage calls), [1] list overflow max count,
@@ -193,7 +193,7 @@ struct capac_ctx {
     unsigned char *cl_metal = nullptr; // [cl_max] the cluster has a metal neighbour (or, on the
                                        // half list, a metal member)
     bool cl_half = false;              // half list: every pair once, Newton's third law (pair_list 2)
-    int *cl_of = nullptr;              // [N] the cluster of each atom (half list)
+    int *cl_first = nullptr;           // [cl_max] sorted position of each cluster's first member
     int *cl_next = nullptr;            // the cluster pair kernel's work counter (next cluster to take)
     int *cl_sel = nullptr;             // [cl_max] clusters with a metal member or neighbour (any order)
     int *n_cl_sel = nullptr;           // their count (device)

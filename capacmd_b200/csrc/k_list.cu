@@ -4,9 +4,10 @@
 // visits every j < i and keeps a pair when it is not excluded and
 // dist_2(pbc_12(r_j - r_i)) < rCut^2.  Here atoms are binned into cells of edge
 // >= (rc + skin) / 2 (wrapped coordinates) and sorted by cell, with a
-// cell-ordered copy of the positions; each atom's full list holds every
-// non-excluded j within rc + skin under the same pbc_12 metric on the
-// unwrapped coordinates.  A warp scans the 5 x 5 cells around its atom in x
+// cell-ordered FP32 copy of the wrapped positions; each atom's full list holds
+// every non-excluded j within rc + skin, the radius widened beyond the rounding
+// (a superset of the pairs under the pbc_12 metric on the unwrapped
+// coordinates, whose distance is at least the nearest image's).  A warp scans the 5 x 5 cells around its atom in x
 // and y, each as one contiguous run of five z cells of the sorted copy
 // (coalesced loads), tests the distance first and the exclusions only for
 // the survivors.  The pair kernel re-applies the exact FP64 cut-off
@@ -23,10 +24,9 @@
 // Mixed path, cluster list: the atoms of each cell are cut, in that order,
 // into clusters of up to four.  Per cluster a warp scans the same 5 x 5 x 5
 // cell window; a candidate j within rc + skin + (cluster radius) of the
-// cluster's centroid is tested against each member k in FP32 (j's FP64
-// minimum image from the centroid, rounded, minus the member's offset) with
-// the list radius widened by 1e-5 relative, far beyond the rounding, and
-// against the exclusions, and kept with the mask of the members that pass.
+// cluster's centroid is tested against each member k in FP32 (j's
+// difference from the centroid minus the member's offset) with the
+// list radius widened beyond the rounding, and against the exclusions, and kept with the mask of the members that pass.
 // Each member's entries are thus a superset of its atom-list row; the pair
 // kernel's per-step cut-off decides the pair set, which the pair-set
 // fingerprint checks against the reference.  The pair kernel rounds j's minimum-image
@@ -102,14 +102,29 @@ __global__ void k_cell_starts(int N, int n_cells, int sub_bits, const int *__res
     for (int c = prev + 1; c <= cur; ++c) start[c] = p;
 }
 
-// Positions in cell order, with the atom index in w.
-__global__ void k_sorted_positions(int N, const int *__restrict__ ids, const double *__restrict__ rx,
-                                   const double *__restrict__ ry, const double *__restrict__ rz, double4 *spos)
+// The builders' candidate tests are FP32, on coordinates wrapped into the box in
+// FP64 and rounded: each is off by at most 2^-24 L, so that differences with their
+// single shift are within 2^-22 L of the nearest image's and distances within
+// 2^-21 L.  Radii are widened by 2^-20 L: the lists are supersets of those
+// of the FP64 distances, and of any other image's.
+__device__ __forceinline__ float wrapped(double x, double L) { return (float)(x - L * floor(x / L)); }
+__device__ __forceinline__ float near1(float d, float L, float H) { return fabsf(d) > H ? d - copysignf(L, d) : d; }
+__device__ __forceinline__ float widened2(double radius, const Box &b)
+{
+    const double r = radius + 0x1p-20 * fmax(b.L[0], fmax(b.L[1], b.L[2]));
+    return __double2float_ru(r * r * 1.000001);
+}
+
+// Wrapped FP32 positions in cell order, with the atom's list entry in w.
+__global__ void k_sorted_positions(int N, const int *__restrict__ ids, const int *__restrict__ type,
+                                   const double *__restrict__ rx, const double *__restrict__ ry,
+                                   const double *__restrict__ rz, Box box, float4 *spos)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= N) return;
     const int j = ids[p];
-    spos[p] = make_double4(rx[j], ry[j], rz[j], (double)j);
+    spos[p] = make_float4(wrapped(rx[j], box.L[0]), wrapped(ry[j], box.L[1]), wrapped(rz[j], box.L[2]),
+                          __uint_as_float(pack_nb(j, type[j])));
 }
 
 __device__ __forceinline__ bool excluded(const DevParams &P, int i, int j)
@@ -146,12 +161,13 @@ __device__ __forceinline__ ZRuns z_runs(int cz, int nz)
     return z;
 }
 
-// One warp per atom i, for the rows i0 .. i0 + rows - 1.
+// One warp per atom i, for the rows i0 .. i0 + rows - 1.  Bound by issue (a
+// quarter of the window's candidates pass).
 __global__ void __launch_bounds__(256) k_build_list(DevParams P, Grid g, int i0, int rows,
                                                     const double *__restrict__ rx,
                                                     const double *__restrict__ ry,
                                                     const double *__restrict__ rz,
-                                                    const double4 *__restrict__ spos,
+                                                    const float4 *__restrict__ spos,
                                                     const int *__restrict__ cell_start, int cap,
                                                     uint32_t *__restrict__ nbr, int *__restrict__ nnb,
                                                     double *rx0, double *ry0, double *rz0, int *flags)
@@ -169,6 +185,10 @@ __global__ void __launch_bounds__(256) k_build_list(DevParams P, Grid g, int i0,
     const ZRuns zr = z_runs(c0[2], nz);
     const unsigned lt_mask = (1u << lane) - 1u;
     uint32_t *row = nbr + (size_t)i * cap;
+    const float xf = wrapped(xi, P.box.L[0]), yf = wrapped(yi, P.box.L[1]), zf = wrapped(zi, P.box.L[2]);
+    const float cut = widened2(sqrt(P.list_r2), P.box);
+    const float L[3] = {(float)P.box.L[0], (float)P.box.L[1], (float)P.box.L[2]};
+    const float H[3] = {0.5f * L[0], 0.5f * L[1], 0.5f * L[2]};
     int count = 0;
     for (int ix = 0; ix < nxs; ++ix) {
         for (int iy = 0; iy < nys; ++iy) {
@@ -178,18 +198,18 @@ __global__ void __launch_bounds__(256) k_build_list(DevParams P, Grid g, int i0,
                 for (int base = s; base < e; base += 32) {
                     const int p = base + lane;
                     bool ok = false;
-                    int j = 0;
+                    uint32_t entry = 0;
                     if (p < e) {
-                        const double4 q = spos[p];
-                        j = (int)q.w;
-                        double dx = q.x - xi, dy = q.y - yi, dz = q.z - zi;
-                        image(dx, dy, dz, P.box);
-                        ok = j != i && norm2_exact(dx, dy, dz) < P.list_r2;
-                        if (ok) ok = !excluded(P, i, j);
+                        const float4 q = spos[p];
+                        entry = __float_as_uint(q.w);
+                        const float dx = near1(q.x - xf, L[0], H[0]), dy = near1(q.y - yf, L[1], H[1]),
+                                    dz = near1(q.z - zf, L[2], H[2]);
+                        ok = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < cut;
+                        if (ok) ok = nb_index(entry) != i && !excluded(P, i, nb_index(entry));
                     }
                     const unsigned ballot = __ballot_sync(0xffffffffu, ok);
                     const int pos = count + __popc(ballot & lt_mask);
-                    if (ok && pos < cap) row[pos] = pack_nb(j, P.type[j]);
+                    if (ok && pos < cap) row[pos] = entry;
                     count += __popc(ballot);
                 }
             }
@@ -252,11 +272,11 @@ __device__ __forceinline__ int cluster_offsets(const int m[4], const double *__r
 // A thread finds its cell by bisecting the cells' first clusters: boxes under
 // seven half-cell edges are one cell, whose clusters one thread per cell would
 // form one after the other (3,147 atoms in one cell: 802 us, here 6).
-// cl_of (half list, else null): the cluster of each atom.
+// cl_first: the sorted position of each cluster's first member.
 __global__ void k_make_clusters(int n_cells, const int *__restrict__ cell_start, const int *__restrict__ cl_start,
                                 const int *__restrict__ cell_atoms, const double *__restrict__ rx,
                                 const double *__restrict__ ry, const double *__restrict__ rz, InvBox B,
-                                int4 *cl_atoms, int *cl_of, int *flags)
+                                int4 *cl_atoms, int *cl_first, int *flags)
 {
     const int cl = blockIdx.x * blockDim.x + threadIdx.x;
     float emax = 0.f;
@@ -272,9 +292,7 @@ __global__ void k_make_clusters(int n_cells, const int *__restrict__ cell_start,
 #pragma unroll
         for (int t = 0; t < 4; ++t) m[t] = p + t < e ? cell_atoms[p + t] : -1;
         cl_atoms[cl] = make_int4(m[0], m[1], m[2], m[3]);
-        if (cl_of)
-            for (int t = 0; t < 4; ++t)
-                if (m[t] >= 0) cl_of[m[t]] = cl;
+        cl_first[cl] = p;
         double o[4][3], cc[3], ext = 0.0;
         const int nk = cluster_offsets(m, rx, ry, rz, B, o, cc);
         for (int k = 0; k < nk; ++k)
@@ -290,19 +308,18 @@ __global__ void __launch_bounds__(256) k_build_cluster_list(DevParams P, Grid g,
                                                             const double *__restrict__ rx,
                                                             const double *__restrict__ ry,
                                                             const double *__restrict__ rz,
-                                                            const double4 *__restrict__ spos,
+                                                            const float4 *__restrict__ spos,
                                                             const int *__restrict__ cell_start,
                                                             const int4 *__restrict__ cl_atoms,
                                                             const int *__restrict__ n_cl, int cap,
                                                             uint32_t *__restrict__ nbr, int *__restrict__ nnb,
                                                             unsigned char *__restrict__ cl_metal, double *rx0,
-                                                            double *ry0, double *rz0, int *flags,
-                                                            const int *__restrict__ cl_of,
-                                                            const int *__restrict__ cl_cell_start)
+                                                            double *ry0, double *rz0, int *flags, bool half,
+                                                            const int *__restrict__ cl_first)
 {
-    // cl_of (half list): a pair is listed once, by the lower-numbered cluster
-    // of its two atoms, and inside one cluster by the earlier member; cells
-    // whose clusters all precede this one are skipped
+    // half list: a pair is listed once, by the lower-numbered cluster of its two
+    // atoms, and inside one cluster by the earlier member.  Clusters are numbered
+    // in the sorted order, so the atoms before the cluster's own first are skipped
     const int cl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (cl >= *n_cl) return;
@@ -319,12 +336,13 @@ __global__ void __launch_bounds__(256) k_build_cluster_list(DevParams P, Grid g,
         zm[k] = rz[a];
         if (k < nk) R2 = fmax(R2, o[k][0] * o[k][0] + o[k][1] * o[k][1] + o[k][2] * o[k][2]);
     }
-    // prefilter radius, widened by a relative 1e-12 against rounding
-    const double pre = (sqrt(P.list_r2) + sqrt(R2)) * (1.0 + 1e-12);
-    const double pre2 = pre * pre;
-    // FP32 member test: the list radius widened by 1e-5 relative; the
-    // members' offsets from the centroid (selected by member, in registers)
-    const float lr2f = (float)(P.list_r2 * (1.0 + 1e-5));
+    // prefilter around the centroid, and the member test; the members' offsets
+    // from the centroid are selected by member, in registers
+    const double rl = sqrt(P.list_r2);
+    const float pre2 = widened2(rl + sqrt(R2), P.box), lr2f = widened2(rl, P.box);
+    const float xf = wrapped(cc[0], P.box.L[0]), yf = wrapped(cc[1], P.box.L[1]), zf = wrapped(cc[2], P.box.L[2]);
+    const float L[3] = {(float)P.box.L[0], (float)P.box.L[1], (float)P.box.L[2]};
+    const float H[3] = {0.5f * L[0], 0.5f * L[1], 0.5f * L[2]};
     const float ofx0 = (float)o[0][0], ofy0 = (float)o[0][1], ofz0 = (float)o[0][2];
     const float ofx1 = nk > 1 ? (float)o[1][0] : 0.f, ofy1 = nk > 1 ? (float)o[1][1] : 0.f,
                 ofz1 = nk > 1 ? (float)o[1][2] : 0.f;
@@ -344,35 +362,34 @@ __global__ void __launch_bounds__(256) k_build_cluster_list(DevParams P, Grid g,
     uint32_t *row = nbr + (size_t)cl * cap;
     int count = 0;
     bool metal = false;
+    const int p0 = cl_first[cl];
     for (int ix = 0; ix < nxs; ++ix) {
         for (int iy = 0; iy < nys; ++iy) {
             const int col = (axis_cell(c0[0], g.n[0], ix) * g.n[1] + axis_cell(c0[1], g.n[1], iy)) * nz;
             for (int r = 0; r < zr.n; ++r) {
-                int za = zr.a[r];
-                if (cl_of)
-                    while (za <= zr.b[r] && cl_cell_start[col + za + 1] <= cl) ++za;
-                const int s = cell_start[col + za], e = cell_start[col + zr.b[r] + 1];
+                const int e = cell_start[col + zr.b[r] + 1];
+                int s = cell_start[col + zr.a[r]];
+                if (half) s = max(s, p0);
                 for (int base = s; base < e; base += 32) {
                     const int p = base + lane;
                     unsigned mask = 0;
-                    int j = 0;
-                    const double4 q = p < e ? spos[p] : make_double4(0.0, 0.0, 0.0, 0.0);
-                    const int cj = p < e && cl_of ? cl_of[(int)q.w] : cl + 1;
-                    if (p < e && cj >= cl) {
-                        j = (int)q.w;
-                        // on the half list, members before j's own position when j is one
-                        const int jpos = cj != cl ? 4 : (j == m[0] ? 0 : j == m[1] ? 1 : j == m[2] ? 2 : 3);
-                        const double ex = min_image(q.x - cc[0], B.L[0], B.inv[0]);
-                        const double ey = min_image(q.y - cc[1], B.L[1], B.inv[1]);
-                        const double ez = min_image(q.z - cc[2], B.L[2], B.inv[2]);
-                        if (ex * ex + ey * ey + ez * ez < pre2) {
+                    uint32_t entry = 0;
+                    if (p < e) {
+                        const float4 q = spos[p];
+                        const float ex = near1(q.x - xf, L[0], H[0]), ey = near1(q.y - yf, L[1], H[1]),
+                                    ez = near1(q.z - zf, L[2], H[2]);
+                        entry = __float_as_uint(q.w);
+                        if (fmaf(ez, ez, fmaf(ey, ey, ex * ex)) < pre2) {
+                            const int j = nb_index(entry);
+                            // members before j's own position when j is one (half), all but j
+                            const int at = p - p0, upto = half && at < nk ? at : 4;
 #pragma unroll
                             for (int k = 0; k < 4; ++k) {
-                                if (k >= nk || j == m[k] || k >= jpos) continue;
+                                if (k >= nk || k == at || k >= upto) continue;
                                 const float ox = k == 0 ? ofx0 : k == 1 ? ofx1 : k == 2 ? ofx2 : ofx3;
                                 const float oy = k == 0 ? ofy0 : k == 1 ? ofy1 : k == 2 ? ofy2 : ofy3;
                                 const float oz = k == 0 ? ofz0 : k == 1 ? ofz1 : k == 2 ? ofz2 : ofz3;
-                                const float sx = (float)ex - ox, sy = (float)ey - oy, sz = (float)ez - oz;
+                                const float sx = ex - ox, sy = ey - oy, sz = ez - oz;
                                 if (fmaf(sz, sz, fmaf(sy, sy, sx * sx)) < lr2f && !excluded(P, m[k], j))
                                     mask |= 1u << k;
                             }
@@ -382,15 +399,15 @@ __global__ void __launch_bounds__(256) k_build_cluster_list(DevParams P, Grid g,
                     const unsigned ballot = __ballot_sync(0xffffffffu, ok);
                     const int pos = count + __popc(ballot & lt_mask);
                     if (ok) {
-                        if (pos < cap) row[pos] = pack_cl(j, mask, P.type[j]);
-                        metal |= P.is_metal[j] != 0;
+                        if (pos < cap) row[pos] = pack_cl(nb_index(entry), mask, nb_type(entry));
+                        metal |= P.is_metal[nb_index(entry)] != 0;
                     }
                     count += __popc(ballot);
                 }
             }
         }
     }
-    if (cl_of)  // the half list: a metal member takes water neighbours' CPIM terms too
+    if (half)  // the half list: a metal member takes water neighbours' CPIM terms too
         for (int k = 0; k < nk; ++k) metal |= P.is_metal[m[k]] != 0;
     metal = __any_sync(0xffffffffu, metal);
     if (lane == 0) {
@@ -832,20 +849,22 @@ void ensure_cluster_buffers(capac_ctx *c, int n_cells)
         cudaFree(c->cl_nnb);
         cudaFree(c->cl_metal);
         cudaFree(c->cl_sel);
+        cudaFree(c->cl_first);
         c->cl_atoms = nullptr;
         c->cl_nbr = nullptr;
         c->cl_nnb = nullptr;
         c->cl_metal = nullptr;
         c->cl_sel = nullptr;
+        c->cl_first = nullptr;
         CAPAC_CUDA(cudaMalloc(&c->cl_atoms, sizeof(int4) * need));
         CAPAC_CUDA(cudaMalloc(&c->cl_nbr, sizeof(uint32_t) * (size_t)need * c->cl_cap));
         CAPAC_CUDA(cudaMalloc(&c->cl_nnb, sizeof(int) * need));
         CAPAC_CUDA(cudaMalloc(&c->cl_metal, need));
         CAPAC_CUDA(cudaMalloc(&c->cl_sel, sizeof(int) * need));
+        CAPAC_CUDA(cudaMalloc(&c->cl_first, sizeof(int) * need));
         c->cl_max = need;
     }
     c->cl_half = c->opt.pair_list != 3;  // 0 (default) and 2: every pair once; 3: the full cluster list
-    if (c->cl_half && !c->cl_of) CAPAC_CUDA(cudaMalloc(&c->cl_of, sizeof(int) * N));
     if (!c->cl_next) CAPAC_CUDA(cudaMalloc(&c->cl_next, sizeof(int)));
     if (!c->n_cl_sel) CAPAC_CUDA(cudaMalloc(&c->n_cl_sel, sizeof(int)));
 }
@@ -869,7 +888,7 @@ bool make_clusters(capac_ctx *c, int n_cells)
     CAPAC_CUDA(cudaMemsetAsync(c->flags + 5, 0, sizeof(int), s));
     k_make_clusters<<<grid_for(c->cl_max, 128), 128, 0, s>>>(n_cells, c->cell_start, c->cl_cell_start, c->cell_atoms,
                                                            c->rx, c->ry, c->rz, inv_box(c), c->cl_atoms,
-                                                           c->cl_half ? c->cl_of : nullptr, c->flags);
+                                                           c->cl_first, c->flags);
     c->launches += 3;
     CAPAC_CUDA(cudaMemcpyAsync(c->h_flags + 6, c->cl_cell_start + n_cells, sizeof(int), cudaMemcpyDeviceToHost, s));
     CAPAC_CUDA(cudaMemcpyAsync(c->h_flags + 5, c->flags + 5, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -891,8 +910,8 @@ void build_cluster_list(capac_ctx *c, const Grid &g, int n_cells)
             ProfScope ps(c, K_LIST);
             k_build_cluster_list<<<grid_for((long)c->n_clusters * 32, 256), 256, 0, s>>>(
                 c->P, g, inv_box(c), c->rx, c->ry, c->rz, c->spos, c->cell_start, c->cl_atoms, n_cl, c->cl_cap,
-                c->cl_nbr, c->cl_nnb, c->cl_metal, c->rx0, c->ry0, c->rz0, c->flags,
-                c->cl_half ? c->cl_of : nullptr, c->cl_cell_start);
+                c->cl_nbr, c->cl_nnb, c->cl_metal, c->rx0, c->ry0, c->rz0, c->flags, c->cl_half,
+                c->cl_first);
         }
         ++c->launches;
         CAPAC_CUDA(cudaMemcpyAsync(c->h_flags + 4, c->flags + 4, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1035,7 +1054,7 @@ void build_list(capac_ctx *c)
         CAPAC_CUDA(cudaMalloc(&c->cell_start, sizeof(int) * (n_cells + 1)));
         c->n_cells = n_cells;
     }
-    if (!c->spos) CAPAC_CUDA(cudaMalloc(&c->spos, sizeof(double4) * N));
+    if (!c->spos) CAPAC_CUDA(cudaMalloc(&c->spos, sizeof(float4) * N));
     for (int a = 0; a < 3; ++a) c->ncell[a] = g.n[a];
     const int sub_bits = sub_cell_bits(n_cells);
     c->cell_sub_bits = sub_bits;
@@ -1057,7 +1076,8 @@ void build_list(capac_ctx *c)
     CAPAC_CUDA(cub::DeviceRadixSort::SortPairs(c->sort_tmp, need, c->cell_key, c->cell_key_sorted,
                                                c->atom_ids, c->cell_atoms, N, 0, end_bit, s));
     k_cell_starts<<<grid_for(N + 1, 256), 256, 0, s>>>(N, n_cells, sub_bits, c->cell_key_sorted, c->cell_start);
-    k_sorted_positions<<<grid_for(N, 256), 256, 0, s>>>(N, c->cell_atoms, c->rx, c->ry, c->rz, c->spos);
+    k_sorted_positions<<<grid_for(N, 256), 256, 0, s>>>(N, c->cell_atoms, c->type, c->rx, c->ry, c->rz, c->P.box,
+                                                         c->spos);
     c->launches += 2;
 
     bool use_cl = cluster_list_allowed(c) && make_clusters(c, n_cells);
