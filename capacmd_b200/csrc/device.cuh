@@ -89,24 +89,43 @@ __device__ __forceinline__ R warp_sum_halving(R (&v)[V], int lane)
     return s;
 }
 
-// Sum K values over the block (blockDim.x a multiple of 32, at most 1024) in
-// a fixed order; thread 0 receives the totals in v[].  `sh` needs 32*K doubles.
+// Warp sums of v[k], k = A .. A + K - 1, into out[k], in groups of a power of two
+// (10 values: 8 + 2, 16 shuffles for 50).
+template <int A, int K, int N>
+__device__ __forceinline__ void warp_sums_to(const double (&v)[N], double *out, int lane)
+{
+    constexpr int V = K >= 16 ? 16 : (K >= 8 ? 8 : (K >= 4 ? 4 : (K >= 2 ? 2 : 1)));
+    double u[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) u[k] = v[A + k];
+    const double s = warp_sum_halving<V>(u, lane);
+    constexpr int kStep = 32 / V;
+    if (lane % kStep == 0) out[A + lane / kStep] = s;
+    if constexpr (K > V) warp_sums_to<A + V, K - V>(v, out, lane);
+}
+
+// Sum K <= 32 values over the block (blockDim.x a multiple of 32, at most 1024)
+// in a fixed order; thread 0 receives the totals in v[].  `sh` needs 32*K
+// doubles.
 template <int K>
 __device__ __forceinline__ void block_sum(double (&v)[K], double *sh)
 {
+    static_assert(K <= 32, "one warp adds the warps' sums");
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = warp_sum(v[k]);
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) sh[wid * K + k] = v[k];
-    }
+    warp_sums_to<0, K>(v, sh + wid * K, lane);
     __syncthreads();
     if (wid == 0) {
+        if (lane < K) {
+            double s = sh[lane];
+#pragma unroll 8
+            for (int w = 1; w < nw; ++w) s += sh[w * K + lane];
+            sh[lane] = s;
+        }
+        __syncwarp();
+        if (lane == 0) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = lane < nw ? sh[lane * K + k] : 0.0;
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = warp_sum(v[k]);
+            for (int k = 0; k < K; ++k) v[k] = sh[k];
+        }
     }
     __syncthreads();
 }

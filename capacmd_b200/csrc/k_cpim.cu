@@ -181,62 +181,60 @@ void launch_qsc(capac_ctx *c)
 
 // mpi_cpff_vec_ext, cpff.c:43-198: field and potential of the permanent
 // charges inside the cut-off at each metal atom, converted to atomic units,
-// plus the uniform external field; NP total charges in the last rows.
-__global__ void __launch_bounds__(256) k_cpim_rhs(DevParams P, const double4 *__restrict__ pos4,
+// plus the uniform external field; NP total charges in the last rows.  A block
+// per metal atom: a warp each left the chip idle up to a few hundred atoms.
+constexpr int kRhsBlock = 128;
+__global__ void __launch_bounds__(kRhsBlock) k_cpim_rhs(DevParams P, const double4 *__restrict__ pos4,
                                                   const uint32_t *__restrict__ nbr, const int *__restrict__ nnb,
                                                   int cap, double *vec_ext)
 {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (blockIdx.x == 0 && threadIdx.x < P.n_nps) vec_ext[4 * P.M + threadIdx.x] = P.np_charge[threadIdx.x];
-    if (i >= P.M) return;
-    const int im = P.metal_min + i;
+    __shared__ double sh[32 * 4];
+    const int i = blockIdx.x;
+    if (i == 0)
+        for (int k = threadIdx.x; k < P.n_nps; k += kRhsBlock) vec_ext[4 * P.M + k] = P.np_charge[k];
+    const int im = P.metal_min + i, n = nnb[im];
     const double4 pi = pos4[im];
-    double ex = 0.0, ey = 0.0, ez = 0.0, v = 0.0;
+    const bool shrt = P.w_alpha * P.rc < kDsfMaxX;
+    double t[4] = {0.0, 0.0, 0.0, 0.0};  // field, potential
     const uint32_t *row = nbr + (size_t)im * cap;
-    for (int k = lane; k < nnb[im]; k += 32) {
+    for (int k = threadIdx.x; k < n; k += kRhsBlock) {
         const int j = nb_index(row[k]);
-        if (P.is_metal[j]) continue;
         const double4 pj = pos4[j];
-        if (pj.w == 0.0) continue;
+        if (pj.w == 0.0 || P.is_metal[j]) continue;
         double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
         image(dx, dy, dz, P.box);
         const double r2 = norm2_exact(dx, dy, dz);
         if (r2 >= P.rc2) continue;
-        const double r = sqrt(r2);
         double ef, vf;
         if (P.use_coulomb == 1) {
-            const double ec = erfc(P.w_alpha * r), eg = exp(-P.w_alpha * P.w_alpha * r2);
-            ef = kFQQ * pj.w * (ec / r2 + P.w_a2_sqrtpi * eg / r - P.w_const) / r;
-            vf = kFQQ * pj.w * (ec / r - P.w_erfc_arcut + P.w_const * (r - P.rc));
+            const Dsf d = shrt ? dsf_terms(P.w_alpha, r2) : dsf_terms_any(P.w_alpha, r2);
+            ef = kFQQ * pj.w * (fma(d.ec, d.rinv * d.rinv, P.w_a2_sqrtpi * d.eg * d.rinv) - P.w_const) * d.rinv;
+            vf = kFQQ * pj.w * (fma(d.ec, d.rinv, -P.w_erfc_arcut) + P.w_const * (d.r - P.rc));
         } else {
+            const double r = sqrt(r2);
             ef = kFQQ * pj.w / (r2 * r);
             vf = kFQQ * pj.w / r;
         }
         const double s = ef * kConvE;
-        ex += s * dx;
-        ey += s * dy;
-        ez += s * dz;
-        v += vf * kConvV;
+        t[0] = fma(s, dx, t[0]);
+        t[1] = fma(s, dy, t[1]);
+        t[2] = fma(s, dz, t[2]);
+        t[3] = fma(vf, kConvV, t[3]);
     }
-    ex = warp_sum(ex);
-    ey = warp_sum(ey);
-    ez = warp_sum(ez);
-    v = warp_sum(v);
-    if (lane == 0) {
-        vec_ext[3 * i + 0] = ex + P.efield[0] * kConvE;
-        vec_ext[3 * i + 1] = ey + P.efield[1] * kConvE;
-        vec_ext[3 * i + 2] = ez + P.efield[2] * kConvE;
+    block_sum<4>(t, sh);
+    if (threadIdx.x == 0) {
+        vec_ext[3 * i + 0] = t[0] + P.efield[0] * kConvE;
+        vec_ext[3 * i + 1] = t[1] + P.efield[1] * kConvE;
+        vec_ext[3 * i + 2] = t[2] + P.efield[2] * kConvE;
         const double vext = P.efield[0] * pi.x + P.efield[1] * pi.y + P.efield[2] * pi.z;
-        vec_ext[3 * P.M + i] = v - vext * kConvV;
+        vec_ext[3 * P.M + i] = t[3] - vext * kConvV;
     }
 }
 
 void launch_cpim_rhs(capac_ctx *c)
 {
     ProfScope ps(c, K_CPIM_RHS);
-    k_cpim_rhs<<<grid_for((long)c->M * 32 + 32, 256), 256, 0, c->stream>>>(c->P, c->pos4, c->nbr, c->nnb, c->cap,
-                                                                            c->vec_ext);
+    k_cpim_rhs<<<c->M, kRhsBlock, 0, c->stream>>>(c->P, c->pos4, c->nbr, c->nnb, c->cap, c->vec_ext);
     ++c->launches;
 }
 
@@ -977,48 +975,35 @@ __device__ __forceinline__ void metal_pair(const R r[3], R qi, const R pi[3], R 
     const R ir3 = (R)1 / (r2 * rr), ir5 = ir3 / r2, ir7 = ir5 / r2;
     f[0] = f[1] = f[2] = (R)0;
     e[0] = e[1] = e[2] = (R)0;
+    // the tensors T1_ab, T2_abc contracted with the dipoles by hand: p . r and
+    // pi . pj stand for the sums over their indices
+    const R dpi = pi[0] * r[0] + pi[1] * r[1] + pi[2] * r[2], dpj = pj[0] * r[0] + pj[1] * r[1] + pj[2] * r[2];
+    const R dpp = pi[0] * pj[0] + pi[1] * pj[1] + pi[2] * pj[2];
     // charge - charge
     const R gqq = exp(-(r2 * iqq * iqq)), erq = erf(rr * iqq);
     const R A0 = ir3 * (erq - (R)2 * isp * iqq * rr * gqq);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) f[a] += A0 * r[a] * fq2 * qi * qj;
+    R along = A0 * fq2 * qi * qj;
     e[0] += fq1 * qi * qj * erq / rr * half;
-    // charge - dipole
+    // charge - dipole: T_ab = A1 (3 r_a r_b - d_ab r^2) - B1 r_a r_b
     const R gpq = exp(-(r2 * ipq * ipq));
     const R tpq = erf(rr * ipq) - (R)2 * isp * ipq * rr * gpq;
     const R Apq0 = ir3 * tpq, A1 = ir5 * tpq, B1 = (R)4 * isp * ipq3 / r2 * gpq;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            const R dab = a == b ? (R)1 : (R)0;
-            const R T = A1 * ((R)3 * r[a] * r[b] - dab * r2) - B1 * r[a] * r[b];
-            f[b] += -T * fq2 * qi * pj[a];
-            f[b] += T * fq2 * qj * pi[a];
-        }
-        e[1] += -fq1 * qi * pj[a] * r[a] * Apq0 * half;
-        e[1] += fq1 * qj * pi[a] * r[a] * Apq0 * half;
-    }
-    // dipole - dipole
+    const R mix = qj * dpi - qi * dpj;
+    along += fq2 * ((R)3 * A1 - B1) * mix;
+    R ci = -fq2 * A1 * r2 * qj, cj = fq2 * A1 * r2 * qi;  // coefficients of pi and pj
+    e[1] += fq1 * mix * Apq0 * half;
+    // dipole - dipole: T_abc = A2 (5 r_a r_b r_c - r^2 (r_a d_bc + r_b d_ca + r_c d_ab)) - B2 r_a r_b r_c
     const R gpp = exp(-(r2 * ipp * ipp)), erp = erf(rr * ipp);
     const R App1 = ir5 * (erp - (R)2 * isp * ipp * rr * gpp);
     const R Bpp1 = (R)4 * isp * ipp3 / r2 * gpp;
     const R A2 = ir7 * ((R)3 * erp - (R)6 * isp * ipp * rr * gpp - (R)4 * (r2 * rr) * isp * ipp3 * gpp);
     const R B2 = (R)8 * isp * ipp5 / r2 * gpp;
+    along -= fq2 * (((R)5 * A2 - B2) * dpi * dpj - A2 * r2 * dpp);
+    ci += fq2 * A2 * r2 * dpj;
+    cj += fq2 * A2 * r2 * dpi;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            const R dab = a == b ? (R)1 : (R)0;
-#pragma unroll
-            for (int cc = 0; cc < 3; ++cc) {
-                const R dbc = b == cc ? (R)1 : (R)0, dca = cc == a ? (R)1 : (R)0;
-                f[cc] += -(A2 * ((R)5 * r[a] * r[b] * r[cc] - r2 * (r[a] * dbc + r[b] * dca + r[cc] * dab)) -
-                           B2 * r[a] * r[b] * r[cc]) * fq2 * pi[a] * pj[b];
-            }
-            e[2] += -fq1 * pi[a] * pj[b] * (((R)3 * r[a] * r[b] - dab * r2) * App1 - r[a] * r[b] * Bpp1) * half;
-        }
-    }
+    for (int a = 0; a < 3; ++a) f[a] = along * r[a] + ci * pi[a] + cj * pj[a];
+    e[2] -= fq1 * half * (((R)3 * dpi * dpj - r2 * dpp) * App1 - dpi * dpj * Bpp1);
 }
 
 // mpi_cpff_force (cpff.c:526-950) for one metal atom per block: metal -
@@ -1047,24 +1032,27 @@ __global__ void __launch_bounds__(256) k_cpim_metal(DevParams P, const double4 *
 
     // metal - permanent charge, MD units (cpff.c:578-724)
     const uint32_t *row = nbr + (size_t)im * cap;
-    for (int k = threadIdx.x; k < nnb[im]; k += blockDim.x) {
+    const bool shrt = P.use_coulomb == 1 && P.w_alpha * P.rc < kDsfMaxX;
+    for (int k = threadIdx.x, n = nnb[im]; k < n; k += blockDim.x) {
         const int j = nb_index(row[k]);
-        if (P.is_metal[j]) continue;
         const double4 pj = pos4[j];
-        if (pj.w == 0.0) continue;
+        if (pj.w == 0.0 || P.is_metal[j]) continue;
         double r[3] = {pi4.x - pj.x, pi4.y - pj.y, pi4.z - pj.z};
         image(r[0], r[1], r[2], P.box);
         const double r2 = norm2_exact(r[0], r[1], r[2]);
         if (r2 >= P.rc2) continue;
-        double f[3], a0, ec;
-        cpim_charge_pair(P, r, r2, pj.w, qi, pi, f, a0, ec);
-        const double rr = sqrt(r2);
-        if (P.use_coulomb == 1)
-            acc[4] += kFQQ * pj.w * qi * (ec / rr - P.w_erfc_arcut + P.w_const * (rr - P.rc));
-        else
-            acc[4] += kFQQ * pj.w * qi / rr;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) acc[5] += -kFQQ * pj.w * pi[a] / kNm2Bohr * a0 * r[a];
+        double f[3], a0, v;
+        if (shrt) {
+            const Dsf d = cpim_charge_pair_dsf(P, r, r2, pj.w, qi, pi, f, a0);
+            v = fma(d.ec, d.rinv, -P.w_erfc_arcut) + P.w_const * (d.r - P.rc);
+        } else {
+            double ec;
+            cpim_charge_pair(P, r, r2, pj.w, qi, pi, f, a0, ec);
+            const double rr = sqrt(r2);
+            v = P.use_coulomb == 1 ? ec / rr - P.w_erfc_arcut + P.w_const * (rr - P.rc) : 1.0 / rr;
+        }
+        acc[4] += kFQQ * pj.w * qi * v;
+        acc[5] -= kFQQ / kNm2Bohr * pj.w * a0 * (pi[0] * r[0] + pi[1] * r[1] + pi[2] * r[2]);
         acc[0] += f[0];
         acc[1] += f[1];
         acc[2] += f[2];

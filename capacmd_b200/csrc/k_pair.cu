@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 3 : 2) k_
                     if constexpr (sizeof(Real) == 8) {
                         double a0, ec;
                         if (damped)
-                            cpim_charge_pair_dsf(P, r, r2, pi.w, q, p, g);
+                            cpim_charge_pair_dsf(P, r, r2, pi.w, q, p, g, a0);
                         else
                             cpim_charge_pair(P, r, r2, pi.w, q, p, g, a0, ec);
                     } else {

@@ -70,21 +70,33 @@ __device__ __forceinline__ Dsf dsf_terms(double alpha, double r2)
     return d;
 }
 
+// The same for any x, by the library's functions.
+__device__ __forceinline__ Dsf dsf_terms_any(double alpha, double r2)
+{
+    Dsf d;
+    d.r = sqrt(r2);
+    d.rinv = 1.0 / d.r;
+    d.eg = exp(-alpha * alpha * r2);
+    d.ec = erfc(alpha * d.r);
+    return d;
+}
+
 // cpim_charge_pair with the damped form and alpha r < kDsfMaxX.
-__device__ __forceinline__ void cpim_charge_pair_dsf(const DevParams &P, const double r[3], double r2, double q_perm,
-                                                     double q_ind, const double p[3], double f[3])
+__device__ __forceinline__ Dsf cpim_charge_pair_dsf(const DevParams &P, const double r[3], double r2, double q_perm,
+                                                    double q_ind, const double p[3], double f[3], double &a0)
 {
     const Dsf d = dsf_terms(P.w_alpha, r2);
     const double r2inv = d.rinv * d.rinv, ir3 = r2inv * d.rinv, al3 = P.w_alpha * P.w_alpha * P.w_alpha;
     const double s = kFQQ * q_perm, sp = s / kNm2Bohr;
-    const double a0 = fma(d.ec, r2inv, P.w_a2_sqrtpi * d.eg * d.rinv) - P.w_const;
+    a0 = (fma(d.ec, r2inv, P.w_a2_sqrtpi * d.eg * d.rinv) - P.w_const) * d.rinv;
     const double a1 = ir3 * r2inv * fma(P.w_a2_sqrtpi * d.r, d.eg, d.ec), b1 = 4.0 * kInvSqrtPi * al3 * r2inv * d.eg,
                  c1 = P.w_const * ir3;
     const double pr = p[0] * r[0] + p[1] * r[1] + p[2] * r[2];
     // sum_a T_ab p_a, T_ab = a1 (3 r_a r_b - d_ab r^2) + b1 r_a r_b - c1 (r_a r_b - d_ab r^2)
-    const double along = fma(a0 * d.rinv, s * q_ind, -(3.0 * a1 + b1 - c1) * pr * sp), off = (a1 - c1) * r2 * sp;
+    const double along = fma(a0, s * q_ind, -(3.0 * a1 + b1 - c1) * pr * sp), off = (a1 - c1) * r2 * sp;
 #pragma unroll
     for (int b = 0; b < 3; ++b) f[b] = fma(along, r[b], off * p[b]);
+    return d;
 }
 
 // Force on the metal atom from the permanent charge q of a non-metal atom at
