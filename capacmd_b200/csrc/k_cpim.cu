@@ -91,80 +91,112 @@ void launch_force_sums(capac_ctx *c)
 
 // --------------------------------------------------------- Sutton-Chen
 
+// (a/r)^e of an exponent e from t = (a/r)^2.  The reference's
+// exponents are integers: products of t (a square root more where odd) then
+// take 4-5 operations where log and exp take ~60.  Real exponents (parameter
+// gradients) go through exp(e log(a/r)), within ~1e-15 of pow.
+struct QscPower {
+    double e;
+    int half;  // floor(e / 2), -1: not an integer of 0..64
+    bool odd;
+    __device__ __forceinline__ explicit QscPower(double x) : e(x)
+    {
+        const bool whole = x >= 0.0 && x <= 64.0 && x == floor(x);
+        half = whole ? (int)x >> 1 : -1;
+        odd = whole && ((int)x & 1);
+    }
+    // log_t: log(t), read where the exponent is no such integer
+    __device__ __forceinline__ double operator()(double t, double log_t) const
+    {
+        if (half < 0) return exp(0.5 * e * log_t);
+        double y = odd ? sqrt(t) : 1.0, b = t;
+        for (int k = half; k; k >>= 1, b *= b)
+            if (k & 1) y *= b;
+        return y;
+    }
+};
+
 // mpi_qsc_dens, force.c:385-461: rho_i = sum_{j != i, r < rc} (a/r)^m.
-__global__ void __launch_bounds__(256) k_qsc_density(DevParams P, const double4 *__restrict__ pos4, double *isd)
+// A block per atom here and below: with a warp per atom (as many warps on the chip
+// as the metal has atoms) a warp waited for one load of its row after another.
+constexpr int kQscBlock = 128;
+__global__ void __launch_bounds__(kQscBlock) k_qsc_density(DevParams P, const double4 *__restrict__ pos4, double *isd)
 {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (i >= P.M) return;
+    __shared__ double sh[32];
+    const int i = blockIdx.x;
     const double4 pi = pos4[P.metal_min + i];
-    double rho = 0.0;
-    for (int j = lane; j < P.M; j += 32) {
-        if (j == i) continue;
+    double rho[1] = {0.0};
+    const QscPower pm(P.qsc_m);
+    const double a2 = P.qsc_a * P.qsc_a;
+#pragma unroll 2
+    for (int j = threadIdx.x; j < P.M; j += kQscBlock) {
         const double4 pj = pos4[P.metal_min + j];
         double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
         image(dx, dy, dz, P.box);
         const double r2 = norm2_exact(dx, dy, dz);
-        // (a/r)^m as exp(m log(a/r)): within ~1e-15 relative of pow
-        if (r2 < P.rc2) rho += exp(P.qsc_m * log(P.qsc_a / sqrt(r2)));
+        if (j != i && r2 < P.rc2) {
+            const double t = a2 / r2;
+            rho[0] += pm(t, pm.half < 0 ? log(t) : 0.0);
+        }
     }
-    rho = warp_sum(rho);
-    if (lane == 0) isd[i] = 1.0 / sqrt(rho);
+    block_sum<1>(rho, sh);
+    if (threadIdx.x == 0) isd[i] = 1.0 / sqrt(rho[0]);
 }
 
 // mpi_qsc_force, force.c:468-542: forces on i only, virial halved.
-__global__ void __launch_bounds__(256) k_qsc_force(DevParams P, const double4 *__restrict__ pos4,
-                                                   const double *__restrict__ isd, double *fx, double *fy,
-                                                   double *fz, double *partials)
+__global__ void __launch_bounds__(kQscBlock) k_qsc_force(DevParams P, const double4 *__restrict__ pos4,
+                                                         const double *__restrict__ isd, double *fx, double *fy,
+                                                         double *fz, double *partials)
 {
     __shared__ double sh[32 * 10];
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    double acc[10] = {0.0};  // energy, virial[9]
-    if (i < P.M) {
-        const double4 pi = pos4[P.metal_min + i];
-        const double cm2 = P.qsc_c * P.qsc_m / 2.0;
-        double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-        for (int j = lane; j < P.M; j += 32) {
-            if (j == i) continue;
-            const double4 pj = pos4[P.metal_min + j];
-            double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-            image(dx, dy, dz, P.box);
-            const double r2 = norm2_exact(dx, dy, dz);
-            if (r2 >= P.rc2) continue;
-            const double r = sqrt(r2), lar = log(P.qsc_a / r);
-            // (a/r)^n and (a/r)^m from one logarithm: within ~1e-15 relative of pow
-            const double an = exp(P.qsc_n * lar), am = exp(P.qsc_m * lar);
-            const double f = P.qsc_eps * (P.qsc_n * an - cm2 * (isd[i] + isd[j]) * am) / r2;
-            const double gx = f * dx, gy = f * dy, gz = f * dz;
-            f0 -= gx; f1 -= gy; f2 -= gz;
-            acc[1] -= dx * gx * 0.5; acc[2] -= dx * gy * 0.5; acc[3] -= dx * gz * 0.5;
-            acc[4] -= dy * gx * 0.5; acc[5] -= dy * gy * 0.5; acc[6] -= dy * gz * 0.5;
-            acc[7] -= dz * gx * 0.5; acc[8] -= dz * gy * 0.5; acc[9] -= dz * gz * 0.5;
-            acc[0] += P.qsc_eps * an * 0.5;
-        }
-        f0 = warp_sum(f0);
-        f1 = warp_sum(f1);
-        f2 = warp_sum(f2);
-        if (lane == 0) {
-            const int a = P.metal_min + i;
-            fx[a] += f0;
-            fy[a] += f1;
-            fz[a] += f2;
-            acc[0] -= P.qsc_eps * P.qsc_c / isd[i];
-        }
+    const int i = blockIdx.x;
+    const double4 pi = pos4[P.metal_min + i];
+    const double isd_i = isd[i], cm2 = P.qsc_c * P.qsc_m / 2.0;
+    const QscPower pn(P.qsc_n), pm(P.qsc_m);
+    const double a2 = P.qsc_a * P.qsc_a;
+    double acc[10] = {0.0};  // (a/r)^n, virial xx xy xz yy yz zz, force
+#pragma unroll 2
+    for (int j = threadIdx.x; j < P.M; j += kQscBlock) {
+        const double4 pj = pos4[P.metal_min + j];
+        const double isd_j = isd[j];
+        double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+        image(dx, dy, dz, P.box);
+        const double r2 = norm2_exact(dx, dy, dz);
+        if (j == i || r2 >= P.rc2) continue;
+        const double r2inv = 1.0 / r2, t = a2 * r2inv, lt = pn.half < 0 || pm.half < 0 ? log(t) : 0.0;
+        const double an = pn(t, lt), am = pm(t, lt);
+        const double f = P.qsc_eps * (P.qsc_n * an - cm2 * (isd_i + isd_j) * am) * r2inv;
+        const double gx = f * dx, gy = f * dy, gz = f * dz;
+        acc[0] += an;
+        acc[1] -= dx * gx; acc[2] -= dx * gy; acc[3] -= dx * gz;
+        acc[4] -= dy * gy; acc[5] -= dy * gz; acc[6] -= dz * gz;
+        acc[7] -= gx; acc[8] -= gy; acc[9] -= gz;
     }
-    block_partials<10>(acc, sh, partials);
+    block_sum<10>(acc, sh);
+    if (threadIdx.x == 0) {
+        const int a = P.metal_min + i;
+        fx[a] += acc[7];
+        fy[a] += acc[8];
+        fz[a] += acc[9];
+        double *out = partials + (size_t)i * 10;  // energy, virial[9]
+        out[0] = 0.5 * P.qsc_eps * acc[0] - P.qsc_eps * P.qsc_c / isd_i;
+        out[1] = 0.5 * acc[1];
+        out[2] = out[4] = 0.5 * acc[2];
+        out[3] = out[7] = 0.5 * acc[3];
+        out[5] = 0.5 * acc[4];
+        out[6] = out[8] = 0.5 * acc[5];
+        out[9] = 0.5 * acc[6];
+    }
 }
 
 void launch_qsc(capac_ctx *c)
 {
-    const unsigned grid = grid_for((long)c->M * 32, 256);
+    const unsigned grid = (unsigned)c->M;
     {
         ProfScope ps(c, K_QSC);
-        k_qsc_density<<<grid, 256, 0, c->stream>>>(c->P, c->pos4, c->isd);
-        k_qsc_force<<<grid, 256, 0, c->stream>>>(c->P, c->pos4, c->isd, c->fx, c->fy, c->fz,
-                                                force_partials(c, FP_QSC));
+        k_qsc_density<<<grid, kQscBlock, 0, c->stream>>>(c->P, c->pos4, c->isd);
+        k_qsc_force<<<grid, kQscBlock, 0, c->stream>>>(c->P, c->pos4, c->isd, c->fx, c->fy, c->fz,
+                                                       force_partials(c, FP_QSC));
     }
     c->launches += 2;
     if (c->defer) {
@@ -1167,7 +1199,7 @@ void launch_external_field(capac_ctx *c)
 size_t force_partial_areas(const capac_ctx *c, size_t off[4])
 {
     const size_t pair = std::max((size_t)grid_for((long)c->N * 32, 256), (size_t)c->num_sms * 4) * 11;
-    const size_t n[4] = {(size_t)grid_for((long)c->M * 32, 256) * 10, pair, (size_t)c->M * 15,
+    const size_t n[4] = {(size_t)c->M * 10, pair, (size_t)c->M * 15,
                          (size_t)grid_for(c->N, 256)};
     size_t at = 0;
     for (int k = 0; k < 4; ++k) {
