@@ -43,10 +43,6 @@ constexpr int kRows = 4 * kT;  // internal rows of a group
 constexpr int kInvThreads = 1024;
 constexpr int kMaxCoarse = 384;  // coarse columns the inversion handles (2 kMaxCoarse <= kInvThreads)
 
-__host__ __device__ __forceinline__ size_t tile_index(int I, int J, int nT)
-{
-    return (size_t)I * nT - (size_t)I * (I - 1) / 2 + (size_t)(J - I);
-}
 __device__ __forceinline__ int elem_offset(int p, int a, int b)
 {
     return ((p * (kT / 4) + (b >> 2)) * (kT * 4)) + a * 4 + (b & 3);
@@ -77,8 +73,7 @@ __global__ void __launch_bounds__(256) k_coarse_az(const float *__restrict__ mat
 {
     __shared__ float rs[kPlanes][kT], cs[kPlanes][kT];
     const size_t t = blockIdx.x;
-    int I = 0;
-    while (tile_index(I + 1, I + 1, nG) <= t && I + 1 < nG) ++I;
+    const int I = tile_row(t, nG);
     const int J = I + (int)(t - tile_index(I, I, nG));
     const float *tile = mat + t * kTileElems;
     for (int q = threadIdx.x; q < 2 * kPlanes * kT; q += blockDim.x) {

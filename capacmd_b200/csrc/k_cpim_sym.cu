@@ -33,12 +33,6 @@ constexpr int kT = 32;        // atoms per tile edge
 constexpr int kPlanes = 10;   // A_xx A_xy A_xz A_yy A_yz A_zz m_x m_y m_z C
 constexpr size_t kTileElems = (size_t)kPlanes * kT * kT;
 
-__host__ __device__ __forceinline__ size_t tile_index(int I, int J, int nT)
-{
-    // row-major upper triangle including the diagonal
-    return (size_t)I * nT - (size_t)I * (I - 1) / 2 + (size_t)(J - I);
-}
-
 __host__ __device__ __forceinline__ size_t elem_offset(int p, int a, int b)
 {
     return ((size_t)p * (kT / 4) + (b >> 2)) * (kT * 4) + (size_t)a * 4 + (b & 3);
@@ -74,8 +68,7 @@ __global__ void __launch_bounds__(256) k_sym_assemble(DevParams P, const double4
 {
     // decode the tile from the linear index
     const size_t t = blockIdx.x;
-    int I = 0;
-    while (tile_index(I + 1, I + 1, nT) <= t && I + 1 < nT) ++I;
+    const int I = tile_row(t, nT);
     const int J = I + (int)(t - tile_index(I, I, nT));
     T *tile = mat + t * kTileElems;
     for (int q = blockIdx.y * blockDim.x + threadIdx.x; q < kT * kT; q += gridDim.y * blockDim.x) {
@@ -113,8 +106,7 @@ __global__ void __launch_bounds__(256) k_sym_tiles(int M, int nT, const T *__res
     __shared__ double rowacc[8][kT][4];
     if (ss && ss->done) return;
     const size_t t = blockIdx.x;
-    int I = 0;
-    while (tile_index(I + 1, I + 1, nT) <= t && I + 1 < nT) ++I;
+    const int I = tile_row(t, nT);
     const int J = I + (int)(t - tile_index(I, I, nT));
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x < kT) {
@@ -218,8 +210,7 @@ __global__ void __launch_bounds__(256) k_sym_free_tiles(DevParams P, const doubl
     __shared__ double colacc[kT][4];
     const int M = P.M;
     const size_t t = blockIdx.x;
-    int I = 0;
-    while (tile_index(I + 1, I + 1, nT) <= t && I + 1 < nT) ++I;
+    const int I = tile_row(t, nT);
     const int J = I + (int)(t - tile_index(I, I, nT));
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x < 2 * kT) {

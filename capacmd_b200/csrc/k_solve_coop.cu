@@ -81,10 +81,6 @@ constexpr unsigned kSuspendNs = 1000;
 
 enum { MODE_X = 0, MODE_P = 1, MODE_S = 2 };
 
-__host__ __device__ __forceinline__ size_t tile_index(int I, int J, int nT)
-{
-    return (size_t)I * nT - (size_t)I * (I - 1) / 2 + (size_t)(J - I);
-}
 __device__ __forceinline__ int elem_offset(int p, int a, int b)
 {
     return ((p * (kT / 4) + (b >> 2)) * (kT * 4)) + a * 4 + (b & 3);
@@ -295,13 +291,20 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p)
     return v;
 }
 
-__device__ bool grid_barrier(CoopSync *bar, long limit)
+// In two halves, so that a block can work between its arrival and its wait:
+// thread 0's count before the arrival is passed from one to the other.
+__device__ __forceinline__ unsigned grid_arrive(CoopSync *bar)
+{
+    __syncthreads();
+    if (threadIdx.x != 0) return 0;
+    __threadfence();
+    return atomicAdd(&bar->count, 1u);
+}
+
+__device__ bool grid_wait(CoopSync *bar, long limit, unsigned arrived)
 {
     __shared__ int ok;
-    __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned arrived = atomicAdd(&bar->count, 1u);
         bool good = (arrived & kBarAbort) == 0;
         const unsigned target = ((arrived & ~kBarAbort) / gridDim.x + 1) * gridDim.x;
         long spins = 0;
@@ -325,6 +328,11 @@ __device__ bool grid_barrier(CoopSync *bar, long limit)
     return ok != 0;
 }
 
+__device__ __forceinline__ bool grid_barrier(CoopSync *bar, long limit)
+{
+    return grid_wait(bar, limit, grid_arrive(bar));
+}
+
 // A block that stops early (a ring wait that gave up) ends the other blocks'
 // barrier waits.
 __device__ __forceinline__ void grid_abort(CoopSync *bar, int code)
@@ -336,17 +344,23 @@ __device__ __forceinline__ void grid_abort(CoopSync *bar, int code)
 // Dot partials: kBp doubles per block.  sum_bp sums them over the blocks
 // in one fixed order, so every block gets the same K sums.
 constexpr int kBp = 16;
-template <int K>
-__device__ void sum_bp(const double *bp, int nb, double (&out)[K])
+// Shared memory of the dot sums, one piece for all of them (an array in each
+// instance of the functions below cost a block 1 KB each, and the second block
+// per SM its place).
+__device__ __forceinline__ double *dot_scratch()
 {
-    __shared__ double sh[kWarps * kBp];
-    __shared__ double res[kBp];
-    double v[K];
+    __shared__ double sh[kWarps * kBp + kBp];
+    return sh;
+}
+
+// In two halves: this thread's share of the partials (loads only), and the
+// sums over the block.
+template <int K>
+__device__ __forceinline__ void load_bp(const double *bp, int nb, double (&v)[K])
+{
 #pragma unroll
     for (int q = 0; q < K; ++q) v[q] = 0.0;
-    // two blocks' partials per thread per round of loads (the grid is at
-    // most two blocks per SM, so one round covers it)
-    for (int k = threadIdx.x; k < nb; k += 2 * blockDim.x) {
+    for (int k = threadIdx.x; k < nb; k += 2 * (int)blockDim.x) {
         const int k2 = k + (int)blockDim.x;
         double a[K], b[K];
 #pragma unroll
@@ -357,6 +371,12 @@ __device__ void sum_bp(const double *bp, int nb, double (&out)[K])
 #pragma unroll
         for (int q = 0; q < K; ++q) v[q] += a[q] + b[q];
     }
+}
+
+template <int K>
+__device__ void total_bp(double (&v)[K], double (&out)[K])
+{
+    double *sh = dot_scratch(), *res = sh + kWarps * kBp;
     block_sum<K>(v, sh);
     if (threadIdx.x == 0)
 #pragma unroll
@@ -368,10 +388,17 @@ __device__ void sum_bp(const double *bp, int nb, double (&out)[K])
 }
 
 template <int K>
+__device__ __forceinline__ void sum_bp(const double *bp, int nb, double (&out)[K])
+{
+    double v[K];
+    load_bp<K>(bp, nb, v);
+    total_bp<K>(v, out);
+}
+
+template <int K>
 __device__ void put_bp(double *bp, double (&v)[K])
 {
-    __shared__ double sh[kWarps * kBp];
-    block_sum<K>(v, sh);
+    block_sum<K>(v, dot_scratch());
     if (threadIdx.x == 0)
 #pragma unroll
         for (int q = 0; q < K; ++q) bp[(size_t)kBp * blockIdx.x + q] = v[q];
@@ -504,8 +531,7 @@ __device__ bool tiles_pass(const CoopArgs &A, const PassScalars &S, Ring<T> &rin
         const int nc = min(kChunk, ring.n_my - c0);
         if (threadIdx.x < nc) {
             const int t = blockIdx.x + (c0 + threadIdx.x) * gridDim.x;
-            int I = 0;
-            while (tile_index(I + 1, I + 1, A.nT) <= (size_t)t && I + 1 < A.nT) ++I;
+            const int I = tile_row(t, A.nT);
             sm.tile_i[threadIdx.x] = I;
             sm.tile_j[threadIdx.x] = I + (int)((size_t)t - tile_index(I, I, A.nT));
         }
@@ -1080,7 +1106,7 @@ constexpr uint32_t kTmemCols = 512;    // columns allocated per block
 static_assert(kResTiles * kResCols <= (int)kTmemCols, "resident tiles exceed the allocation");
 template <int MODE>
 __device__ bool tiles_pass_g(const GroupArgs &A, const PassScalars &S, Ring<float> &ring, PassSmem<float> &sm,
-                             int n_res, uint32_t tw)
+                             int n_res, uint32_t tw, bool &decoded)
 {
     constexpr int Stages = Ring<float>::Stages;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1100,14 +1126,18 @@ __device__ bool tiles_pass_g(const GroupArgs &A, const PassScalars &S, Ring<floa
     const int n_all = n_res + ring.n_my;
     for (int c0 = 0; c0 < n_all; c0 += kChunk) {
         const int nc = min(kChunk, n_all - c0);
-        if (threadIdx.x < nc) {
-            const int t = blockIdx.x + (c0 + threadIdx.x) * gridDim.x;
-            int I = 0;
-            while (tile_index(I + 1, I + 1, nT) <= (size_t)t && I + 1 < nT) ++I;
-            sm.tile_i[threadIdx.x] = I;
-            sm.tile_j[threadIdx.x] = I + (int)((size_t)t - tile_index(I, I, nT));
+        // a block whose tiles are one chunk (all up to 2,200 atoms) finds their rows
+        // and columns in its first pass
+        if (!decoded) {
+            if (threadIdx.x < nc) {
+                const int t = blockIdx.x + (c0 + threadIdx.x) * gridDim.x;
+                const int I = tile_row(t, nT);
+                sm.tile_i[threadIdx.x] = I;
+                sm.tile_j[threadIdx.x] = I + (int)((size_t)t - tile_index(I, I, nT));
+            }
+            decoded = n_all <= kChunk;
+            __syncthreads();
         }
-        __syncthreads();
 #pragma unroll 4
         for (int e = threadIdx.x; e < nc * 256; e += kBlock) {
             const int kk = e >> 8, side = (e >> 7) & 1, q4 = e & 127;
@@ -1373,8 +1403,15 @@ constexpr int kCoarseMax = 384;  // coarse columns the solver's shared buffer ho
 // in place of the block-Jacobi K alone: first the rows of `out` (v, t or r),
 // the dots that do not involve K out, and the mode sums (and the constraint
 // rows) into zbuf; a grid barrier; then K out = Z c + K out - (K W) zbuf,
-// c = E^-1 zbuf, with the dots of K out.  Returns false when the grid barrier
-// gave up.  scratch: 256 + 2 kCoarseMax doubles of shared memory (the pass
+// c = E^-1 zbuf, with the dots of K out; then the grid barrier that ends the
+// phase.  Returns false when a grid barrier gave up.  RED_START leaves the block
+// partials of (r, r) in bp.  RED_V and RED_T sum their dots into dots (the same
+// in every block).  RED_V's one comes from the first step: it is written before the
+// barrier between the steps, loaded beside the second step's operands and summed
+// while the last blocks arrive at the closing barrier (S phase at 91,122 atoms 8.6
+// -> 7.0 us).  Five of RED_T's seven could go the same way, but two cannot, and
+// two sums cost more than one (9.5 -> 10.5 us).
+// scratch: 256 + 2 kCoarseMax doubles of shared memory (the pass
 // inputs' buffer, idle between passes).
 //
 // A work item is a quarter of a group, 32 rows, so that 4 nG blocks share
@@ -1386,7 +1423,7 @@ constexpr int kCoarseMax = 384;  // coarse columns the solver's shared buffer ho
 // 10.3 of 69.5 (2,057); now 4.5 and 5.0, 5.4 and 6.4.
 template <int RED>
 __device__ bool reduce_group2(const GroupArgs &A, const PassScalars &S, double *bp, bool products, double *scratch,
-                              int iter = 0, int mark = -1)
+                              double (&dots)[7], int iter = 0, int mark = -1)
 {
     // vq: mode sums of the step's 8 atoms; vs: the group's rows of out; ps:
     // partial sums of the warps; cc, zs: c of the group's columns, Z^T out
@@ -1488,8 +1525,11 @@ __device__ bool reduce_group2(const GroupArgs &A, const PassScalars &S, double *
         }
         __syncthreads();
     }
+    double early[1] = {d[0]};
+    if (RED == RED_V) put_bp<1>(bp, early);
     if (!grid_barrier(A.sync, A.spin_limit)) return false;
     if (mark >= 0) g_phase_mark(A, iter, mark);  // the phase timer splits the two steps
+    if (RED == RED_V) load_bp<1>(bp, gridDim.x, early);
 
     const bool mine = (int)blockIdx.x < 4 * nG || (int)gridDim.x - 1 - (int)blockIdx.x < A.n_nps;
     if (mine) {
@@ -1573,12 +1613,20 @@ __device__ bool reduce_group2(const GroupArgs &A, const PassScalars &S, double *
         }
         __syncthreads();
     }
+    if (RED == RED_V) {
+        const unsigned arrived = grid_arrive(A.sync);
+        double sum[1];
+        total_bp<1>(early, sum);
+        dots[0] = sum[0];
+        return grid_wait(A.sync, A.spin_limit, arrived);
+    }
     if (RED == RED_T) {
         put_bp<7>(bp, d);
     } else {
-        double d1[1] = {d[0]};
-        put_bp<1>(bp, d1);
+        put_bp<1>(bp, early);
     }
+    if (!grid_barrier(A.sync, A.spin_limit)) return false;
+    if (RED == RED_T) sum_bp<7>(bp, gridDim.x, dots);
     return true;
 }
 
@@ -1648,6 +1696,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_bicgstab_group(GroupArgs A)
 
     PassScalars S{0.0, 0.0, 0.0, 0, 1};
     int iter = 0, status = 0;
+    bool decoded = false;  // the block's tile table holds (tiles_pass_g)
     double bTb = 0.0, crit = 0.0, rTr = 0.0, rr0 = 0.0;
     double ref_rTr = 0.0;  // (r, r) when it last halved
     int last_gain = 0;
@@ -1682,14 +1731,16 @@ __global__ void __launch_bounds__(kBlock, 2) k_bicgstab_group(GroupArgs A)
     if (!done) {
         // r0 = r = b - A x, K r (x zero: no product pass; the ring is
         // untouched, so the next pass starts on the same tiles)
-        if (!x_zero) ok = tiles_pass_g<MODE_X>(A, S, ring, psm, n_res, tw) && grid_barrier(A.sync, A.spin_limit);
+        if (!x_zero) ok = tiles_pass_g<MODE_X>(A, S, ring, psm, n_res, tw, decoded) && grid_barrier(A.sync, A.spin_limit);
         if (ok) {
-            if (A.nc > 0)
-                ok = reduce_group2<RED_START>(A, S, bpB, !x_zero, pscratch);
-            else
+            double none[7];
+            if (A.nc > 0) {
+                ok = reduce_group2<RED_START>(A, S, bpB, !x_zero, pscratch, none);
+            } else {
                 reduce_group<RED_START>(A, S, bpB, !x_zero);
+                ok = grid_barrier(A.sync, A.spin_limit);
+            }
         }
-        ok = ok && grid_barrier(A.sync, A.spin_limit);
         done = !ok;
     }
     double rho = 0.0, rho_old = 1.0, alpha = 1.0, omega = 1.0;
@@ -1706,30 +1757,29 @@ __global__ void __launch_bounds__(kBlock, 2) k_bicgstab_group(GroupArgs A)
         S.beta = (rho / rho_old) * (alpha / omega);
         S.omega = omega;
         S.alpha = alpha;
-        ok = tiles_pass_g<MODE_P>(A, S, ring, psm, n_res, tw);
+        ok = tiles_pass_g<MODE_P>(A, S, ring, psm, n_res, tw, decoded);
         g_phase_mark(A, iter, 1);
         ok = ok && grid_barrier(A.sync, A.spin_limit);
         if (!ok) break;
         pending = false;  // the P pass applied the previous iteration's x update
         g_phase_mark(A, iter, 2);
         S.first = 0;
+        double d[7];
         if (A.nc > 0) {
-            if (!reduce_group2<RED_V>(A, S, bpA, true, pscratch, iter, 3)) {
-                ok = false;
-                break;
-            }
+            ok = reduce_group2<RED_V>(A, S, bpA, true, pscratch, d, iter, 3);
         } else {
             reduce_group<RED_V>(A, S, bpA, true);
+            ok = grid_barrier(A.sync, A.spin_limit);
         }
-        if (!grid_barrier(A.sync, A.spin_limit)) {
-            ok = false;
-            break;
-        }
+        if (!ok) break;
         if (A.nc == 0) g_phase_mark(A, iter, 3);
         g_phase_mark(A, iter, 4);
-        double r0v[1];
-        sum_bp<1>(bpA, nb, r0v);
-        const double al = rho / r0v[0];
+        if (A.nc == 0) {
+            double r0v[1];
+            sum_bp<1>(bpA, nb, r0v);
+            d[0] = r0v[0];
+        }
+        const double al = rho / d[0];
         if (!isfinite(al)) {  // breakdown: x is the start of this iteration
             status = rTr < crit * 100.0 ? 1 : -2;
             break;
@@ -1737,25 +1787,19 @@ __global__ void __launch_bounds__(kBlock, 2) k_bicgstab_group(GroupArgs A)
         alpha = al;
         S.cur ^= 1;
         S.alpha = alpha;
-        ok = tiles_pass_g<MODE_S>(A, S, ring, psm, n_res, tw) && grid_barrier(A.sync, A.spin_limit);
+        ok = tiles_pass_g<MODE_S>(A, S, ring, psm, n_res, tw, decoded) && grid_barrier(A.sync, A.spin_limit);
         if (!ok) break;
         g_phase_mark(A, iter, 5);
         if (A.nc > 0) {
-            if (!reduce_group2<RED_T>(A, S, bpB, true, pscratch, iter, 6)) {
-                ok = false;
-                break;
-            }
+            ok = reduce_group2<RED_T>(A, S, bpB, true, pscratch, d, iter, 6);
         } else {
             reduce_group<RED_T>(A, S, bpB, true);
+            ok = grid_barrier(A.sync, A.spin_limit);
         }
-        if (!grid_barrier(A.sync, A.spin_limit)) {
-            ok = false;
-            break;
-        }
+        if (!ok) break;
         if (A.nc == 0) g_phase_mark(A, iter, 6);
         g_phase_mark(A, iter, 7);
-        double d[7];
-        sum_bp<7>(bpB, nb, d);
+        if (A.nc == 0) sum_bp<7>(bpB, nb, d);
         const double om = d[0] / d[1];
         if (!isfinite(om) || om == 0.0) {
             status = rTr < crit * 100.0 ? 1 : -2;
