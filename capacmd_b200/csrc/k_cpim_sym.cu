@@ -251,18 +251,10 @@ __global__ void __launch_bounds__(256) k_sym_free_tiles(DevParams P, const doubl
             cb[k][3] = m[0] * xr[a][0] + m[1] * xr[a][1] + m[2] * xr[a][2] + C * xr[a][3];
         }
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) cb[k][c] = warp_sum(cb[k][c]);
+    const double col = warp_sum_halving<16>(reinterpret_cast<double(&)[16]>(cb), lane);
 #pragma unroll
     for (int c = 0; c < 4; ++c) rowacc[w][a][c] = ra[c];
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) colacc[4 * w + k][c] = cb[k][c];
-    }
+    if ((lane & 1) == 0) colacc[4 * w + (lane >> 3)][(lane >> 1) & 3] = col;
     __syncthreads();
     double *pr = part + ((size_t)I * nT + J) * (kT * 4);
     double *pc = part + ((size_t)J * nT + I) * (kT * 4);
