@@ -1198,7 +1198,7 @@ void launch_external_field(capac_ctx *c)
 // The areas of a force call's partials; returns their doubles.
 size_t force_partial_areas(const capac_ctx *c, size_t off[4])
 {
-    const size_t pair = std::max((size_t)grid_for((long)c->N * 32, 256), (size_t)c->num_sms * 5) * 11;  // or a resident grid
+    const size_t pair = std::max((size_t)grid_for(c->N, 4), (size_t)c->num_sms * 5) * 11;  // or a resident grid
     const size_t n[4] = {(size_t)c->M * 10, pair, (size_t)c->M * 15,
                          (size_t)grid_for(c->N, 256)};
     size_t at = 0;
@@ -1211,7 +1211,7 @@ size_t force_partial_areas(const capac_ctx *c, size_t off[4])
 
 size_t partials_needed(const capac_ctx *c)
 {
-    const size_t pair_blocks = grid_for((long)c->N * 32, 256);
+    const size_t pair_blocks = grid_for(c->N, 4);  // k_pair: four warps of one atom each
     size_t need = pair_blocks * 11;
     need = std::max(need, (size_t)c->num_sms * 5 * 11);  // resident pair grids (at most five blocks per SM)
     need = std::max(need, (size_t)grid_for((long)c->N, 256) * 16);

@@ -14,7 +14,9 @@
 // every pair the FP64 test accepts, and the entries that pass are compacted in
 // shared memory, 4 bytes each; then full warps form the FP64 difference, test it
 // and compute, their positions loaded one set ahead.  In FP64 the terms of an
-// ordinary pair are dsf_terms' ~55 operations.
+// ordinary pair are dsf_terms' ~55 operations.  Bound by latency and issue together:
+// at 24,000 atoms (FP64) 499 -> 347 us a launch, issue slots 55% busy, FP64 pipe 30%,
+// sixteen warps per SM of 128 registers, a quarter of the instructions FP64.
 //
 // The same traversal adds, on each charged non-metal atom, the force from the
 // induced charges and dipoles of metal neighbours inside the cut-off: the
@@ -32,7 +34,7 @@ namespace capac {
 
 namespace {
 
-constexpr int kPairWarps = 8;  // warps per block
+constexpr int kPairWarps = 4;  // warps per block: a block ends with its longest row (24,000 atoms, eight: 2% more)
 
 // FP32 constants of the run.
 struct PairConstsF {
@@ -73,6 +75,7 @@ __device__ __forceinline__ float rcp_approx(float x)
     return r;
 }
 
+__device__ __forceinline__ float erfc_from_gauss_f(float x, float gauss);
 // erfc(x) for 0 <= x in FP32 as exp(-x^2) R(x), with R(x) = erfc(x) exp(x^2)
 // (the scaled complementary error function) fitted on [0, 5] by a degree-9
 // polynomial in t = 1 / (1 + x / 2), least squares in relative error
@@ -307,12 +310,15 @@ __device__ __forceinline__ double image1(double d, double L, double H) { return 
 
 // One warp per atom i (grid-stride); see the file comment.
 template <typename Real, bool NONBONDED, bool CPIM>
-__global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 3 : 2) k_pair(
+__global__ void __launch_bounds__(kPairWarps * 32, sizeof(Real) == 4 ? 6 : 4) k_pair(
     DevParams P, PairConstsF K, const double4 *__restrict__ pos4, const float4 *__restrict__ pos4f,
     const uint32_t *__restrict__ nbr, const int *__restrict__ nnb, int cap, const double *__restrict__ vec_pq,
     double *__restrict__ fx, double *__restrict__ fy, double *__restrict__ fz, double *__restrict__ partials)
 {
-    constexpr int NB = 2;                            // chunks of 32 candidates tested together
+    // chunks of 32 candidates tested together; one where the FP64 CPIM terms need
+    // the registers (9,309 atoms in 3,000 waters: two take 3.5% more of a step, without
+    // those terms one takes 2% more)
+    constexpr int NB = sizeof(Real) == 8 && CPIM ? 1 : 2;
     __shared__ uint32_t queue[kPairWarps][32 * (NB + 1)];  // < 32 left over and NB x 32 appended
     __shared__ double sh[32 * 11];
     __shared__ double wacc[kPairWarps][8];  // per warp: e_qq, e_vdw, virial xx xy xz yy yz zz
