@@ -725,8 +725,16 @@ bool dense_fits(int device, int n, bool mixed)
     CAPAC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const void *k = dense_kernel(n, sms, mixed);
     if (!k) return false;
+    // The limit on a launch's dynamic shared memory belongs to the kernel, which
+    // contexts of other sizes launch too: all that a block can have, not this
+    // system's need, so that creating one context takes nothing from another.
     const size_t smem = dense_smem(n, mixed);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    int most = 0;
+    cudaFuncAttributes fa{};
+    CAPAC_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes) !=
+            cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kBlock, smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
