@@ -39,7 +39,7 @@ constexpr int kPairWarps = 4;  // warps per block: a block ends with its longest
 // FP32 constants of the run.
 struct PairConstsF {
     float rc, inv_rc, inv_rc12, inv_rc6, alpha, a2_sqrtpi, w_const, w_erfc_arcut, fqq, rc2;
-    float gauss2;  // -alpha^2 log2(e)
+    float gauss2, gauss2_lo;  // -alpha^2 log2(e) as a sum of two
     int use_vdw, use_coulomb;
     double iL[3];  // 1 / box edge
 };
@@ -879,11 +879,14 @@ __device__ __forceinline__ float rsqrt_approx(float x)
 // and the options are the shifted-force van der Waals and the damped Coulomb
 // form with alpha rc < 5, the range of the fitted erfc; `general` otherwise
 // (pair_term_f, all forms; also with more types than the shared tables hold).
-// The short route takes the Gaussian as 2^(-alpha^2 log2(e) r^2) from r^2 itself
-// and sharpens 1/r by a Newton step.  Against 64 bits, alpha 2, r 0.12..1.2 nm: the
-// Gaussian within 4e-7 (expf of the rounded (alpha r)^2: 1.5e-6), the Coulomb
-// force's rms error 9.80e-6 (9.84e-6) nm^-2, the energy's mean error weighted by r^2
-// -0.8e-9 (1.2e-9) and its rms 7.3e-9 (8.5e-9) nm.  The virial from the entry's
+// The short route takes the Gaussian as 2^(-alpha^2 log2(e) r^2) from r^2 itself,
+// the constant as a sum of two (rounded to one, the Gaussian is off by up to 6e-8
+// (alpha r)^2 of one sign in all pairs alike), and sharpens 1/r by a Newton step.
+// Against 64 bits, alpha 2, r 0.12..1.2 nm: the Gaussian within 4e-7 and its mean
+// within 2e-10 (expf of the rounded (alpha r)^2: 1.5e-6, 9e-10).  Net forces, rms
+// relative error with expf and rsqrtf -> one rounded constant -> now: 7.58e-7 ->
+// 7.91e-7 -> 7.45e-7 (8,000 waters around Au561), 6.86e-7 -> 6.97e-7 -> 6.94e-7
+// (30,000 waters, two Au561).  The virial from the entry's
 // summed force instead of per pair is 1% faster and 15% less accurate.
 //
 // The water-side CPIM term walks the entries a second time, only for clusters next
@@ -1075,7 +1078,7 @@ __global__ void __launch_bounds__(kHalfWarps * 32, kHalfBlocks) k_pair_half(
                         }
                     }
                     if (mk.w != 0.f && bq != 0.f) {
-                        const float qq = K.fqq * mk.w * bq, eg = exp2_approx(K.gauss2 * r2),
+                        const float qq = K.fqq * mk.w * bq, eg = exp2_approx(fmaf(K.gauss2, r2, K.gauss2_lo * r2)),
                                     ec = erfc_near_f(K.alpha * r, eg);
                         fp += qq * ((ec * r2inv + K.a2_sqrtpi * eg * rinv) - K.w_const) * rinv;
                         eq = qq * (ec * rinv - K.w_erfc_arcut + K.w_const * (r - K.rc));
@@ -1357,7 +1360,9 @@ PairConstsF pair_consts_f(const capac_ctx *c)
     K.w_erfc_arcut = (float)c->P.w_erfc_arcut;
     K.fqq = (float)kFQQ;
     K.rc2 = (float)c->P.rc2;
-    K.gauss2 = (float)(-c->P.w_alpha * c->P.w_alpha * 1.4426950408889634074);
+    const double g2 = -c->P.w_alpha * c->P.w_alpha * 1.4426950408889634074;
+    K.gauss2 = (float)g2;
+    K.gauss2_lo = (float)(g2 - (double)K.gauss2);
     K.use_vdw = c->P.use_vdw;
     K.use_coulomb = c->P.use_coulomb;
     for (int a = 0; a < 3; ++a) K.iL[a] = 1.0 / c->P.box.L[a];
