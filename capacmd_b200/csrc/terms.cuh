@@ -6,16 +6,25 @@
 namespace capac {
 
 // exp(-x^2) and erfc(x) with x = alpha r, and 1/r, of one damped Coulomb pair,
-// for alpha r < kDsfMaxX: no branch and no call, ~55 FP64 operations where
+// for alpha r < kDsfMaxX: no branch and no call, ~63 FP64 operations where
 // sqrt, the division, exp and erfc take about 200.
 //
-// 1/r: the hardware approximation and one step of third order (remainder
-// 5/16 e^3 of an e below 2^-19).  exp(-x^2): x^2 with its rounding error, 2^n
-// split off, and 1 + f + f^2 q(f) on |f| <= ln2 / 2 with q a Chebyshev
-// interpolant (1.6e-17 of the result).  erfc(x) = exp(-x^2) R(x), R the scaled
-// complementary error function as a polynomial of degree 18 in
+// 1/r: the hardware's approximation y and one step of the series of r^2 y^2 = 1 - e,
+// 1/r = y (1 - e)^(-1/2), to e^2: third order (remainder 5/16 e^3 of an e below
+// 2^-19).  exp(-x^2): -alpha^2 r^2 with the product's rounding error (from r already
+// rounded it would carry 2 x^2 of that rounding: 3.0e-16 for 5.1e-17 at the alpha
+// and r below), 2^n split off, and 1 + f + f^2 q(f) on |f| <= ln2 / 2 with q a
+// Chebyshev interpolant (1.6e-17 of the result).  erfc(x) = exp(-x^2) R(x), R the
+// scaled complementary error function as a polynomial of degree 18 in
 // u = (x - 3.5) / (x + 3.5), Chebyshev interpolant on [0, 5] (3.7e-17 of R with
-// the rounded coefficients); both polynomials in two chains.
+// the rounded coefficients); both polynomials in two chains.  R changes by up to
+// twice the relative change of u, so u is rounded once: without the sum's and the
+// quotient's remainders erfc's error was 2.2e-16 where it is 1.05e-16.
+//
+// Rms relative error against 64 bits of alpha 2, r 0.12 .. 1.2 (CUDA's functions on
+// the same r^2 in brackets): Gaussian 5.1e-17 (4.8e-17), erfc 1.05e-16 (1.8e-16);
+// the damped Coulomb force and energy of unit charges, absolute, 1.48e-14 (1.55e-14)
+// and 1.70e-16 (1.83e-16).
 //
 // W of them side by side (the three widths of a metal pair share the constants'
 // moves).  Two pairs a lane in k_pair take ~160 registers, twelve warps per SM
@@ -41,9 +50,9 @@ __device__ __forceinline__ void dsf_terms(const double (&alpha)[W], const double
     });
     // exp(-x^2): n = round(-x^2 log2 e) from the low word of an addition to 1.5 2^52
     each([&](int w) {
-        const double x = alpha[w] * d[w].r;
-        x2[w] = x * x;
-        const double lo = fma(x, x, -x2[w]);
+        const double al2 = alpha[w] * alpha[w];
+        x2[w] = al2 * r2[w];
+        const double lo = fma(al2, r2[w], -x2[w]);
         kd[w] = fma(x2[w], -1.4426950408889634, 0x1.8p52);
         const double n = kd[w] - 0x1.8p52;
         f[w] = fma(n, -0x1.473de6af278edp-34, fma(n, -0x1.62e42fef00000p-1, -x2[w])) - lo;
@@ -60,11 +69,13 @@ __device__ __forceinline__ void dsf_terms(const double (&alpha)[W], const double
     each([&](int w) {
         const double g = 1.0 + fma(f2[w], fma(a[w], f[w], b[w]), f[w]);
         d[w].eg = __hiloint2double(__double2hiint(g) + (__double2loint(kd[w]) << 20), __double2loint(g));
-        // R(x)
-        const double z = fma(alpha[w], d[w].r, 3.5);
+        // R(x): u = 1 - 7 / (x + 3.5), the sum as z and its rounding error, the
+        // quotient as q and the rest of its division
+        const double z = fma(alpha[w], d[w].r, 3.5), dz = fma(alpha[w], d[w].r, 3.5 - z);
         asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y[w]) : "d"(z));
-        e[w] = fma(-z, y[w], 1.0);
-        u[w] = fma(-7.0, fma(y[w], fma(e[w], e[w], e[w]), y[w]), 1.0);
+        y[w] = fma(y[w], fma(-z, y[w], 1.0), y[w]);
+        const double q = 7.0 * y[w];
+        u[w] = fma(-y[w], fma(-dz, q, fma(-z, q, 7.0)), 1.0 - q);
         u2[w] = u[w] * u[w];
         a[w] = fma(1.44851080807840048e-07, u2[w], 9.39502676422655287e-07);
         b[w] = fma(1.21445591197839242e-08, u2[w], 6.32563657300747914e-07);
@@ -84,7 +95,10 @@ __device__ __forceinline__ void dsf_terms(const double (&alpha)[W], const double
     chain(a, u2, -2.89265044832767437e-01);
     chain(b, u2, 2.33130481600251627e-01);
     chain(b, u2, 1.55293655608894299e-01);
-    each([&](int w) { d[w].ec = d[w].eg * fma(a[w], u[w], b[w]); });
+    each([&](int w) {  // with the last addition's rounding error
+        const double R = fma(a[w], u[w], b[w]);
+        d[w].ec = fma(d[w].eg, R, d[w].eg * fma(a[w], u[w], b[w] - R));
+    });
 }
 __device__ __forceinline__ Dsf dsf_terms(double alpha, double r2)
 {
@@ -186,10 +200,12 @@ __device__ __forceinline__ void cpim_block(const DevParams &P, const double4 &pi
     r[0] *= kNm2Bohr;
     r[1] *= kNm2Bohr;
     r[2] *= kNm2Bohr;
-    // the three widths' Gaussians and erf = 1 - erfc side by side; erfc is below
-    // 1e-17 beyond the fitted range, where its relative error grows, and x is
-    // held below 26 there, where all is zero.  Below 1 the library's erf keeps
-    // the relative error that 1 - erfc loses.
+    // the three widths' Gaussians and erf = 1 - erfc side by side.  Beyond the fitted
+    // range R is a polynomial continued outside its interval: it grows no faster
+    // than the Chebyshev polynomial of degree 18, and times 3.7e-17 of R and
+    // erfc(x) that is below 1e-24 everywhere beyond x = 5.  x is held below 26, where
+    // all is zero.  Below 1 the library's erf keeps the relative error that 1 - erfc
+    // loses.
     const double r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
     const double ip[3] = {P.inv_r_pp, P.inv_r_pq, P.inv_r_qq};
     double al[3], er[3], g[3];
@@ -203,7 +219,7 @@ __device__ __forceinline__ void cpim_block(const DevParams &P, const double4 &pi
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         g[k] = d[k].eg;
-        er[k] = rr * ip[k] < 1.0 ? erf(rr * ip[k]) : 1.0 - d[k].ec;
+        er[k] = rr * ip[k] < 1.0 ? erf(sqrt(r2) * ip[k]) : 1.0 - d[k].ec;
     }
     const double c1 = ir3 * r2inv * (er[0] - 2.0 * kInvSqrtPi * ip[0] * rr * g[0]);
     const double c2 = 4.0 * kInvSqrtPi * (ip[0] * ip[0] * ip[0]) * r2inv * g[0];

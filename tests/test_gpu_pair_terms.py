@@ -1,4 +1,4 @@
-"""Systematic error of the mixed path's pair terms, on isolated ion pairs.
+"""Errors of the pair terms on isolated ion pairs.
 
 4,096 pairs of opposite charges, more than the cut-off from each other, at
 separations r between 0.7 and 1.0 nm (alpha r between 1.7 and 2.45, where the
@@ -12,7 +12,16 @@ the two terms (6e-8 of a share that varies by a tenth: 2e-9), and the rounding
 of r^2, the Gaussian and the products, zero on average, 4e-7 a pair and so
 7e-9 on the slope of 4,096.  In all below 1.5e-8; half the rounded constant's
 slope, 2.5e-8, is the bound.
+
+FP64 path: the force of each pair over its separation against decimal
+arithmetic on the same r^2.  Its roundings: the Gaussian and erfc 1.1e-16 each
+(rms; a quarter of the force is erfc's), the sum, the two products with 1/r and
+1/r itself 0.5e-16 each, the constants 1e-16, the product with the component and
+the test's division by it 0.5e-16 each: 2.5e-16.  A Gaussian of a rounded r has
+2 (alpha r)^2, about nine, times that rounding's 0.6e-16 and more: above 5e-16.
+The bound is 4e-16.
 """
+import decimal
 import os
 
 import numpy as np
@@ -96,3 +105,44 @@ def test_half_list_gaussian_has_no_systematic_error(tmp_path):
     x2 = ALPHA ** 2 * (d * d).sum(1)
     slope = np.polyfit(x2, rel, 1)[0]
     assert abs(slope) < 2.5e-8, slope
+
+
+def _decimal_force(r2, alpha, rc):
+    """Damped shifted Coulomb force over r of unit charges, in 40 digits (alpha r below 3)."""
+    D = decimal.Decimal
+    with decimal.localcontext() as ctx:
+        ctx.prec = 40
+        isp = D("0.56418958354775628694807945156077258584405")
+        isp_field = D("0.564189583547756")  # the force field's constant, in fifteen digits (typedef.h:44)
+
+        def erfc(x):
+            t = s = x
+            k = 0
+            while abs(t) > D("1e-38"):
+                k += 1
+                t *= -x * x / k
+                s += t / (2 * k + 1)
+            return 1 - 2 * isp * s
+
+        def f(v):
+            r = v.sqrt()
+            return erfc(alpha * r) / v + 2 * alpha * isp_field * (-alpha * alpha * v).exp() / r
+
+        alpha, rc = D(alpha), D(rc)
+        shift = f(rc * rc)
+        return [(f(D(float(v))) - shift) / D(float(v)).sqrt() for v in r2]
+
+
+def test_fp64_damped_terms(tmp_path):
+    desc, n, _ = _ions(tmp_path)
+    s = cm.Simulation(desc)
+    x = s.positions()  # as read from the file
+    s.force()
+    d = x[n:] - x[:n]
+    r2 = d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1] + d[:, 2] * d[:, 2]  # rounded as the kernel rounds it
+    at, axis = np.arange(0, n, 4), np.abs(d).argmax(1)[::4]
+    got = s.forces()[at, axis] / d[at, axis]
+    exact = _decimal_force(r2[at], ALPHA, "1.2")
+    fqq = decimal.Decimal("138.935457696552")
+    rel = np.array([float(decimal.Decimal(float(g)) / (fqq * e) - 1) for g, e in zip(got, exact)])
+    assert np.sqrt((rel * rel).mean()) < 4e-16
