@@ -36,12 +36,18 @@ void check_ctx(capac_ctx *c)
     if (!c) throw Error(CAPAC_ERR_INVALID, "null context");
 }
 
-// Throws when a solve whose status has landed did not converge.
+// Throws when a solve whose status has landed did not converge or gave up; the
+// state is then no longer one that gradients can be taken of.
 void settle(capac_ctx *c)
 {
-    const int st = settle_solve(c);
-    if (st == CAPAC_OK) return;
+    if (!c->pending_solve) return;
+    const bool ready = c->grad_ready;
     c->grad_ready = false;
+    const int st = settle_solve(c);
+    if (st == CAPAC_OK) {
+        c->grad_ready = ready;
+        return;
+    }
     char msg[160];
     snprintf(msg, sizeof msg, "Error: bicg_stab not converged. rTr= %e, bTb= %e", c->h_ss->rTr, c->h_ss->bTb);
     throw Error(st, msg);
