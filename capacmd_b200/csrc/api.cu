@@ -53,6 +53,15 @@ void settle(capac_ctx *c)
     throw Error(st, msg);
 }
 
+// Waits for a solve whose status is still out, not for what is queued behind it,
+// and settles it.
+void await_solve(capac_ctx *c)
+{
+    if (!c->pending_solve) return;
+    CAPAC_CUDA(cudaEventSynchronize(c->ev_solve));
+    settle(c);
+}
+
 // Waits for the stream; throws the failures of RATTLE and of a pending solve.
 void check_flags(capac_ctx *c)
 {
@@ -678,6 +687,7 @@ int capac_create(const capac_desc *d, const capac_options *opt, capac_ctx **out)
             c->scount = dalloc<int>(2);
             CAPAC_CUDA(cudaMemsetAsync(c->scount, 0, sizeof(int) * 2, s));
             CAPAC_CUDA(cudaEventCreateWithFlags(&c->ev_flags, cudaEventDisableTiming));
+            CAPAC_CUDA(cudaEventCreateWithFlags(&c->ev_solve, cudaEventDisableTiming));
             if (const char *ps = getenv("CAPAC_PAIR_SPLIT")) c->pair_split_force = ps[0] == '0' ? 0 : 1;
             if (o.precision == CAPAC_PREC_MIXED && d->n_metal > 0 && d->use_cpff && getenv("CAPAC_OVERLAP")) {
                 c->overlap = true;
@@ -750,6 +760,7 @@ int capac_destroy(capac_ctx *c)
             if (e) cudaEventDestroy(e);
     }
     if (c->ev_flags) cudaEventDestroy(c->ev_flags);
+    if (c->ev_solve) cudaEventDestroy(c->ev_solve);
     for (auto &e : c->ev_stage)
         if (e) cudaEventDestroy(e);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -784,6 +795,7 @@ int capac_mpi_force(capac_ctx *c, const double *rx, const double *ry, const doub
         if (vec_pq && c->M > 0)
             CAPAC_CUDA(cudaMemcpyAsync(c->vec_pq, vec_pq, sizeof(double) * c->n_mat, cudaMemcpyHostToDevice, s));
         force(c);
+        await_solve(c);  // a failed solve leaves the caller's arrays as they are
         if (fx) fetch(c, fx, c->fx, nb);
         if (fy) fetch(c, fy, c->fy, nb);
         if (fz) fetch(c, fz, c->fz, nb);

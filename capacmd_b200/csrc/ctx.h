@@ -321,6 +321,7 @@ struct capac_ctx {
     cudaEvent_t ev_stage[8] = {};
     double *xyz = nullptr;
     bool pending_solve = false;  // the last solve's status is not read yet (settle_solve)
+    cudaEvent_t ev_solve = nullptr;  // behind that solve: its status has landed
     double pending_tol = 0.0;
     double *pot = nullptr, *vir = nullptr;  // [15], [9]
     capac::ThermoState *th = nullptr;

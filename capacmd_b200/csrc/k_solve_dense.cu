@@ -798,7 +798,10 @@ int bicgstab_dense(capac_ctx *c, const double *b, double *x, double tol, double 
                                                dim3(kBlock), args, dense_smem(A.n, mixed), c->stream));
     }
     ++c->launches;
-    if (defer) return CAPAC_OK;
+    if (defer) {
+        CAPAC_CUDA(cudaEventRecord(c->ev_solve, c->stream));
+        return CAPAC_OK;
+    }
     CAPAC_CUDA(cudaStreamSynchronize(c->stream));
     return dense_status(c, skip);
 }

@@ -36,6 +36,28 @@ def _both(monkeypatch, desc, **options):
     return small, tiled
 
 
+def _mpi_force(sim, pos, pq):
+    """capac_mpi_force on arrays of known contents; returns the status and the outputs."""
+    out = {k: np.full(sim.n_atoms, -7.0) for k in ("fx", "fy", "fz")}
+    out.update(potential=np.full(15, -7.0), virial=np.full(9, -7.0), vec_pq=pq.copy(), vec_ext=np.full(sim.n_mat, -7.0),
+               diag_relay=np.full(sim.n_mat, -7.0), inv_sqrt_dens=np.full(sim.desc.n_metal, -7.0))
+    xyz = [np.ascontiguousarray(pos[:, a]) for a in range(3)]
+    rc = cm.lib().capac_mpi_force(sim._p, *[a.ctypes.data for a in xyz], *[a.ctypes.data for a in out.values()])
+    return rc, out
+
+
+@pytest.mark.parametrize("how,code", [("max_iter", cm.ERR_NOT_CONVERGED), ("wait_polls", cm.ERR_CUDA)])
+def test_drop_in_call_leaves_the_callers_arrays(how, code, monkeypatch):
+    d = cm.Desc.from_paths(golden_paths("t_2np"))
+    pq = np.random.default_rng(5).normal(scale=1e-3, size=d.n_mat)
+    for sim in _both(monkeypatch, d, **{how: 1}, solver_tol=1e-26):
+        rc, out = _mpi_force(sim, sim.positions(), pq)
+        assert rc == code
+        assert np.array_equal(out.pop("vec_pq"), pq)
+        for name, v in out.items():
+            assert np.all(v == -7.0), name
+
+
 @pytest.mark.parametrize("prec", PRECS)
 def test_no_gradient_after_a_wait_that_ran_out(prec, monkeypatch):
     d = cm.Desc.from_paths(golden_paths("t_2np"))
