@@ -62,6 +62,18 @@ void await_solve(capac_ctx *c)
     settle(c);
 }
 
+// A solve whose call another failure ended before its status was read is not
+// this call's: its words are cleared.
+void drop_solve(capac_ctx *c)
+{
+    if (!c->pending_solve) return;
+    CAPAC_CUDA(cudaEventSynchronize(c->ev_solve));
+    try {
+        settle_solve(c);
+    } catch (const Error &) {
+    }
+}
+
 // Waits for the stream; throws the failures of RATTLE and of a pending solve.
 void check_flags(capac_ctx *c)
 {
@@ -78,14 +90,14 @@ void record(capac_ctx *c, int k)
 }
 
 // One mpi_force equivalent on the device state; solve = false keeps the
-// induced vector as it is.  The host waits once, for the displacement check
-// (and the previous call's solve, whose status is read there): the Sutton-Chen
-// and matrix kernels, which need no list, are queued before.  The caller waits
-// for this call's own status (check_flags) unless another force call follows.
+// induced vector as it is.  The host waits once, for the displacement check:
+// the Sutton-Chen and matrix kernels, which need no list, are queued before.
+// The caller waits for the status of the solve (await_solve, check_flags).
 void force(capac_ctx *c, bool solve = true)
 {
     cudaStream_t s = c->stream;
     c->grad_ready = false;
+    drop_solve(c);
     struct Defer {  // the launches' sums are left to launch_force_sums
         capac_ctx *c;
         explicit Defer(capac_ctx *cc) : c(cc)
@@ -106,7 +118,6 @@ void force(capac_ctx *c, bool solve = true)
     if (cpim) launch_cpim_matrix(c);
     record(c, 3);
     finish_begin_force(c);
-    settle(c);
     // the nonbonded pairs (their own stream) meanwhile with the CPIM stages
     const bool ovl = c->overlap && cpim && solve && c->clusters && c->cl_half;
     if (ovl) launch_pair_nonbonded_async(c);
@@ -140,8 +151,14 @@ void force(capac_ctx *c, bool solve = true)
     c->grad_ready = solve;
 }
 
+// A failed solve ends the run in its own step: its positions, half-kicked
+// velocities and forces are what the caller then finds.  A deferred one is
+// known to the host only after the rest of its step is queued, so that rest
+// looks at the solver's word itself and does nothing (halted, k_md.cu), and the
+// next step waits for the status before it changes anything.
 void md_step(capac_ctx *c, bool last)
 {
+    await_solve(c);
     const long step = ++c->md_step;
     const bool nvt = c->ensemble == CAPAC_NVT;
     if (nvt) launch_nhc(c, step);
@@ -159,6 +176,7 @@ void md_step(capac_ctx *c, bool last)
     launch_rattle(c, 1, true);
     launch_step_sums(c, c->ensemble, c->has_cstr);
     if (step % c->n_save == 0) {
+        await_solve(c);
         launch_apply_pbc(c);
         launch_fmax_rms(c);
     }

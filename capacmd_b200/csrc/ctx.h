@@ -19,6 +19,7 @@ struct SolverScalars {
     double rr0;      // (r, r) of the warm start
     int iter, done, status, max_iter;
     int error;       // dense solver: a bounded poll gave up
+    int failed;      // dense solver: the status is a failure (of the FP64 path, or of the refined solve)
     int outer;       // dense solver, mixed path: refinement sweeps
 };
 
@@ -320,7 +321,9 @@ struct capac_ctx {
     size_t stage_bytes = 0;
     cudaEvent_t ev_stage[8] = {};
     double *xyz = nullptr;
-    bool pending_solve = false;  // the last solve's status is not read yet (settle_solve)
+    // the last solve's status is not read yet (settle_solve; kernels that only a
+    // good one lets run look at ss, see halting)
+    bool pending_solve = false;
     cudaEvent_t ev_solve = nullptr;  // behind that solve: its status has landed
     double pending_tol = 0.0;
     double *pot = nullptr, *vir = nullptr;  // [15], [9]
@@ -435,6 +438,8 @@ void launch_rattle(capac_ctx *c, int second, bool in_step = false);
 void launch_step_sums(capac_ctx *c, int thermostat, bool rattle_virial);
 void launch_apply_pbc(capac_ctx *c);
 void launch_fmax_rms(capac_ctx *c);
+// for kernels that must not run after a failed solve: its scalars while the host has not read them
+inline const capac::SolverScalars *halting(const capac_ctx *c) { return c->pending_solve ? c->ss : nullptr; }
 void launch_interleave(capac_ctx *c, const double *x, const double *y, const double *z, double *out);
 void launch_sum_potential(capac_ctx *c);
 void launch_build_vsites(capac_ctx *c);   // k_bonded.cu

@@ -184,12 +184,16 @@ __global__ void k_kick_drift(MdParams m, const unsigned char *is_metal, const do
     vx[i] = a; vy[i] = b; vz[i] = c;
 }
 
+// A step's second half after a solve that failed (md_step): nothing may change.
+__device__ __forceinline__ bool halted(const SolverScalars *ss) { return ss && (ss->error | ss->failed) != 0; }
+
 // v += dt/2 F/m for atoms that move.
 __global__ void k_half_kick(MdParams m, const unsigned char *is_metal, const double *inv_mass, const double *fx,
-                            const double *fy, const double *fz, double *vx, double *vy, double *vz)
+                            const double *fy, const double *fz, double *vx, double *vy, double *vz,
+                            const SolverScalars *ss)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.N || (m.fix_metal == 1 && is_metal[i])) return;
+    if (i >= m.N || (m.fix_metal == 1 && is_metal[i]) || halted(ss)) return;
     const double im = inv_mass[i];
     vx[i] += m.dt_2 * fx[i] * im;
     vy[i] += m.dt_2 * fy[i] * im;
@@ -354,9 +358,11 @@ __global__ void __launch_bounds__(kRattleBlock) k_rattle1(MdParams m, CstrView c
 // virial goes to per-block partials.
 __global__ void __launch_bounds__(kRattleBlock) k_rattle2(MdParams m, CstrView cv, const double *rx, const double *ry,
                                                  const double *rz, double *vx, double *vy, double *vz,
-                                                 volatile int *failed, double *partials)
+                                                 volatile int *failed, double *partials,
+                                                 const SolverScalars *ss)
 {
     __shared__ double sh[32 * 9];
+    if (halted(ss)) return;
     double vir[9] = {0.0};
     const int im = blockIdx.x * blockDim.x + threadIdx.x;
     if (im < m.n_mols) {
@@ -489,9 +495,11 @@ __global__ void __launch_bounds__(256) k_step_sums(MdParams m, const double *__r
                                                    const double *__restrict__ vx, const double *__restrict__ vy,
                                                    const double *__restrict__ vz, int thermostat, double dt_over_tau,
                                                    ThermoState *th, double *partials, int *count,
-                                                   const double *__restrict__ rattle, int n_rattle, double *vir)
+                                                   const double *__restrict__ rattle, int n_rattle, double *vir,
+                                                   const SolverScalars *ss)
 {
     __shared__ double sh[32 * 9];
+    if (halted(ss)) return;
     double v[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.N; i += gridDim.x * blockDim.x) {
         const double mm = mass[i];
@@ -531,9 +539,10 @@ __global__ void __launch_bounds__(256) k_step_sums(MdParams m, const double *__r
 // finishes it), with sum_potential (force.c:322-331).
 __global__ void __launch_bounds__(256) k_step_apply(MdParams m, const double *__restrict__ mass, double *vx, double *vy,
                                                     double *vz, ThermoState *th, double *partials, int *count,
-                                                    double *pot)
+                                                    double *pot, const SolverScalars *ss)
 {
     __shared__ double sh[32 * 3];
+    if (halted(ss)) return;
     const double s = th->scale, c0 = th->vcom[0], c1 = th->vcom[1], c2 = th->vcom[2];
     double v[3] = {0.0, 0.0, 0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.N; i += gridDim.x * blockDim.x) {
@@ -730,7 +739,7 @@ void launch_md_kick_drift(capac_ctx *c, bool nvt, long step)
 void launch_md_half_kick(capac_ctx *c)
 {
     k_half_kick<<<grid_for(c->N, 256), 256, 0, c->stream>>>(md_params(c), c->is_metal, c->inv_mass, c->fx, c->fy,
-                                                           c->fz, c->vx, c->vy, c->vz);
+                                                           c->fz, c->vx, c->vy, c->vz, halting(c));
     ++c->launches;
 }
 
@@ -739,9 +748,9 @@ void launch_step_sums(capac_ctx *c, int thermostat, bool rattle_virial)
     const unsigned grid = std::min(grid_for(c->N, 256), (unsigned)kSumBlocks);
     const int nr = rattle_virial ? (int)grid_for(c->n_mols, kRattleBlock) : 0;
     k_step_sums<<<grid, 256, 0, c->stream>>>(md_params(c), c->mass, c->vx, c->vy, c->vz, thermostat, c->dt_over_tau,
-                                             c->th, c->spart, c->scount, c->partials, nr, c->vir);
+                                             c->th, c->spart, c->scount, c->partials, nr, c->vir, halting(c));
     k_step_apply<<<grid, 256, 0, c->stream>>>(md_params(c), c->mass, c->vx, c->vy, c->vz, c->th, c->spart,
-                                              c->scount + 1, c->pot);
+                                              c->scount + 1, c->pot, halting(c));
     c->launches += 2;
 }
 
@@ -755,7 +764,7 @@ void launch_rattle(capac_ctx *c, int second, bool in_step)
         ++c->launches;
     } else {
         k_rattle2<<<grid, kRattleBlock, 0, c->stream>>>(md_params(c), cstr_view(c), c->rx, c->ry, c->rz, c->vx, c->vy, c->vz,
-                                               c->sig + 2, c->partials);
+                                               c->sig + 2, c->partials, halting(c));
         ++c->launches;
         if (in_step) return;
         static const int pot_slots[9] = {-1, -1, -1, -1, -1, -1, -1, -1, -1};

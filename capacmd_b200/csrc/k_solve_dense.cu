@@ -680,6 +680,9 @@ __global__ void __launch_bounds__(kBlock, 1) k_bicgstab_dense(const __grid_const
             if (moved || predicted) A.x[rr] = xs[m][tid];
         }
         if (tid == 0) {
+            // as settle_solve decides it
+            if (BJ) A.ss->failed = bTb >= A.skip && (status < 0 || !(rTr <= crit)) && !(rTr < 1.0e-8 * bTb);
+            else A.ss->failed = status < 0;
             volatile SolverScalars *ss = A.out;
             ss->bTb = bTb;
             ss->crit = crit;

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import capacmd_b200 as cm
-from conftest import golden_paths
+from conftest import golden_paths, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -76,3 +76,53 @@ def test_no_gradient_after_a_wait_that_ran_out(prec, monkeypatch):
         sim.set("vec_pq", np.zeros(d.n_mat))
         sim.force()
         sim.energy_grad()
+
+
+STATE = ("rx", "ry", "rz", "vx", "vy", "vz", "fx", "fy", "fz", "virial", "thermo", "vQ")
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("case", ["t_2np", "t_au55w"])
+def test_failed_step_is_the_last_one(case, prec, monkeypatch):
+    """md_steps stops in the step whose solve failed: positions, velocities,
+    thermostat and step count are that step's, as after a solve that is
+    waited for at once."""
+    d = cm.Desc.from_paths(golden_paths(case))
+    small, tiled = _both(monkeypatch, d, precision=prec, **_tight(prec))
+    for sim in (small, tiled):
+        sim.md_init()
+        sim.md_steps(2)
+        sim.set("wait_polls", [1])
+        with pytest.raises(cm.CapacError) as e:
+            sim.md_steps(4)
+        assert e.value.code == cm.ERR_CUDA
+        assert sim.stats().md_step == 3
+    for name in STATE:
+        if name not in ("fx", "fy", "fz", "virial"):  # of a vector that no solve has left defined
+            assert rel_err(small.get(name), tiled.get(name)) < 1e-9, name
+    # and goes on from there once the limit is gone
+    for sim in (small, tiled):
+        sim.set("wait_polls", [0])
+        sim.md_steps(2)
+        assert sim.stats().md_step == 5
+        assert np.all(np.isfinite(sim.positions()))
+
+
+@pytest.mark.parametrize("case", ["t_2np", "t_au55w"])
+def test_unconverged_step_is_the_last_one(case, monkeypatch):
+    """The same with the reference's iteration limit: two iterations of the
+    same recurrence, so the forces agree too."""
+    d = cm.Desc.from_paths(golden_paths(case))
+    small, tiled = _both(monkeypatch, d, max_iter=1, solver_tol=1e-26)
+    rng = np.random.default_rng(9)
+    f = {k: rng.normal(scale=100.0, size=d.n_atoms) for k in ("fx", "fy", "fz")}
+    for sim in (small, tiled):
+        for k, v in f.items():
+            sim.set(k, v)
+        with pytest.raises(cm.CapacError) as e:
+            sim.md_steps(3)
+        assert e.value.code == cm.ERR_NOT_CONVERGED
+        assert "bicg_stab not converged" in str(e.value)
+        assert sim.stats().md_step == 1
+    for name in STATE:
+        assert rel_err(small.get(name), tiled.get(name)) < 1e-9, name
