@@ -74,7 +74,16 @@ void drop_solve(capac_ctx *c)
     }
 }
 
-// Waits for the stream; throws the failures of RATTLE and of a pending solve.
+// Throws when the host's words tell of a RATTLE failure.
+void check_rattle(capac_ctx *c)
+{
+    if (!c->sig[1] && !c->sig[2]) return;
+    const bool first = c->sig[1] != 0;
+    c->sig[1] = c->sig[2] = 0;
+    throw Error(CAPAC_ERR_RATTLE, first ? "RATTLE_1 not converged!" : "RATTLE_2 not converged!");
+}
+
+// Waits for the stream; throws the failures of a pending solve and of RATTLE.
 void check_flags(capac_ctx *c)
 {
     CAPAC_CUDA(cudaStreamSynchronize(c->stream));
@@ -172,6 +181,9 @@ void md_step(capac_ctx *c, bool last)
         c->phases = last;
         force(c);
     }
+    // RATTLE's words of the stages before this force call (seen with its
+    // displacement check): the step ends here, the solve's failure first
+    if (c->sig[1] || c->sig[2]) check_flags(c);
     launch_md_half_kick(c);
     launch_rattle(c, 1, true);
     launch_step_sums(c, c->ensemble, c->has_cstr);
@@ -243,14 +255,6 @@ double *state_array(capac_ctx *c, const std::string &n, int *count)
 }  // namespace
 
 void set_last_error(const std::string &msg) { g_last_error = msg; }
-
-void check_rattle(capac_ctx *c)
-{
-    if (!c->sig[1] && !c->sig[2]) return;
-    const bool first = c->sig[1] != 0;
-    c->sig[1] = c->sig[2] = 0;
-    throw Error(CAPAC_ERR_RATTLE, first ? "RATTLE_1 not converged!" : "RATTLE_2 not converged!");
-}
 
 constexpr int kProfSlots = 4096;
 

@@ -357,7 +357,6 @@ void launch_list_maintenance(capac_ctx *c, bool force_rebuild);
 // rebuilds the list); what needs no list may be launched in between
 void launch_begin_force(capac_ctx *c);
 void finish_begin_force(capac_ctx *c);
-void check_rattle(capac_ctx *c);  // throws when sig tells of a RATTLE failure
 // Rebuild the lists with an atom-list row for every atom, now and at every
 // later build (the gradient kernels walk all rows).
 void ensure_full_atom_list(capac_ctx *c);

@@ -1155,7 +1155,6 @@ void launch_begin_force(capac_ctx *c)
 void finish_begin_force(capac_ctx *c)
 {
     CAPAC_CUDA(cudaEventSynchronize(c->ev_flags));
-    check_rattle(c);
     if (!c->list_valid || c->sig[0] == c->disp_tag) {
         const bool cl = c->clusters || c->cpairs;
         build_list(c);

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import capacmd_b200 as cm
-from conftest import golden_paths, rel_err
+from conftest import golden_paths, impossible_constraints, rel_err, variant
 
 pytestmark = pytest.mark.gpu
 
@@ -126,3 +126,23 @@ def test_unconverged_step_is_the_last_one(case, monkeypatch):
         assert sim.stats().md_step == 1
     for name in STATE:
         assert rel_err(small.get(name), tiled.get(name)) < 1e-9, name
+
+
+def test_failed_solve_comes_before_failed_constraints(tmp_path, monkeypatch):
+    """A step in which the solve and RATTLE fail reports the solve (the force
+    call comes first), and no later call reports it again."""
+    d = cm.Desc.from_paths(variant("t_au55w", tmp_path, par=impossible_constraints))
+    for sim in _both(monkeypatch, d, solver_tol=1e-26):
+        sim.md_init()
+        sim.set("wait_polls", [1])
+        with pytest.raises(cm.CapacError) as e:
+            sim.md_steps(1)
+        assert e.value.code == cm.ERR_CUDA
+        sim.set("wait_polls", [0])
+        sim.set("vec_pq", np.zeros(d.n_mat))
+        try:
+            sim.force()
+        except cm.CapacError as later:  # the constraints' own failure, not read yet
+            assert later.code == cm.ERR_RATTLE
+            sim.force()
+        assert np.all(np.isfinite(sim.forces()))
