@@ -197,15 +197,15 @@ void md_step(capac_ctx *c, bool last)
 // Device memory to the caller's, after the stream's work.  A pageable
 // destination is filled from a pinned buffer, in chunks, so that the copy over
 // the bus runs beside the host's (452,057 doubles into fresh memory: 818 us by
-// the runtime's own staging with the two copies around it, 290 so); a pinned
-// one is copied to directly.
+// the runtime's own staging with the two copies around it, 290 so); one that the
+// runtime knows (pinned, managed or device memory) is copied to directly.
 void fetch(capac_ctx *c, void *dst, const void *src, size_t bytes)
 {
     if (bytes == 0) return;
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) cudaGetLastError();
-    if (at.type == cudaMemoryTypeHost || at.type == cudaMemoryTypeManaged) {
-        CAPAC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream));
+    if (at.type != cudaMemoryTypeUnregistered) {
+        CAPAC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, c->stream));
         CAPAC_CUDA(cudaStreamSynchronize(c->stream));
         return;
     }
