@@ -1295,6 +1295,11 @@ int capac_get(capac_ctx *c, const char *name, double *out)
             count = 5;
             return;
         }
+        if (n == "dense_solver") {  // 1 when solves run on the small systems' solver (k_solve_dense.cu)
+            out[0] = c->dense_ex ? 1.0 : 0.0;
+            count = 1;
+            return;
+        }
         if (n == "inner_stalls") {  // inner solves of the refinement stopped for lack of progress
             out[0] = (double)c->inner_stalls;
             count = 1;

@@ -364,6 +364,8 @@ int capac_checkpoint_load(capac_ctx *ctx, const char *path);
  * all are streamed from HBM each pass; the resident blocks per SM of the
  * group-ordered solver without and with tiles in tensor memory; the CTAs of
  * the cluster that last inverted the coarse matrix, 1 for one block, 0 none),
+ * dense_solver(1: 1 when solves run on the small systems' solver, which keeps
+ * the whole FP64 matrix on the chip and uses none of that layout),
  * inner_stalls(1: inner solves of the mixed path's refinement that stopped
  * because their (r, r) had not halved in 60 iterations and handed their
  * iterate back to the FP64 refinement),
