@@ -450,32 +450,33 @@ __global__ void __launch_bounds__(128) k_coarse_w(int nG, int nc, int n_nps, con
 
 // K W (the layout of W), K the inverse blocks dinv[g][c][o]: block (g, 32
 // columns), thread r one row of group g, the columns of W staged in shared
-// memory 32 rows at a time.
+// memory 32 rows at a time.  Summed in FP64, as the solver sums all products with
+// these matrices, and rounded once, as K and W are.
 __global__ void __launch_bounds__(128) k_coarse_kw(int nc, const float *__restrict__ dinv, const float *__restrict__ w,
                                                    float *__restrict__ kw)
 {
-    __shared__ float ws[32][33];  // [column][row of the chunk]
+    __shared__ double ws[32][33];  // [column][row of the chunk]
     const int g = blockIdx.x, j0 = blockIdx.y * 32, r = threadIdx.x;
-    float acc[32];
+    double acc[32];
 #pragma unroll
-    for (int q = 0; q < 32; ++q) acc[q] = 0.f;
+    for (int q = 0; q < 32; ++q) acc[q] = 0.0;
     for (int c0 = 0; c0 < kRows; c0 += 32) {
         __syncthreads();
         for (int q = threadIdx.x; q < 32 * 32; q += blockDim.x) {
             const int jj = q >> 5, cc = q & 31;
-            ws[jj][cc] = j0 + jj < nc ? w[((size_t)g * nc + j0 + jj) * kRows + c0 + cc] : 0.f;
+            ws[jj][cc] = j0 + jj < nc ? (double)w[((size_t)g * nc + j0 + jj) * kRows + c0 + cc] : 0.0;
         }
         __syncthreads();
 #pragma unroll 4
         for (int cc = 0; cc < 32; ++cc) {
-            const float k = dinv[((size_t)g * kRows + c0 + cc) * kRows + r];
+            const double k = (double)dinv[((size_t)g * kRows + c0 + cc) * kRows + r];
 #pragma unroll
-            for (int q = 0; q < 32; ++q) acc[q] = fmaf(k, ws[q][cc], acc[q]);
+            for (int q = 0; q < 32; ++q) acc[q] = fma(k, ws[q][cc], acc[q]);
         }
     }
 #pragma unroll
     for (int q = 0; q < 32; ++q)
-        if (j0 + q < nc) kw[((size_t)g * nc + j0 + q) * kRows + r] = acc[q];
+        if (j0 + q < nc) kw[((size_t)g * nc + j0 + q) * kRows + r] = (float)acc[q];
 }
 
 }  // namespace
