@@ -75,14 +75,12 @@ __device__ __forceinline__ float rcp_approx(float x)
     return r;
 }
 
-__device__ __forceinline__ float erfc_from_gauss_f(float x, float gauss);
 // erfc(x) for 0 <= x in FP32 as exp(-x^2) R(x), with R(x) = erfc(x) exp(x^2)
 // (the scaled complementary error function) fitted on [0, 5] by a degree-9
 // polynomial in t = 1 / (1 + x / 2), least squares in relative error
 // (relative error of R below 4e-8 in exact arithmetic, 3e-7 in FP32).  The
 // caller has exp(-x^2) already, for the Gaussian term of the same pair.
-// Beyond x = 5 the library erfcf.
-__device__ __forceinline__ float erfc_near_f(float x, float gauss)
+__device__ __forceinline__ float erfc_from_gauss_f(float x, float gauss)
 {
     const float t = rcp_approx(fmaf(0.5f, x, 1.0f));
     float r = -3.71903017e-02f;
@@ -97,9 +95,10 @@ __device__ __forceinline__ float erfc_near_f(float x, float gauss)
     r = fmaf(r, t, -9.64172679e-05f);
     return gauss * r;
 }
-__device__ __forceinline__ float erfc_from_gauss_f(float x, float gauss)
+// The same for any x: the library's beyond the fitted range.
+__device__ __forceinline__ float erfc_any_f(float x, float gauss)
 {
-    return x >= 5.0f ? erfcf(x) : erfc_near_f(x, gauss);
+    return x >= 5.0f ? erfcf(x) : erfc_from_gauss_f(x, gauss);
 }
 
 // FP64 pair term (force on j = f * rvec), reference formulas with the
@@ -199,7 +198,7 @@ __device__ __forceinline__ float pair_term_f(const PairConstsF &K, const TypePai
     if (qi != 0.f && qj != 0.f) {
         const float qq = K.fqq * qi * qj;
         if (K.use_coulomb == 1) {
-            const float ar = K.alpha * r, eg = expf(-ar * ar), ec = erfc_from_gauss_f(ar, eg);
+            const float ar = K.alpha * r, eg = expf(-ar * ar), ec = erfc_any_f(ar, eg);
             f += qq * ((ec * r2inv + K.a2_sqrtpi * eg * rinv) - K.w_const) * rinv;
             e_qq += qq * (ec * rinv - K.w_erfc_arcut + K.w_const * (r - K.rc));
         } else {
@@ -220,7 +219,7 @@ __device__ __forceinline__ void cpim_charge_pair_f(const PairConstsF &K, const f
     if (K.use_coulomb == 1) {
         const float ar = K.alpha * rr;
         eg = expf(-ar * ar);
-        ec = erfc_from_gauss_f(ar, eg);
+        ec = erfc_any_f(ar, eg);
         a0 = (ec * r2inv + K.a2_sqrtpi * eg * rinv - K.w_const) * rinv;
     } else {
         a0 = r2inv * rinv;
@@ -1079,7 +1078,7 @@ __global__ void __launch_bounds__(kHalfWarps * 32, kHalfBlocks) k_pair_half(
                     }
                     if (mk.w != 0.f && bq != 0.f) {
                         const float qq = K.fqq * mk.w * bq, eg = exp2_approx(fmaf(K.gauss2, r2, K.gauss2_lo * r2)),
-                                    ec = erfc_near_f(K.alpha * r, eg);
+                                    ec = erfc_from_gauss_f(K.alpha * r, eg);
                         fp += qq * ((ec * r2inv + K.a2_sqrtpi * eg * rinv) - K.w_const) * rinv;
                         eq = qq * (ec * rinv - K.w_erfc_arcut + K.w_const * (r - K.rc));
                     }
