@@ -6,8 +6,12 @@
 // reduction and the preconditioner, twice), each a grid barrier with dependent
 // round trips to L2 on both sides, 19 us (FP64) and 29 us (mixed path) per
 // iteration whatever the size.  Here block b holds 12 whole rows of the dense
-// matrix, column e = tid + 256 m in the registers of thread tid, and every
-// block carries all the vectors (the same elements in the same threads).  A
+// matrix, column e = tid + 256 m with thread tid, and every block carries all the
+// vectors (the same elements in the same threads).  Up to three columns a thread
+// all of it is in registers.  With five and seven (769 unknowns and more) 255
+// registers do not hold the rows' 480 and 672 bytes beside the vectors: the
+// compiler keeps 248 and 664 bytes a thread on the stack (mixed path 192 and 640),
+// and the products read what of the rows is among them back through L1.  A
 // product is 12 C fused multiply-adds per thread and a block reduction; what
 // the blocks exchange is only their 12 new values, and all that follows (dots,
 // scalars, vector updates) every block does on the same numbers in the same
@@ -25,8 +29,9 @@
 // them cost ~70 ns per writer (17 us per iteration with one flag word per
 // block packed together).  The first read waits 600 cycles: earlier it misses
 // and the polls slow the stores (n = 1,237: 7.0 us per iteration without the
-// wait, 5.3 with it, 5.9 with 300).  12 rows because fewer blocks read less
-// from the same lines (n = 589: 4 rows on 148 blocks 5.8 us, 12 on 50 4.6).
+// wait, 5.3 with it, 5.9 with 300; measured at that size only).  12 rows
+// because fewer blocks read less from the same lines (n = 589: 4 rows on 148
+// blocks 5.8 us, 12 on 50 4.6).
 // Every poll is bounded (wait_polls); a block that gives up sets the error
 // word, which ends the other blocks' polls, and all return.
 //
@@ -42,8 +47,8 @@
 //     so one sweep usually reaches refine_tol.
 //
 // Which systems: 12 rows per block, one block per SM, 256 x 7 columns: up to
-// 443 metal atoms with one nanoparticle on 148 SMs;
-// beyond, the chip's registers do not hold the FP64 matrix.
+// 443 metal atoms with one nanoparticle on 148 SMs, whose blocks have no rows for
+// more.
 // Cold solves of Au55/147/309 in water against the tiled solvers (one B200):
 // FP64 to rTr < 1e-24 bTb 954 -> 349, 1,532 -> 346, 2,081 -> 621 us (6.2, 3.8
 // and 5.3 us per iteration); mixed to 1e-10, with the sweeps and residuals

@@ -1,12 +1,13 @@
-"""The register-resident solver of small CPIM systems against the tiled one.
+"""The solver of small CPIM systems against the tiled one.
 
 Both run the reference's BiCGSTAB (bicg_stab.c:253-573) on the same matrix and
 differ in the order of the sums only, so at rTr < 1e-26 bTb the induced
-vectors agree to the 1e-10 of the other tight solver comparisons.  Sizes at the
-edges of the kernel's variants (rows per block x columns per thread): 13 atoms
-(4 x 1), 55 (4 x 1), 110 in two particles (4 x 3), 147 (589 unknowns: all 148
-blocks of 4 rows), two of 147 (1,178: all 148 blocks of 8 rows), 309 (12 x 5),
-309 + 55 (12 x 7) and 309 + 147 (1,826: beyond, tiled both times).
+vectors agree to the 1e-10 of the other tight solver comparisons.  Every block
+has 12 rows; the kernel's variants are its columns per thread (256 unknowns
+each): 13 atoms in one particle (53 unknowns, 5 blocks) and 55 (221) have one
+column, two of 55 (442) two, 147 (589) three, two of 147 (1,178) and 309 (1,237)
+five, 309 + 55 (1,458) seven, and 309 + 147 (1,826) is beyond, tiled both times.
+Four columns and the last size that fits: test_gpu_solver_tiled.py.
 """
 import os
 
