@@ -375,16 +375,22 @@ int capac_create(const capac_desc *d, const capac_options *opt, capac_ctx **out)
         if (opt) o = *opt;
         if (o.skin <= 0.0) o.skin = 0.2;
         if (o.device < 0 || o.device >= ndev) throw Error(CAPAC_ERR_NO_DEVICE, "device ordinal out of range");
-        cudaDeviceProp prop;
-        CAPAC_CUDA(cudaGetDeviceProperties(&prop, o.device));
-        if (prop.major != 10) throw Error(CAPAC_ERR_NO_DEVICE, std::string("needs an sm_100 device, found ") + prop.name);
+        // (all properties at once take 2.4 ms, half of a small system's creation)
+        int major = 0, sms = 0;
+        CAPAC_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, o.device));
+        CAPAC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, o.device));
+        if (major != 10) {
+            cudaDeviceProp prop;
+            CAPAC_CUDA(cudaGetDeviceProperties(&prop, o.device));
+            throw Error(CAPAC_ERR_NO_DEVICE, std::string("needs an sm_100 device, found ") + prop.name);
+        }
         CAPAC_CUDA(cudaSetDevice(o.device));
 
         capac_ctx *c = new capac_ctx();
         try {
             c->opt = o;
             c->device = o.device;
-            c->num_sms = prop.multiProcessorCount;
+            c->num_sms = sms;
             c->use_graphs = getenv("CAPAC_NO_GRAPHS") == nullptr;
             c->phase_timer = getenv("CAPAC_SOLVER_PHASES") != nullptr;
             derive(d, &c->c);
@@ -421,8 +427,15 @@ int capac_create(const capac_desc *d, const capac_options *opt, capac_ctx **out)
                 c->fz = c->fy + ns;
                 c->xyz = c->fz + ns;
             }
-            c->ox = dalloc<double>(N); c->oy = dalloc<double>(N); c->oz = dalloc<double>(N);
-            c->rx0 = dalloc<double>(N); c->ry0 = dalloc<double>(N); c->rz0 = dalloc<double>(N);
+            {  // six arrays in one allocation: each of more than about 1 MB takes 0.33 ms
+                const size_t ns = (N + 31) & ~31L;
+                c->ox = dalloc<double>(6 * ns);
+                c->oy = c->ox + ns;
+                c->oz = c->oy + ns;
+                c->rx0 = c->oz + ns;
+                c->ry0 = c->rx0 + ns;
+                c->rz0 = c->ry0 + ns;
+            }
             c->pos4 = dalloc<double4>(N + (N + 1) / 2);
             c->pos4f = reinterpret_cast<float4 *>(c->pos4 + N);
 
@@ -580,11 +593,13 @@ int capac_create(const capac_desc *d, const capac_options *opt, capac_ctx **out)
             c->flags = dalloc<int>(8);
             CAPAC_CUDA(cudaMemsetAsync(c->flags, 0, sizeof(int) * 8, s));
             {
-                // one allocation for all pinned memory: each takes 1.6 to 3.6 ms
-                // whatever its size up to 2 MB (11 MB: 9 ms)
+                // one allocation for all pinned memory, at most the 2 MB that the runtime
+                // hands out in one piece: a new piece takes 2.5 ms, room in one that
+                // another context has 4 us.  A buffer of half the size would let a large
+                // system share too, and reads its forces 8% slower.
                 const size_t part = 1024;
                 static_assert(sizeof(SolverScalars) <= 1024 && sizeof(ThermoState) <= 1024, "parts of the pinned block");
-                c->stage_bytes = std::min<size_t>(std::max<size_t>(sizeof(double) * 3 * N, 1 << 16), 2 << 20);
+                c->stage_bytes = std::min<size_t>(std::max<size_t>(sizeof(double) * 3 * N, 1 << 16), (2 << 20) - 4 * part);
                 CAPAC_CUDA(cudaMallocHost(&c->pinned, 4 * part + c->stage_bytes));
                 unsigned char *b = static_cast<unsigned char *>(c->pinned);
                 memset(b, 0, 4 * part);
@@ -756,8 +771,7 @@ int capac_destroy(capac_ctx *c)
 {
     if (!c) return CAPAC_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    void *dev[] = {c->rx, c->ry, c->rz, c->vx, c->vy, c->vz, c->fx, c->ox, c->oy, c->oz,
-                   c->rx0, c->ry0, c->rz0, c->pos4, c->type, c->mol_id, c->mol_type,
+    void *dev[] = {c->rx, c->ry, c->rz, c->vx, c->vy, c->vz, c->fx, c->ox, c->pos4, c->type, c->mol_id, c->mol_type,
                    c->atom_in_mol, c->is_metal, c->type_metal, c->charge, c->mass, c->inv_mass, c->mol_atoms,
                    c->excl_offset, c->excl, c->nb_funct, c->nb_par, c->mol_first, c->mol_last, c->cstr_off,
                    c->cstr_cnt, c->cstr_i, c->cstr_j, c->cstr_r, c->np_start, c->np_end, c->np_charge,
