@@ -336,7 +336,7 @@ def main() -> int:
             ia = _issue_active("pair")
             r["note"] = ("FP32 pair terms on the CUDA cores, one list pass per step: bound by instruction issue "
                          "and latency, not by bytes" + (f" (ncu issue active {ia:.0%} of peak on the 91k-atom "
-                                                         f"workload, profiles/k_pair_cl_half_c3.md)" if ia else ""))
+                                                         f"workload, profiles/k_pair_half_c3.md)" if ia else ""))
         return r
 
     dom = max(("pair", "spmv", "matrix", "solve"), key=lambda k: prof[k][1])

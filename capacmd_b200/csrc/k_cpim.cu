@@ -328,7 +328,8 @@ void launch_cpim_matrix(capac_ctx *c)
 {
     if (c->msym) {
         // (the dense solver forms the mixed path's matrix from the positions
-        // itself: the tiles then serve the coarse refreshes only)
+        // itself: the tiles then serve the coarse refreshes only, whose result it
+        // does not use)
         const bool due = c->dinv && c->precond_age % kPrecondEvery == 0;
         const bool coarse = due && c->twolevel && (c->precond_age == 0 || c->coarse_age % kCoarseEvery == 0);
         if (!c->dense_ex || c->opt.precision != CAPAC_PREC_MIXED || coarse) launch_sym_assemble(c);

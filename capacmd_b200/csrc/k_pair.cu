@@ -14,9 +14,9 @@
 // every pair the FP64 test accepts, and the entries that pass are compacted in
 // shared memory, 4 bytes each; then full warps form the FP64 difference, test it
 // and compute, their positions loaded one set ahead.  In FP64 the terms of an
-// ordinary pair are dsf_terms' ~55 operations.  Bound by latency and issue together:
-// at 24,000 atoms (FP64) 499 -> 347 us a launch, issue slots 55% busy, FP64 pipe 30%,
-// sixteen warps per SM of 128 registers, a quarter of the instructions FP64.
+// ordinary pair are dsf_terms' ~63 operations.  Bound by latency and issue together:
+// at 24,000 atoms (FP64) 499 -> 338 us a launch, at 91,122 2.28 -> 1.45 ms with issue
+// slots 52% busy, FP64 pipe 30%, sixteen warps per SM of 128 registers.
 //
 // The same traversal adds, on each charged non-metal atom, the force from the
 // induced charges and dipoles of metal neighbours inside the cut-off: the
