@@ -427,15 +427,8 @@ int capac_create(const capac_desc *d, const capac_options *opt, capac_ctx **out)
                 c->fz = c->fy + ns;
                 c->xyz = c->fz + ns;
             }
-            {  // six arrays in one allocation: each of more than about 1 MB takes 0.33 ms
-                const size_t ns = (N + 31) & ~31L;
-                c->ox = dalloc<double>(6 * ns);
-                c->oy = c->ox + ns;
-                c->oz = c->oy + ns;
-                c->rx0 = c->oz + ns;
-                c->ry0 = c->rx0 + ns;
-                c->rz0 = c->ry0 + ns;
-            }
+            c->ox = dalloc<double>(N); c->oy = dalloc<double>(N); c->oz = dalloc<double>(N);
+            c->rx0 = dalloc<double>(N); c->ry0 = dalloc<double>(N); c->rz0 = dalloc<double>(N);
             c->pos4 = dalloc<double4>(N + (N + 1) / 2);
             c->pos4f = reinterpret_cast<float4 *>(c->pos4 + N);
 
@@ -771,7 +764,7 @@ int capac_destroy(capac_ctx *c)
 {
     if (!c) return CAPAC_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
-    void *dev[] = {c->rx, c->ry, c->rz, c->vx, c->vy, c->vz, c->fx, c->ox, c->pos4, c->type, c->mol_id, c->mol_type,
+    void *dev[] = {c->rx, c->ry, c->rz, c->vx, c->vy, c->vz, c->fx, c->ox, c->oy, c->oz, c->rx0, c->ry0, c->rz0, c->pos4, c->type, c->mol_id, c->mol_type,
                    c->atom_in_mol, c->is_metal, c->type_metal, c->charge, c->mass, c->inv_mass, c->mol_atoms,
                    c->excl_offset, c->excl, c->nb_funct, c->nb_par, c->mol_first, c->mol_last, c->cstr_off,
                    c->cstr_cnt, c->cstr_i, c->cstr_j, c->cstr_r, c->np_start, c->np_end, c->np_charge,
