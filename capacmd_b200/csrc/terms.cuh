@@ -26,6 +26,9 @@ namespace capac {
 // the damped Coulomb force and energy of unit charges, absolute, 1.48e-14 (1.55e-14)
 // and 1.70e-16 (1.83e-16).
 //
+// CLOSE = false: without the remainders of u and of the last addition, for a caller
+// that needs erfc to an absolute 1e-17 only, beyond x = 1.5 (metal blocks).
+//
 // W of them side by side (the three widths of a metal pair share the constants'
 // moves).  Two pairs a lane in k_pair take ~160 registers, twelve warps per SM
 // instead of sixteen: 398 us for 350 at 24,000 atoms.
@@ -33,7 +36,7 @@ constexpr double kDsfMaxX = 5.0;
 struct Dsf {
     double rinv, r, eg, ec;
 };
-template <int W>
+template <int W, bool CLOSE = true>
 __device__ __forceinline__ void dsf_terms(const double (&alpha)[W], const double (&r2)[W], Dsf (&d)[W])
 {
     double y[W], e[W], x2[W], kd[W], f[W], f2[W], a[W], b[W], u[W], u2[W];
@@ -73,9 +76,14 @@ __device__ __forceinline__ void dsf_terms(const double (&alpha)[W], const double
         // quotient as q and the rest of its division
         const double z = fma(alpha[w], d[w].r, 3.5), dz = fma(alpha[w], d[w].r, 3.5 - z);
         asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y[w]) : "d"(z));
-        y[w] = fma(y[w], fma(-z, y[w], 1.0), y[w]);
-        const double q = 7.0 * y[w];
-        u[w] = fma(-y[w], fma(-dz, q, fma(-z, q, 7.0)), 1.0 - q);
+        e[w] = fma(-z, y[w], 1.0);
+        if (CLOSE) {
+            y[w] = fma(y[w], e[w], y[w]);
+            const double q = 7.0 * y[w];
+            u[w] = fma(-y[w], fma(-dz, q, fma(-z, q, 7.0)), 1.0 - q);
+        } else {
+            u[w] = fma(-7.0, fma(y[w], fma(e[w], e[w], e[w]), y[w]), 1.0);
+        }
         u2[w] = u[w] * u[w];
         a[w] = fma(1.44851080807840048e-07, u2[w], 9.39502676422655287e-07);
         b[w] = fma(1.21445591197839242e-08, u2[w], 6.32563657300747914e-07);
@@ -95,9 +103,9 @@ __device__ __forceinline__ void dsf_terms(const double (&alpha)[W], const double
     chain(a, u2, -2.89265044832767437e-01);
     chain(b, u2, 2.33130481600251627e-01);
     chain(b, u2, 1.55293655608894299e-01);
-    each([&](int w) {  // with the last addition's rounding error
+    each([&](int w) {  // CLOSE: with the last addition's rounding error
         const double R = fma(a[w], u[w], b[w]);
-        d[w].ec = fma(d[w].eg, R, d[w].eg * fma(a[w], u[w], b[w] - R));
+        d[w].ec = CLOSE ? fma(d[w].eg, R, d[w].eg * fma(a[w], u[w], b[w] - R)) : d[w].eg * R;
     });
 }
 __device__ __forceinline__ Dsf dsf_terms(double alpha, double r2)
@@ -204,8 +212,8 @@ __device__ __forceinline__ void cpim_block(const DevParams &P, const double4 &pi
     // range R is a polynomial continued outside its interval: it grows no faster
     // than the Chebyshev polynomial of degree 18, and times 3.7e-17 of R and
     // erfc(x) that is below 1e-24 everywhere beyond x = 5.  x is held below 26, where
-    // all is zero.  Below 1 the library's erf keeps the relative error that 1 - erfc
-    // loses.
+    // all is zero.  Below 1.5 the library's erf; beyond, erfc's error (2.2e-16 of at
+    // most 0.034) is below the rounding of 1 - erfc.
     const double r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
     const double ip[3] = {P.inv_r_pp, P.inv_r_pq, P.inv_r_qq};
     double al[3], er[3], g[3];
@@ -214,12 +222,12 @@ __device__ __forceinline__ void cpim_block(const DevParams &P, const double4 &pi
     const double top = 26.0 * rsqrt(r2);
 #pragma unroll
     for (int k = 0; k < 3; ++k) al[k] = fmin(ip[k], top);
-    dsf_terms<3>(al, rs, d);
+    dsf_terms<3, false>(al, rs, d);
     const double rr = d[0].r, rinv = d[0].rinv, r2inv = rinv * rinv, ir3 = r2inv * rinv;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         g[k] = d[k].eg;
-        er[k] = rr * ip[k] < 1.0 ? erf(sqrt(r2) * ip[k]) : 1.0 - d[k].ec;
+        er[k] = rr * ip[k] < 1.5 ? erf(sqrt(r2) * ip[k]) : 1.0 - d[k].ec;
     }
     const double c1 = ir3 * r2inv * (er[0] - 2.0 * kInvSqrtPi * ip[0] * rr * g[0]);
     const double c2 = 4.0 * kInvSqrtPi * (ip[0] * ip[0] * ip[0]) * r2inv * g[0];

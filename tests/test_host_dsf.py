@@ -105,7 +105,7 @@ def _approx(v):
     return float((np.array([v]).view(np.int64) & np.int64(-1 << 32)).view(np.float64)[0])
 
 
-def _dsf(alpha, r2, chains):
+def _dsf(alpha, r2, chains, close=True):
     odd_e, even_e, odd, even = chains
     hi, lo = (float.fromhex(v) for v in ("0x1.62e42fef00000p-1", "0x1.473de6af278edp-34"))
     assert "0x1.62e42fef00000p-1" in BODY and "0x1.473de6af278edp-34" in BODY
@@ -128,13 +128,17 @@ def _dsf(alpha, r2, chains):
     z = fma(alpha, r, 3.5)
     dz = fma(alpha, r, 3.5 - z)
     y = _approx(1.0 / z)
-    y = fma(y, fma(-z, y, 1.0), y)
-    q = 7.0 * y
-    u = fma(-y, fma(-dz, q, fma(-z, q, 7.0)), 1.0 - q)
+    e = fma(-z, y, 1.0)
+    if close:
+        y = fma(y, e, y)
+        q = 7.0 * y
+        u = fma(-y, fma(-dz, q, fma(-z, q, 7.0)), 1.0 - q)
+    else:
+        u = fma(-7.0, fma(y, fma(e, e, e), y), 1.0)
     u2 = u * u
     a, b = horner(odd, u2), horner(even, u2)
     R = fma(a, u, b)
-    return eg, fma(eg, R, eg * fma(a, u, b - R))
+    return eg, fma(eg, R, eg * fma(a, u, b - R)) if close else eg * R
 
 
 @pytest.mark.parametrize("alpha,r_max", [(2.0, 1.2), (4.0, 1.2), (0.75, 6.6)])
@@ -150,3 +154,17 @@ def test_rounded_evaluation(alpha, r_max):
     rms, most = np.sqrt((np.array(err) ** 2).mean(0)), np.abs(err).max(0)
     assert rms[0] < 0.8e-16 and most[0] < 2.0e-16, (rms, most)
     assert rms[1] < 1.8e-16 and most[1] < 6.0e-16, (rms, most)
+
+
+def test_rounded_erf_of_the_metal_blocks():
+    """1 - erfc beyond x = 1.5, in the form without the remainders: half an ulp of
+    the subtraction (5.6e-17) and erfc's error, at most 0.034 x 8e-16."""
+    rng = np.random.default_rng(9)
+    chains = _chains()
+    err = []
+    for x in rng.uniform(1.5, 6.0, 300):
+        alpha = 0.5
+        r2 = float((x / alpha) ** 2)
+        ec = _dsf(alpha, r2, chains, close=False)[1]
+        err.append(float(D(1.0 - ec) - (1 - _erfc((D(alpha) * D(alpha) * D(r2)).sqrt()))))
+    assert np.abs(err).max() < 8.4e-17, np.abs(err).max()
