@@ -15,7 +15,7 @@
 // shared memory, 4 bytes each; then full warps form the FP64 difference, test it
 // and compute, their positions loaded one set ahead.  In FP64 the terms of an
 // ordinary pair are dsf_terms' ~63 operations.  Bound by latency and issue together:
-// at 24,000 atoms (FP64) 499 -> 338 us a launch, at 91,122 2.28 -> 1.45 ms with issue
+// at 24,000 atoms (FP64) 499 -> 336 us a launch, at 91,122 2.28 -> 1.45 ms with issue
 // slots 52% busy, FP64 pipe 30%, sixteen warps per SM of 128 registers.
 //
 // The same traversal adds, on each charged non-metal atom, the force from the

@@ -14,6 +14,7 @@ import numpy as np
 import pytest
 
 import capacmd_b200 as cm
+import test_gpu_dense_solver as small
 import test_gpu_errors as errors
 import test_gpu_solver as solver
 from capacmd_b200 import configs
@@ -116,3 +117,10 @@ def test_edges_of_the_small_systems_solver(atoms, dense, prec, tmp_path, monkeyp
     bar = 1e-10 if prec == cm.PREC_FP64 else 1e-8  # as test_gpu_dense_solver.py
     assert rel_err(a.get("vec_pq"), b.get("vec_pq")) < bar
     assert rel_err(a.forces(), b.forces()) < bar
+
+
+@pytest.mark.parametrize("prec", PRECS)
+def test_which_systems_the_comparisons_solve_so(prec, tmp_path):
+    """Every system that test_gpu_dense_solver.py compares but its last, which is beyond."""
+    got = [cm.Simulation(small._desc(s, tmp_path), precision=prec).get("dense_solver")[0] for s in small.SHELLS]
+    assert got == [1.0] * (len(got) - 1) + [0.0]
